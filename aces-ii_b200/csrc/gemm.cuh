@@ -89,6 +89,34 @@ int gemv_f64(int M, int K, double alpha, const double *A, long long lda, const d
 int gemm_nt_f64_scratch(int M, int N, int K, double alpha, const double *A, long long lda,
                         const double *B, long long ldb, double beta, const CView &C,
                         double *ws, size_t cap, cudaStream_t st);
+
+// Several FP64 products in one launch: a device table of tasks, each
+//   C = alpha * sum_s A_s B_s^T + beta * C   over up to 4 K segments.
+// tri: C is symmetric (the two sides of every segment are the same rows, M = N,
+// beta = 0): only the lower triangle of tiles is computed, each stored twice.
+struct F64Seg {
+  const double *A, *B;
+  long long lda, ldb;
+  int K;
+};
+struct F64Task {
+  F64Seg seg[4];
+  int nseg, M, N, tri;
+  int tile0;  // first tile of the task in the launch (set by f64_tasks_plan)
+  CView C;
+};
+struct F64TaskPlan {
+  int tile = 0, tiles = 0, per_task = 0;
+  bool vec2 = false;
+};
+// tile shape of a table and the tile0 of its tasks (host side, before the
+// table is uploaded)
+int f64_tasks_plan(F64Task *tasks, int n, F64TaskPlan *plan);
+// the launch over tasks dev[0 .. n) of a planned table; with per_task != 0 any
+// run of equal-shaped tasks may be launched with tiles = n * per_task
+int f64_tasks_run(const F64Task *dev, int n, const F64TaskPlan &plan, double alpha, double beta,
+                  cudaStream_t st);
+
 // split-K support shared by the contraction kernels
 double *splitk_workspace(size_t doubles);
 // C = alpha * sum_z part[z] + beta * C; part[z] is [M][N] row-major, or

@@ -1,12 +1,8 @@
 // gemm_f64.cu -- FP64 contraction on the DMMA tensor-core path
-// (mma.sync.m8n8k4.f64): the plain-FP64 comparator of the engine and the
-// arithmetic of the reference's XGEMM -> DGEMM (tools/xgemm.F:10-49).
-//
-// Tile 128 x 128 x 16, 256 threads (8 warps as 2 x 4, each warp 64 x 32), a
-// 4-stage cp.async pipeline (three k tiles in flight while one is computed,
-// one barrier per k tile), padded shared-memory rows (20 doubles) so the
-// fragment loads of a half-warp hit 32 distinct banks.
+// (mma.sync .f64): the plain-FP64 path of the engine and the arithmetic of the
+// reference's XGEMM -> DGEMM (tools/xgemm.F:10-49).
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "gemm.cuh"
@@ -14,184 +10,319 @@
 namespace acesb200 {
 
 namespace {
-constexpr int BM = 128, BN = 128, BK = 16, LDS = BK + 4;
-constexpr int kThreads = 256;
-constexpr int kStages = 4;
-constexpr int kStageDoubles = (BM + BN) * LDS;
-constexpr int kSmemBytes = kStages * kStageDoubles * 8;
-static_assert(kSmemBytes <= 227 * 1024, "pipeline depth");
+// ---------------------------------------------------------------------------
+// k_gemm_f64: C = alpha * sum_s A_s B_s^T + beta * C over up to 4 K segments.
+//
+// A block computes one BM x BN tile (or one split-K slice of it) of one task;
+// a launch is a single task passed by value, or a device table of tasks.  The
+// k tiles (16 doubles, one 128-byte row per operand row) of all segments form
+// one sequence through a 4-stage cp.async pipeline.  Rows lie unpadded in
+// shared memory with the 16-byte chunk index XORed by 4 on odd rows: the
+// 8 lanes of a 128-bit load phase (two neighbouring rows x four chunks) then
+// cover all 32 banks, and so do the copies (one row per 8 lanes).
+//
+// A thread's fragment of a k step of 8 is one double2 per row: its two k
+// values are 2t and 2t+1 (t the lane's position in its group of four) in A
+// and in B alike.  The product sums over k, so this order is as good as the
+// instruction's own (t, t+4) and takes half the shared-memory loads.
+// ---------------------------------------------------------------------------
+constexpr int BK = 16, kStages = 4;
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
 template <int VEC>
-__device__ __forceinline__ void cp_async(double *dst, const double *src, bool valid) {
-  unsigned d = smem_u32(dst);
+__device__ __forceinline__ void cp_async(unsigned dst, const double *src, bool valid) {
   int sz = valid ? VEC * 8 : 0;
   if (VEC == 2)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(sz));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(sz));
   else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(sz));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(sz));
 }
 
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
+// c (16 x 8) += a (16 x 8) b (8 x 8)^T: a = rows g and g+8 x k (2t, 2t+1)
+__device__ __forceinline__ void dmma(double (&c)[4], const double2 &a0, const double2 &a1,
+                                     const double2 &b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0.x), "d"(a1.x), "d"(a0.y), "d"(a1.y), "d"(b.x), "d"(b.y));
 }
 
-// The copies of one operand tile (BM rows x BK doubles) in VEC-double chunks:
-// thread t always takes the chunks of k offset kc = (t % CPR) * VEC in rows
-// t / CPR + i * RS, so the row pointers, their bounds and the shared-memory
-// offsets are computed once per block; a k tile then adds its k0 and tests
-// one K bound.
-template <int VEC>
+// Tile shape: BM x BN, WR x WC warps, OCC blocks per SM the registers allow for
+template <int BM_, int BN_, int WR_, int WC_, int OCC_>
+struct TileF64 {
+  static constexpr int BM = BM_, BN = BN_, WR = WR_, WC = WC_, OCC = OCC_;
+  static constexpr int kThreads = 32 * WR * WC;
+  static constexpr int TM = BM / WR, TN = BN / WC, MI = TM / 16, NI = TN / 8;
+  static constexpr int kStageBytes = (BM + BN) * BK * 8;
+  static constexpr int kSmem = kStages * kStageBytes;
+  static_assert(TM % 16 == 0 && TN % 8 == 0, "warp tile of 16 x 8 products");
+  static_assert(kSmem * OCC <= 225 * 1024, "shared memory");
+};
+
+// The copies of one operand tile (ROWS x BK doubles) in VEC-double chunks:
+// thread t always takes the chunks of k offset kc in rows r0 + i * RS.
+template <int ROWS, int kThreads, int VEC>
 struct CopyPlan {
-  static constexpr int CPR = BK / VEC;          // chunks per row
-  static constexpr int RS = kThreads / CPR;     // row step between a thread's chunks
-  static constexpr int kPer = BM / RS;          // chunks per thread and operand
-  const double *row[kPer];                      // &X[row][kc] (X itself for rows past the end)
-  unsigned live;                                // bit i: row i inside the operand
-  int kc, soff0;                                // k offset; shared offset of chunk 0
-  __device__ __forceinline__ CopyPlan(const double *X, long long ld, int rows, int r0base) {
-    const int t = threadIdx.x;
+  static constexpr int CPR = BK / VEC;
+  static constexpr int RS = kThreads / CPR;
+  static constexpr int kPer = (ROWS + RS - 1) / RS;
+  static_assert(RS % 2 == 0, "a thread's rows share their parity (one swizzle)");
+  const double *base;   // &X[row0 + r0][kc] of the current segment
+  const double *safe;   // any valid address (the source of zero-size copies)
+  long long step;       // RS rows
+  unsigned live;        // bit i: row r0 + i RS inside the operand and the tile
+  int kc, soff;         // k offset; byte offset of chunk 0 inside the stage's tile
+  __device__ __forceinline__ void init(int rows, int row0) {
+    const int t = threadIdx.x, r0 = t / CPR;
     kc = (t % CPR) * VEC;
-    const int r0 = t / CPR;
-    soff0 = r0 * LDS + kc;
+    const int ch = (kc >> 1) ^ ((r0 & 1) << 2);
+    soff = (r0 * BK + ch * 2 + (kc & 1)) * 8;
     live = 0;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int gr = r0base + r0 + i * RS;
-      const bool ok = gr < rows;
-      row[i] = ok ? X + (long long)gr * ld + kc : X;
-      live |= ok ? 1u << i : 0u;
-    }
+    for (int i = 0; i < kPer; ++i)
+      live |= (r0 + i * RS < ROWS && row0 + r0 + i * RS < rows) ? 1u << i : 0u;
   }
-  __device__ __forceinline__ void issue(double *stage, const double *X, int k0, int ke) const {
-    const bool kok = k0 + kc < ke;
+  __device__ __forceinline__ void segment(const double *X, long long ld, int row0) {
+    safe = X;
+    base = X + (long long)(row0 + (int)threadIdx.x / CPR) * ld + kc;
+    step = (long long)RS * ld;
+  }
+  __device__ __forceinline__ void issue(unsigned tile, int k0, int K) const {
+    const bool kok = k0 + kc < K;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
+      if (ROWS % RS != 0 && i == kPer - 1 && (int)threadIdx.x / CPR + i * RS >= ROWS) break;
       const bool v = kok && ((live >> i) & 1u);
-      cp_async<VEC>(stage + soff0 + i * RS * LDS, v ? row[i] + k0 : X, v);
+      cp_async<VEC>(tile + soff + i * RS * BK * 8, v ? base + i * step + k0 : safe, v);
     }
   }
 };
-static_assert(BM == BN, "one copy plan shape for both operands");
 
-template <int VEC>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_gemm_nt_f64(int M, int N, int K, double alpha, const double *__restrict__ A, long long lda,
-                  const double *__restrict__ B, long long ldb, double beta, CView C, int kchunk,
-                  double *__restrict__ part) {
-  extern __shared__ double smem[];
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+__host__ __device__ __forceinline__ int f64_ktiles(const F64Task &T) {
+  int n = 0;
+  for (int s = 0; s < T.nseg; ++s) n += (T.seg[s].K + BK - 1) / BK;
+  return n;
+}
+// output tiles of a task
+__host__ __device__ __forceinline__ int f64_tiles(int M, int N, int tri, int BM, int BN) {
+  const int tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
+  return tri ? tm * (tm + 1) / 2 : tm * tn;
+}
+
+struct F64Launch {
+  F64Task one;            // the task when table is null
+  const F64Task *table;   // device table of ntask tasks
+  int ntask;
+  int per_task;           // tiles per task when all have the same shape, else 0
+  int kchunk;             // k tiles per split-K slice (blockIdx.y), 0: no split
+  double alpha, beta;
+  double *part;           // split-K partials [z][M][N]
+};
+
+template <class T, int VEC>
+__global__ void __launch_bounds__(T::kThreads, T::OCC)
+    k_gemm_f64(const __grid_constant__ F64Launch L) {
+  constexpr int BM = T::BM, BN = T::BN, MI = T::MI, NI = T::NI;
+  extern __shared__ __align__(128) unsigned char f64_smem[];
+  int t = blockIdx.x;
+  const F64Task *tk = &L.one;
+  if (L.table) {
+    int i = 0;
+    if (L.per_task) {
+      i = t / L.per_task;
+      t -= i * L.per_task;
+    } else {
+      while (i + 1 < L.ntask && t >= L.table[i + 1].tile0) ++i;
+      t -= L.table[i].tile0;
+    }
+    tk = L.table + i;
+  }
+  const int M = tk->M, N = tk->N, tri = tk->tri;
+  int tm, tn;
+  if (tri) {  // lower triangle of square tiles, row by row
+    tm = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (tm * (tm + 1) / 2 > t) --tm;
+    while ((tm + 1) * (tm + 2) / 2 <= t) ++tm;
+    tn = t - tm * (tm + 1) / 2;
+  } else {
+    // bands of 8 m tiles, m fastest inside a band: the tiles running together
+    // share few rows of both operands
+    const int tilesM = (M + BM - 1) / BM, tilesN = (N + BN - 1) / BN;
+    const int g = t / (8 * tilesN), r = t - g * 8 * tilesN, gm = min(8, tilesM - g * 8);
+    tm = g * 8 + r % gm;
+    tn = r / gm;
+  }
+  const int m0 = tm * BM, n0 = tn * BN;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps
-  const int lr = lane >> 2, lc = lane & 3;
-  double acc[8][4][2];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int wm = warp / T::WC, wn = warp % T::WC;
+  const int g = lane >> 2, q = lane & 3;
 
-  // split-K: blockIdx.z owns K range [kb, ke)
-  const int kb = blockIdx.z * kchunk;
-  const int ke = min(K, kb + kchunk);
-  const int nk = ke > kb ? (ke - kb + BK - 1) / BK : 0;
-  auto stA = [&](int s) { return smem + s * kStageDoubles; };
-  auto stB = [&](int s) { return smem + s * kStageDoubles + BM * LDS; };
-  const CopyPlan<VEC> pa(A, lda, M, m0), pb(B, ldb, N, n0);
-  // prologue: k tiles 0 .. kStages-2 in flight (one commit group each, empty
-  // groups past the end keep the count uniform)
-#pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) {
-    if (s < nk) {
-      pa.issue(stA(s), A, kb + s * BK, ke);
-      pb.issue(stB(s), B, kb + s * BK, ke);
+  const int nkt = f64_ktiles(*tk);
+  const int kb = L.kchunk ? (int)blockIdx.y * L.kchunk : 0;
+  const int ke = L.kchunk ? min(nkt, kb + L.kchunk) : nkt;
+  const int nk = max(0, ke - kb);
+
+  CopyPlan<BM, T::kThreads, VEC> pa;
+  CopyPlan<BN, T::kThreads, VEC> pb;
+  pa.init(M, m0);
+  pb.init(N, n0);
+  // segment of the next k tile to issue, its K and the k offset inside it
+  int sg = 0, segK = 0, kin = kb * BK;
+  auto enter = [&]() {
+    segK = tk->seg[sg].K;
+    pa.segment(tk->seg[sg].A, tk->seg[sg].lda, m0);
+    pb.segment(tk->seg[sg].B, tk->seg[sg].ldb, n0);
+  };
+  if (nk > 0) {
+    while (sg + 1 < tk->nseg && kin >= (tk->seg[sg].K + BK - 1) / BK * BK) {
+      kin -= (tk->seg[sg].K + BK - 1) / BK * BK;
+      ++sg;
+    }
+    enter();
+  }
+  const unsigned sbase = smem_u32(f64_smem);
+  int issued = 0, slot_w = 0;
+  auto issue_next = [&]() {
+    if (issued < nk) {
+      if (kin >= segK) {  // the previous segment is done
+        ++sg;
+        kin = 0;
+        enter();
+      }
+      const unsigned st = sbase + slot_w * T::kStageBytes;
+      pa.issue(st, kin, segK);
+      pb.issue(st + BM * BK * 8, kin, segK);
+      kin += BK;
+      ++issued;
+      slot_w = slot_w + 1 == kStages ? 0 : slot_w + 1;
     }
     cp_commit();
-  }
+  };
+
+  double acc[MI][NI][4];
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
+
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) issue_next();
+  const int sw = (g & 1) << 2;
+  int slot = 0;
   for (int kt = 0; kt < nk; ++kt) {
-    // group kt complete: at most kStages-2 younger groups still pending
-    cp_wait<kStages - 2>();
+    cp_wait<kStages - 2>();   // k tile kt has landed
     __syncthreads();
-    // refill the slot computed in the previous iteration (every thread is past it)
-    const int nxt = kt + kStages - 1;
-    if (nxt < nk) {
-      pa.issue(stA(nxt % kStages), A, kb + nxt * BK, ke);
-      pb.issue(stB(nxt % kStages), B, kb + nxt * BK, ke);
-    }
-    cp_commit();
-    const double *a_s = stA(kt % kStages) + (wm * 64) * LDS;
-    const double *b_s = stB(kt % kStages) + (wn * 32) * LDS;
+    issue_next();             // into the slot every thread left before the barrier
+    const unsigned char *st = f64_smem + slot * T::kStageBytes;
+    slot = slot + 1 == kStages ? 0 : slot + 1;
+    const double *a_s = reinterpret_cast<const double *>(st) + (wm * T::TM + g) * BK;
+    const double *b_s = reinterpret_cast<const double *>(st) + (BM + wn * T::TN + g) * BK;
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double af[8], bf[4];
+    for (int s = 0; s < 2; ++s) {
+      const int ch = ((s * 4 + q) ^ sw) * 2;
+      double2 af[MI][2], bf[NI];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) af[i] = a_s[(i * 8 + lr) * LDS + kk + lc];
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = b_s[(j * 8 + lr) * LDS + kk + lc];
+        for (int h = 0; h < 2; ++h)
+          af[i][h] = *reinterpret_cast<const double2 *>(a_s + (i * 16 + h * 8) * BK + ch);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int j = 0; j < NI; ++j)
+        bf[j] = *reinterpret_cast<const double2 *>(b_s + j * 8 * BK + ch);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) dmma(acc[i][j], af[i][0], af[i][1], bf[j]);
     }
   }
-  cp_wait0();
-  if (part) {
-    // split-K partial: dense [z][M][N]
-    double *pz = part + (size_t)blockIdx.z * M * N;
+  cp_wait<0>();
+
+  if (L.part) {  // split-K partial: dense [z][M][N]
+    double *pz = L.part + (size_t)blockIdx.y * M * N;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int m = m0 + wm * 64 + i * 8 + lr;
-      if (m >= M) continue;
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int h = 0; h < 2; ++h) {
+        const int m = m0 + wm * T::TM + i * 16 + h * 8 + g;
+        if (m >= M) continue;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          int n = n0 + wn * 32 + j * 8 + lc * 2 + h;
-          if (n < N) pz[(size_t)m * N + n] = acc[i][j][h];
-        }
-    }
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int n = n0 + wn * T::TN + j * 8 + q * 2 + e;
+            if (n < N) pz[(size_t)m * N + n] = acc[i][j][2 * h + e];
+          }
+      }
     return;
   }
   // epilogue through the two-level output view; the beta*C loads of a row
   // are issued together before its stores
+  const CView C = tk->C;
+  const double alpha = L.alpha, beta = L.beta;
+  const bool mirror = tri && tm != tn;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int m = m0 + wm * 64 + i * 8 + lr;
-    if (m >= M) continue;
-    long long mo = cview_dim(C.mdiv, C.sm1, C.sm0, m);
-    double old[4][2];
-    if (beta != 0.0) {
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+    for (int h = 0; h < 2; ++h) {
+      const int m = m0 + wm * T::TM + i * 16 + h * 8 + g;
+      if (m >= M) continue;
+      const long long mo = cview_dim(C.mdiv, C.sm1, C.sm0, m);
+      double old[NI][2];
+      if (beta != 0.0) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          int n = n0 + wn * 32 + j * 8 + lc * 2 + h;
-          old[j][h] = n < N ? __ldg(C.p + mo + cview_dim(C.ndiv, C.sn1, C.sn0, n)) : 0.0;
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int n = n0 + wn * T::TN + j * 8 + q * 2 + e;
+            old[j][e] = n < N ? __ldg(C.p + mo + cview_dim(C.ndiv, C.sn1, C.sn0, n)) : 0.0;
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < NI; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int n = n0 + wn * T::TN + j * 8 + q * 2 + e;
+          if (n >= N) continue;
+          double r = alpha * acc[i][j][2 * h + e];
+          if (beta != 0.0) r += beta * old[j][e];
+          C.p[mo + cview_dim(C.ndiv, C.sn1, C.sn0, n)] = r;
+          if (mirror)
+            C.p[cview_dim(C.mdiv, C.sm1, C.sm0, n) + cview_dim(C.ndiv, C.sn1, C.sn0, m)] = r;
         }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        int n = n0 + wn * 32 + j * 8 + lc * 2 + h;
-        if (n >= N) continue;
-        double r = alpha * acc[i][j][h];
-        if (beta != 0.0) r += beta * old[j][h];
-        C.p[mo + cview_dim(C.ndiv, C.sn1, C.sn0, n)] = r;
-      }
-    }
+}
+
+// launch of one tile shape; the shared-memory opt-in is per device
+template <class T, int VEC>
+int launch_tile(const F64Launch &L, unsigned tiles, unsigned z, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  ACES_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) {
+    set_error("gemm_nt_f64: device %d outside 0..63", dev);
+    return ACES_ERR_ARG;
   }
+  if (!attr_set[dev]) {
+    ACES_CUDA(cudaFuncSetAttribute(k_gemm_f64<T, VEC>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
+    attr_set[dev] = true;
+  }
+  k_gemm_f64<T, VEC><<<dim3(tiles, z), T::kThreads, T::kSmem, st>>>(L);
+  count_launch();
+  ACES_CUDA(cudaGetLastError());
+  return ACES_OK;
 }
 }  // namespace
 
@@ -335,80 +466,11 @@ __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double 
   }
 }
 
-// ---------------------------------------------------------------------------
-// Thin contractions (one output dimension S <= 32): out(l, s) = sum_k X[l,k] Y[s,k]
-// with X the long operand (L rows) and Y the short one.  64 x 32 output tile
-// per block, K staged in 32-wide shared-memory chunks, 8 outputs per thread in
-// FP64 FMA; split-K over blockIdx.z.  Written to C(m,n) = out(l,s) or out(s,l).
-// These products stream their long operand once: bandwidth bound.
-// ---------------------------------------------------------------------------
-constexpr int TL = 64, TS = 32, TK = 32;
-
-__global__ void __launch_bounds__(256)
-    k_gemm_thin_f64(int L, int S, int K, double alpha, const double *__restrict__ X,
-                    long long ldx, const double *__restrict__ Y, long long ldy, double beta,
-                    CView C, bool s_is_m, int kchunk, double *__restrict__ part) {
-  __shared__ double Xs[TL][TK + 1];
-  __shared__ double Ys[TS][TK + 1];
-  const int l0 = blockIdx.x * TL;
-  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  const int t = threadIdx.x, r = t >> 3, c = t & 7;
-  double acc[2][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (int k0 = kb; k0 < ke; k0 += TK) {
-    for (int e = t; e < TL * TK; e += 256) {
-      int rr = e / TK, kk = e % TK;
-      int l = l0 + rr, k = k0 + kk;
-      Xs[rr][kk] = (l < L && k < ke) ? X[(long long)l * ldx + k] : 0.0;
-    }
-    for (int e = t; e < TS * TK; e += 256) {
-      int rr = e / TK, kk = e % TK;
-      int k = k0 + kk;
-      Ys[rr][kk] = (rr < S && k < ke) ? Y[(long long)rr * ldy + k] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < TK; ++kk) {
-      double x0 = Xs[2 * r][kk], x1 = Xs[2 * r + 1][kk];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        double y = Ys[4 * c + j][kk];
-        acc[0][j] = fma(x0, y, acc[0][j]);
-        acc[1][j] = fma(x1, y, acc[1][j]);
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    int l = l0 + 2 * r + i;
-    if (l >= L) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int sidx = 4 * c + j;
-      if (sidx >= S) continue;
-      int m = s_is_m ? sidx : l, n = s_is_m ? l : sidx;
-      if (part) {
-        part[(size_t)blockIdx.z * (size_t)L * S + (size_t)l * S + sidx] = acc[i][j];
-        continue;
-      }
-      double *cp = C.p + cview_off(C, m, n);
-      double v = alpha * acc[i][j];
-      if (beta != 0.0) v += beta * *cp;
-      *cp = v;
-    }
-  }
-}
-
 // Split-K reduction with many slices and few outputs: one warp per output,
 // lane k adds slices k, k+32, ..., then a fixed shuffle tree (deterministic).
-// layout 0: part[z][m][n]; 1: part[z][n][m]; 2 / 3: part[z][l][s] of the thin
-// kernel with (m, n) = (l, s) / (s, l) and S the short dimension.
+// part[z][m][n], or part[z][n][m] with mfast.
 __global__ void k_reduce_warp(CView C, const double *__restrict__ part, int M, int N, int Z,
-                              double alpha, double beta, int layout, int S) {
+                              double alpha, double beta, bool mfast) {
   const long long total = (long long)M * N;
   const int lane = threadIdx.x & 31;
   for (long long idx = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; idx < total;
@@ -417,18 +479,8 @@ __global__ void k_reduce_warp(CView C, const double *__restrict__ part, int M, i
     for (int z = lane; z < Z; z += 32) sum += part[(size_t)z * total + idx];
     for (int off = 16; off; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
     if (lane == 0) {
-      int m, n;
-      if (layout == 0) {
-        m = (int)(idx / N);
-        n = (int)(idx % N);
-      } else if (layout == 1) {
-        m = (int)(idx % M);
-        n = (int)(idx / M);
-      } else {  // thin partials: idx = l * S + s
-        const int l = (int)(idx / S), sidx = (int)(idx % S);
-        m = layout == 3 ? sidx : l;
-        n = layout == 3 ? l : sidx;
-      }
+      const int m = mfast ? (int)(idx % M) : (int)(idx / N);
+      const int n = mfast ? (int)(idx / M) : (int)(idx % N);
       double *cp = C.p + cview_off(C, m, n);
       double v = alpha * sum;
       if (beta != 0.0) v += beta * *cp;
@@ -438,29 +490,12 @@ __global__ void k_reduce_warp(CView C, const double *__restrict__ part, int M, i
 }
 
 static void launch_reduce_warp(const CView &C, const double *part, int M, int N, int Z,
-                               double alpha, double beta, int layout, int S, cudaStream_t st) {
+                               double alpha, double beta, bool mfast, cudaStream_t st) {
   const long long total = (long long)M * N;
   long long nb = (total + 7) / 8;  // 8 warps per block
   if (nb > 148 * 32) nb = 148 * 32;
-  k_reduce_warp<<<(unsigned)nb, 256, 0, st>>>(C, part, M, N, Z, alpha, beta, layout, S);
+  k_reduce_warp<<<(unsigned)nb, 256, 0, st>>>(C, part, M, N, Z, alpha, beta, mfast);
   count_launch();
-}
-
-// reduce thin split-K partials part[z][l][s] into C
-__global__ void k_thin_reduce(CView C, const double *__restrict__ part, int L, int S, int Z,
-                              double alpha, double beta, bool s_is_m) {
-  long long total = (long long)L * S;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int l = (int)(idx / S), sidx = (int)(idx % S);
-    double sum = 0.0;
-    for (int z = 0; z < Z; ++z) sum += part[(size_t)z * total + idx];
-    int m = s_is_m ? sidx : l, n = s_is_m ? l : sidx;
-    double *cp = C.p + cview_off(C, m, n);
-    double v = alpha * sum;
-    if (beta != 0.0) v += beta * *cp;
-    *cp = v;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -598,7 +633,7 @@ int splitk_reduce(const CView &C, const double *part, int M, int N, int Z, doubl
   long long total = (long long)M * N;
   if (Z >= 24 && total <= 16384) {
     // few outputs, many slices: a warp per output instead of a serial loop
-    launch_reduce_warp(C, part, M, N, Z, alpha, beta, mfast ? 1 : 0, 0, st);
+    launch_reduce_warp(C, part, M, N, Z, alpha, beta, mfast, st);
     ACES_CUDA(cudaGetLastError());
     return ACES_OK;
   }
@@ -650,12 +685,100 @@ int gemv_f64(int M, int K, double alpha, const double *A, long long lda, const d
   return ACES_OK;
 }
 
-int gemm_nt_f64(int M, int N, int K, double alpha, const double *A, long long lda,
-                const double *B, long long ldb, double beta, const CView &C, cudaStream_t st) {
-  if (M <= 0 || N <= 0) return ACES_OK;
-  if (K <= 0) {
-    // C = beta*C: run with K = 0 is a scale; issue through the kernel with no k tiles
+namespace {
+// Tile shapes.  The DMMA pipe of an SM is filled by several small blocks rather
+// than one large one: while one block waits at its k tile's barrier the others
+// issue.  8192 x 4096 x 4096: 34.8 TFLOP/s with 64 x 64 tiles and three blocks
+// per SM, 33.9 with 128 x 64 and two, 29.7 with 128 x 128 and one (the
+// m8n8k4 and the m16n8k8 form of the instruction measure the same); and the
+// last wave and the ragged edges of a 64-wide grid cost less: 2401 x 1519 x
+// 2050 takes 525 us against 734.  32 x 32 tiles serve outputs too small for
+// that: 120 x 96 x 150 in 8.7 us against 41.9 on one 128 x 128 tile.  The
+// 16- and 32-wide tiles are for products with a short side, which stream
+// their long operand: 404600 x 14 x 170 in 113 us (550 MB, 4.9 TB/s) against
+// 690 us for an FMA kernel with synchronous 64 x 32 tiles.
+using T64 = TileF64<64, 64, 2, 2, 3>;
+using T32 = TileF64<32, 32, 2, 2, 6>;
+using T6432 = TileF64<64, 32, 4, 1, 4>;
+using T6416 = TileF64<64, 16, 4, 1, 5>;
+enum TileId { kT64, kT32, kT6432, kT6416, kTiles };
+struct TileInfo {
+  int BM, BN, occ;
+  double eff[2];  // share of the DMMA rate with one block per SM, and with occ
+};
+// (480 x 480 x 1000 on one 64 x 64 or two 32 x 32 blocks per SM, and the large
+// shapes above)
+constexpr TileInfo kTile[kTiles] = {{64, 64, T64::OCC, {0.60, 0.94}},
+                                    {32, 32, T32::OCC, {0.35, 0.88}},
+                                    {64, 32, T6432::OCC, {0.40, 0.78}},
+                                    {64, 16, T6416::OCC, {0.25, 0.72}}};
+constexpr int kSms = 148;
+
+// Estimated time (us) of `tiles` tiles of nkt k tiles each: the blocks of the
+// fullest SM at the rate of the blocks running there together, plus the
+// pipeline's fill and drain per round of resident blocks.
+double est_us(const TileInfo &t, double tiles, double nkt) {
+  const double per_sm = std::ceil(tiles / kSms), r = std::min(per_sm, (double)t.occ);
+  const double eff = t.eff[0] + (t.eff[1] - t.eff[0]) * (t.occ > 1 ? (r - 1) / (t.occ - 1) : 1);
+  const double work = t.BM * t.BN * nkt * BK / 64.0 / 1.9e3;  // us per tile, 64 FMA/cycle
+  return per_sm * work / eff + 2.0 * std::ceil(per_sm / t.occ);
+}
+
+// Tile shape and split-K slice count of one product, by that estimate; a split
+// pays the write and read of its partials and a reduction launch.  part_cap:
+// doubles of split-K workspace available.
+struct F64Plan {
+  int tile = kT64, Z = 1;
+};
+F64Plan plan_f64(int M, int N, int nkt, size_t part_cap) {
+  F64Plan best;
+  double tbest = 1e300;
+  for (int id = 0; id < kTiles; ++id) {
+    const TileInfo &t = kTile[id];
+    const double tiles = (double)((M + t.BM - 1) / t.BM) * ((N + t.BN - 1) / t.BN);
+    const int zmax = (int)std::min<double>(nkt / 8, std::ceil(4.0 * kSms * t.occ / tiles));
+    for (int z = 1; z <= std::max(1, zmax); z += z < 16 ? 1 : z / 8) {
+      if (z > 1 && (double)z * M * N > (double)part_cap) break;
+      const int kc = (nkt + z - 1) / z;
+      double us = est_us(t, tiles * z, kc);
+      // a short side: the long operand's bytes at the rate the copies reach
+      us = std::max(us, 8.0 * BK * nkt * (double)std::max(M, N) / 5.0e6);
+      if (z > 1) us += 4.0 + 16.0 * z * M * (double)N / 4.0e6;
+      if (us < tbest * 0.999) {
+        tbest = us;
+        best.tile = id;
+        best.Z = z;
+      }
+    }
   }
+  return best;
+}
+
+template <int VEC>
+int launch_id(int id, const F64Launch &L, unsigned tiles, unsigned z, cudaStream_t st) {
+  switch (id) {
+    case kT64: return launch_tile<T64, VEC>(L, tiles, z, st);
+    case kT32: return launch_tile<T32, VEC>(L, tiles, z, st);
+    case kT6432: return launch_tile<T6432, VEC>(L, tiles, z, st);
+    default: return launch_tile<T6416, VEC>(L, tiles, z, st);
+  }
+}
+// 16-byte copies: aligned operands with even leading dimensions and K
+bool vec2_ok(const F64Task &t) {
+  for (int s = 0; s < t.nseg; ++s) {
+    const F64Seg &g = t.seg[s];
+    if (g.lda % 2 || g.ldb % 2 || g.K % 2 || ((uintptr_t)g.A & 15) || ((uintptr_t)g.B & 15))
+      return false;
+  }
+  return true;
+}
+
+// The dispatch of gemm_nt_f64 and gemm_nt_f64_scratch: `ws` is the caller's
+// workspace of `cap` doubles, or null for the library's own.
+int gemm_dispatch(int M, int N, int K, double alpha, const double *A, long long lda,
+                  const double *B, long long ldb, double beta, const CView &C, double *ws,
+                  size_t cap, cudaStream_t st) {
+  if (M <= 0 || N <= 0) return ACES_OK;
   // a few thousand outputs: one warp each (no tiles, no split K)
   if ((long long)M * N <= kTinyOut && K > 0 && K <= 8192) {
     k_gemm_tiny_f64<<<(unsigned)(((long long)M * N * 32 + 255) / 256), 256, 0, st>>>(
@@ -666,187 +789,117 @@ int gemm_nt_f64(int M, int N, int K, double alpha, const double *A, long long ld
   }
   // K <= 32: output-bound low-rank update
   if (K <= LR_K) return launch_lowrank(M, N, K, alpha, A, lda, B, ldb, beta, C, st);
-  // one output dimension <= 32: thin kernel over the long dimension
-  if (M <= TS || N <= TS) {
-    bool s_is_m = M <= TS && (M <= N);
-    int L = s_is_m ? N : M, S = s_is_m ? M : N;
-    const double *X = s_is_m ? B : A;
-    const double *Y = s_is_m ? A : B;
-    long long ldx = s_is_m ? ldb : lda, ldy = s_is_m ? lda : ldb;
-    long long lt = (L + TL - 1) / TL;
-    int Z = 1, kchunk = K;
-    double *part = nullptr;
-    if (lt < 592 && K >= 4 * TK) {
-      Z = (int)std::min<long long>((592 + lt - 1) / lt, K / (2 * TK));
-      if (Z > 1) {
-        kchunk = ((K + Z - 1) / Z + TK - 1) / TK * TK;
-        Z = (K + kchunk - 1) / kchunk;
-        part = splitk_workspace((size_t)Z * L * S);
-        if (!part) {
-          set_error("gemm thin: split-K workspace allocation failed");
-          return ACES_ERR_NOMEM;
-        }
-      }
-    }
-    dim3 g((unsigned)lt, 1, Z);
-    k_gemm_thin_f64<<<g, 256, 0, st>>>(L, S, K, alpha, X, ldx, Y, ldy, beta, C, s_is_m, kchunk,
-                                       Z > 1 ? part : nullptr);
-    count_launch();
-    ACES_CUDA(cudaGetLastError());
-    if (Z >= 24 && (long long)L * S <= 16384) {
-      launch_reduce_warp(C, part, M, N, Z, alpha, beta, s_is_m ? 3 : 2, S, st);
-      ACES_CUDA(cudaGetLastError());
-    } else if (Z > 1) {
-      long long total = (long long)L * S;
-      long long nb = (total + 255) / 256;
-      if (nb > 148 * 16) nb = 148 * 16;
-      k_thin_reduce<<<(unsigned)nb, 256, 0, st>>>(C, part, L, S, Z, alpha, beta, s_is_m);
-      count_launch();
-      ACES_CUDA(cudaGetLastError());
-    }
-    return ACES_OK;
+  F64Launch L{};
+  F64Task &t = L.one;
+  t.nseg = 1;
+  t.M = M;
+  t.N = N;
+  t.seg[0] = F64Seg{A, B, lda, ldb, K};
+  t.C = C;
+  if (M < N) {  // the longer side takes the tile's longer edge
+    std::swap(t.M, t.N);
+    t.seg[0] = F64Seg{B, A, ldb, lda, K};
+    t.C = CView{C.p, C.ndiv, C.sn1, C.sn0, C.mdiv, C.sm1, C.sm0};
   }
-  static bool attr_set[64] = {false};  // the shared-memory opt-in is per device
-  int dev = 0;
-  ACES_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) {
-    set_error("gemm_nt_f64: device %d outside 0..63", dev);
+  L.alpha = alpha;
+  L.beta = beta;
+  const int nkt = f64_ktiles(t);
+  const size_t kOwn = size_t(1) << 25;  // of the library's own workspace: 256 MB
+  const F64Plan p = plan_f64(t.M, t.N, nkt, ws ? cap : kOwn);
+  const long long tiles = (long long)((t.M + kTile[p.tile].BM - 1) / kTile[p.tile].BM) *
+                          ((t.N + kTile[p.tile].BN - 1) / kTile[p.tile].BN);
+  if (tiles > 0x7fffffffLL) {
+    set_error("gemm_nt_f64: %lld output tiles", tiles);
     return ACES_ERR_ARG;
   }
-  if (!attr_set[dev]) {
-    ACES_CUDA(cudaFuncSetAttribute(k_gemm_nt_f64<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kSmemBytes));
-    ACES_CUDA(cudaFuncSetAttribute(k_gemm_nt_f64<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kSmemBytes));
-    attr_set[dev] = true;
-  }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) {
-    set_error("gemm_nt_f64: M=%d too large", M);
-    return ACES_ERR_ARG;
-  }
-  // split K when the output has too few tiles to fill the GPU
-  int Z = 1;
-  long long tiles = (long long)grid.x * grid.y;
-  int nkt = (K + BK - 1) / BK;
-  if (tiles < 148 && nkt >= 16) {
-    Z = (int)std::min<long long>((296 + tiles - 1) / tiles, nkt / 8);
-    if (Z < 1) Z = 1;
-  }
-  int kchunk = K;
-  double *part = nullptr;
+  int Z = p.Z;
   if (Z > 1) {
-    kchunk = ((K + Z - 1) / Z + BK - 1) / BK * BK;
-    Z = (K + kchunk - 1) / kchunk;
-    part = splitk_workspace((size_t)Z * M * N);
-    if (!part) {
+    L.kchunk = (nkt + Z - 1) / Z;
+    Z = (nkt + L.kchunk - 1) / L.kchunk;
+    L.part = ws ? ws : splitk_workspace((size_t)Z * t.M * t.N);
+    if (!L.part) {
       set_error("gemm_nt_f64: split-K workspace allocation failed");
       return ACES_ERR_NOMEM;
     }
-    grid.z = Z;
   }
-  bool vec2 = (lda % 2 == 0) && (ldb % 2 == 0) && (K % 2 == 0) &&
-              ((reinterpret_cast<uintptr_t>(A) & 15) == 0) &&
-              ((reinterpret_cast<uintptr_t>(B) & 15) == 0);
-  if (kchunk % 2) vec2 = false;
-  if (vec2)
-    k_gemm_nt_f64<2><<<grid, kThreads, kSmemBytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                         kchunk, part);
+  if (vec2_ok(t))
+    ACES_TRY(launch_id<2>(p.tile, L, (unsigned)tiles, (unsigned)Z, st));
   else
-    k_gemm_nt_f64<1><<<grid, kThreads, kSmemBytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                         kchunk, part);
-  count_launch();
-  ACES_CUDA(cudaGetLastError());
-  if (part) return splitk_reduce(C, part, M, N, Z, alpha, beta, st);
+    ACES_TRY(launch_id<1>(p.tile, L, (unsigned)tiles, (unsigned)Z, st));
+  if (L.part) return splitk_reduce(t.C, L.part, t.M, t.N, Z, alpha, beta, st);
   return ACES_OK;
 }
+}  // namespace
 
-}  // namespace acesb200
+int gemm_nt_f64(int M, int N, int K, double alpha, const double *A, long long lda,
+                const double *B, long long ldb, double beta, const CView &C, cudaStream_t st) {
+  return gemm_dispatch(M, N, K, alpha, A, lda, B, ldb, beta, C, nullptr, 0, st);
+}
 
-namespace acesb200 {
-
-// The same FP64 contraction dispatch as gemm_nt_f64, with every scratch
-// buffer taken from caller-provided device memory `ws` (capacity `cap`
-// doubles) instead of the library's allocated workspace.  Split-K is reduced
-// to what fits; when even the unsplit form needs no scratch it runs unsplit.
+// The same dispatch with the split-K partials taken from caller-provided
+// device memory `ws` (capacity `cap` doubles) instead of the library's
+// workspace; where they do not fit the product runs unsplit.
 int gemm_nt_f64_scratch(int M, int N, int K, double alpha, const double *A, long long lda,
                         const double *B, long long ldb, double beta, const CView &C,
                         double *ws, size_t cap, cudaStream_t st) {
-  if (M <= 0 || N <= 0) return ACES_OK;
-  if (K <= LR_K) return launch_lowrank(M, N, K, alpha, A, lda, B, ldb, beta, C, st);
-  if (M <= TS || N <= TS) {
-    bool s_is_m = M <= TS && (M <= N);
-    int L = s_is_m ? N : M, S = s_is_m ? M : N;
-    const double *X = s_is_m ? B : A;
-    const double *Y = s_is_m ? A : B;
-    long long ldx = s_is_m ? ldb : lda, ldy = s_is_m ? lda : ldb;
-    long long lt = (L + TL - 1) / TL;
-    int Z = 1, kchunk = K;
-    if (lt < 592 && K >= 4 * TK) {
-      long long zfit = (long long)(cap / ((size_t)L * S));
-      Z = (int)std::min<long long>(std::min<long long>((592 + lt - 1) / lt, K / (2 * TK)), zfit);
-      if (Z > 1) {
-        kchunk = ((K + Z - 1) / Z + TK - 1) / TK * TK;
-        Z = (K + kchunk - 1) / kchunk;
-      } else {
-        Z = 1;
-        kchunk = K;
-      }
+  return gemm_dispatch(M, N, K, alpha, A, lda, B, ldb, beta, C, ws, cap, st);
+}
+
+// ---- task tables --------------------------------------------------------------
+// 64 x 64 tiles unless 32 x 32 ones are estimated faster (triangular tasks
+// need a square tile, and a table mixes both kinds)
+int f64_tasks_plan(F64Task *tasks, int n, F64TaskPlan *plan) {
+  *plan = F64TaskPlan{};
+  double work[2] = {0.0, 0.0};
+  long long total[2] = {0, 0};
+  bool same = true, vec2 = true;
+  for (int i = 0; i < n; ++i) {
+    const F64Task &t = tasks[i];
+    if (t.M < 1 || t.N < 1 || t.nseg < 1 || t.nseg > 4 || (t.tri && t.M != t.N)) {
+      set_error("f64 tasks: task %d is %d x %d with %d segments", i, t.M, t.N, t.nseg);
+      return ACES_ERR_ARG;
     }
-    dim3 g((unsigned)lt, 1, Z);
-    k_gemm_thin_f64<<<g, 256, 0, st>>>(L, S, K, alpha, X, ldx, Y, ldy, beta, C, s_is_m, kchunk,
-                                       Z > 1 ? ws : nullptr);
-    count_launch();
-    ACES_CUDA(cudaGetLastError());
-    if (Z > 1) {
-      long long total = (long long)L * S;
-      long long nb = (total + 255) / 256;
-      if (nb > 148 * 16) nb = 148 * 16;
-      k_thin_reduce<<<(unsigned)nb, 256, 0, st>>>(C, ws, L, S, Z, alpha, beta, s_is_m);
-      count_launch();
-      ACES_CUDA(cudaGetLastError());
+    const int nkt = f64_ktiles(t);
+    for (int b = 0; b < 2; ++b) {
+      const int nt = f64_tiles(t.M, t.N, t.tri, kTile[b].BM, kTile[b].BN);
+      total[b] += nt;
+      work[b] += (double)nt * nkt;
     }
-    return ACES_OK;
+    same = same && t.M == tasks[0].M && t.N == tasks[0].N && t.tri == tasks[0].tri;
+    vec2 = vec2 && vec2_ok(t);
   }
-  ACES_CUDA(cudaFuncSetAttribute(k_gemm_nt_f64<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes));
-  ACES_CUDA(cudaFuncSetAttribute(k_gemm_nt_f64<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes));
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) {
-    set_error("gemm_nt_f64_scratch: M=%d too large", M);
+  if (n == 0) return ACES_OK;
+  int b = 0;
+  if (est_us(kTile[kT32], (double)total[1], work[1] / total[1]) <
+      est_us(kTile[kT64], (double)total[0], work[0] / total[0]))
+    b = 1;
+  if (total[b] > 0x7fffffffLL) {
+    set_error("f64 tasks: %lld output tiles", total[b]);
     return ACES_ERR_ARG;
   }
-  int Z = 1;
-  long long tiles = (long long)grid.x * grid.y;
-  int nkt = (K + BK - 1) / BK;
-  if (tiles < 148 && nkt >= 16) {
-    long long zfit = (long long)(cap / ((size_t)M * N));
-    Z = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, nkt / 8), zfit);
-    if (Z < 1) Z = 1;
+  long long at = 0;
+  for (int i = 0; i < n; ++i) {
+    tasks[i].tile0 = (int)at;
+    at += f64_tiles(tasks[i].M, tasks[i].N, tasks[i].tri, kTile[b].BM, kTile[b].BN);
   }
-  int kchunk = K;
-  double *part = nullptr;
-  if (Z > 1) {
-    kchunk = ((K + Z - 1) / Z + BK - 1) / BK * BK;
-    Z = (K + kchunk - 1) / kchunk;
-    part = ws;
-    grid.z = Z;
-  }
-  bool vec2 = (lda % 2 == 0) && (ldb % 2 == 0) && (K % 2 == 0) &&
-              ((reinterpret_cast<uintptr_t>(A) & 15) == 0) &&
-              ((reinterpret_cast<uintptr_t>(B) & 15) == 0);
-  if (kchunk % 2) vec2 = false;
-  if (vec2)
-    k_gemm_nt_f64<2><<<grid, kThreads, kSmemBytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                         kchunk, part);
-  else
-    k_gemm_nt_f64<1><<<grid, kThreads, kSmemBytes, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                         kchunk, part);
-  count_launch();
-  ACES_CUDA(cudaGetLastError());
-  if (part) return splitk_reduce(C, part, M, N, Z, alpha, beta, st);
+  plan->tile = b;
+  plan->tiles = (int)at;
+  plan->per_task = same ? (int)(at / n) : 0;
+  plan->vec2 = vec2;
   return ACES_OK;
+}
+
+int f64_tasks_run(const F64Task *dev, int n, const F64TaskPlan &plan, double alpha, double beta,
+                  cudaStream_t st) {
+  if (n == 0 || plan.tiles == 0) return ACES_OK;
+  F64Launch L{};
+  L.table = dev;
+  L.ntask = n;
+  L.per_task = plan.per_task;
+  L.alpha = alpha;
+  L.beta = beta;
+  return plan.vec2 ? launch_id<2>(plan.tile, L, (unsigned)plan.tiles, 1, st)
+                   : launch_id<1>(plan.tile, L, (unsigned)plan.tiles, 1, st);
 }
 
 }  // namespace acesb200
