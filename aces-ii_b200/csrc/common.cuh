@@ -112,6 +112,10 @@ struct PairType {
 };
 PairType pair_type(int type);   // type 1..25
 
+// aces_inipck with the choice of leaving a new list's memory unfilled (for a
+// producer that writes every element)
+int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, bool zero);
+
 // Orbital count of irrep h (0-based) for 'O'/'V' (RHF: alpha == beta).
 inline int norb(const SymInfo &s, char c, int h) { return c == 'O' ? s.pop[h] : s.vrt[h]; }
 

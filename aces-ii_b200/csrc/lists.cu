@@ -123,6 +123,53 @@ static int copy_cols(double *ext, int first, int ncols, int irrep, int list, boo
   return ACES_OK;
 }
 
+static int list_touch(int ncols, int nrows, int irrep, int list, bool zero) {
+  State &st = state();
+  std::lock_guard<std::recursive_mutex> lk(st.mu);
+  if (irrep < 1 || irrep > 8 || list < 0 || list > 1000 || ncols < 0 || nrows < 0) {
+    set_error("aces_list_touch: bad arguments (irrep %d list %d)", irrep, list);
+    return ACES_ERR_ARG;
+  }
+  auto &v = st.lists[list];
+  if (v.empty()) v.resize(8);
+  ListBlock &b = v[irrep - 1];
+  if (b.dev) {
+    if (b.nrows == nrows && b.ncols == ncols) return ACES_OK;
+    set_error("aces_list_touch: list %d irrep %d re-touched with %dx%d (was %dx%d)", list, irrep,
+              nrows, ncols, b.nrows, b.ncols);
+    return ACES_ERR_REDIM;
+  }
+  size_t bytes = (size_t)nrows * ncols * sizeof(double);
+  void *p = st.arena.alloc(bytes ? bytes : 256);
+  if (!p) {
+    set_error("aces_list_touch: out of device memory for %zu bytes", bytes);
+    return ACES_ERR_NOMEM;
+  }
+  if (bytes && zero) ACES_CUDA(cudaMemset(p, 0, bytes));
+  b.nrows = nrows;
+  b.ncols = ncols;
+  b.dev = (double *)p;
+  return ACES_OK;
+}
+
+int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, bool zero) {
+  State &st = state();
+  std::lock_guard<std::recursive_mutex> lk(st.mu);
+  const SymInfo &s = st.sym;
+  if (!s.ready) return ACES_ERR_NOSYM;
+  if (sytypl < 1 || sytypl > 22 || sytypr < 1 || sytypr > 22 || irrepx < 1 ||
+      irrepx > s.nirrep) {
+    set_error("aces_inipck: bad pair types %d/%d", sytypl, sytypr);
+    return ACES_ERR_ARG;
+  }
+  for (int r = 1; r <= s.nirrep; ++r) {
+    int l = aces_dirprd(r, irrepx);
+    ACES_TRY(list_touch(s.irpdpd[r - 1][sytypr - 1], s.irpdpd[l - 1][sytypl - 1], r, list, zero));
+  }
+  if (iset) st.isytyp[list == 0 ? 100 : list] = {sytypl, sytypr};
+  return ACES_OK;
+}
+
 }  // namespace acesb200
 
 using namespace acesb200;
@@ -223,32 +270,7 @@ int aces_dirprd(int i, int j) {
 
 int aces_list_touch(int ncols, int nrows, int irrep, int list, int nofrag) {
   (void)nofrag;
-  State &st = state();
-  std::lock_guard<std::recursive_mutex> lk(st.mu);
-  if (irrep < 1 || irrep > 8 || list < 0 || list > 1000 || ncols < 0 || nrows < 0) {
-    set_error("aces_list_touch: bad arguments (irrep %d list %d)", irrep, list);
-    return ACES_ERR_ARG;
-  }
-  auto &v = st.lists[list];
-  if (v.empty()) v.resize(8);
-  ListBlock &b = v[irrep - 1];
-  if (b.dev) {
-    if (b.nrows == nrows && b.ncols == ncols) return ACES_OK;
-    set_error("aces_list_touch: list %d irrep %d re-touched with %dx%d (was %dx%d)", list, irrep,
-              nrows, ncols, b.nrows, b.ncols);
-    return ACES_ERR_REDIM;
-  }
-  size_t bytes = (size_t)nrows * ncols * sizeof(double);
-  void *p = st.arena.alloc(bytes ? bytes : 256);
-  if (!p) {
-    set_error("aces_list_touch: out of device memory for %zu bytes", bytes);
-    return ACES_ERR_NOMEM;
-  }
-  if (bytes) ACES_CUDA(cudaMemset(p, 0, bytes));
-  b.nrows = nrows;
-  b.ncols = ncols;
-  b.dev = (double *)p;
-  return ACES_OK;
+  return list_touch(ncols, nrows, irrep, list, true);
 }
 
 int aces_updmoi(int ncols, int nrows, int irrep, int list, int iarg1, int iarg2) {
@@ -258,21 +280,7 @@ int aces_updmoi(int ncols, int nrows, int irrep, int list, int iarg1, int iarg2)
 }
 
 int aces_inipck(int irrepx, int sytypl, int sytypr, int list, int iset) {
-  State &st = state();
-  std::lock_guard<std::recursive_mutex> lk(st.mu);
-  const SymInfo &s = st.sym;
-  if (!s.ready) return ACES_ERR_NOSYM;
-  if (sytypl < 1 || sytypl > 22 || sytypr < 1 || sytypr > 22 || irrepx < 1 ||
-      irrepx > s.nirrep) {
-    set_error("aces_inipck: bad pair types %d/%d", sytypl, sytypr);
-    return ACES_ERR_ARG;
-  }
-  for (int r = 1; r <= s.nirrep; ++r) {
-    int l = aces_dirprd(r, irrepx);
-    ACES_TRY(aces_list_touch(s.irpdpd[r - 1][sytypr - 1], s.irpdpd[l - 1][sytypl - 1], r, list, 0));
-  }
-  if (iset) st.isytyp[list == 0 ? 100 : list] = {sytypl, sytypr};
-  return ACES_OK;
+  return list_inipck(irrepx, sytypl, sytypr, list, iset, true);
 }
 
 int aces_isytyp(int which, int list) {
