@@ -9,8 +9,8 @@
 // are promoted to FP64 every CHUNK = 512 K elements (fewer for very long K).
 //
 // Persistent kernel, one CTA per SM, k tile 64 (128-byte swizzle):
-//   warp 0  TMA producer (one elected lane)
-//   warp 1  TMEM allocator + MMA issuer (one elected lane)
+//   warp 0  TMA producer (all lanes wait, one elected lane issues)
+//   warp 1  TMEM allocator + MMA issuer (all lanes wait, one elected lane issues)
 //   warps 2.. epilogue: two or three warps per TMEM lane quadrant, each
 //             thread one output row x 48, 64 or 128 columns, accumulated in
 //             FP64 across K chunks
@@ -351,6 +351,19 @@ __device__ __forceinline__ uint32_t idesc_for(int n_live) {
          ((uint32_t)(mma_n<BN>(n_live) >> 3) << 17);
 }
 
+// The producer and MMA warps run their loops with all 32 lanes and issue from
+// one elected lane.  A loop under `lane == 0` is divergent code, where every
+// tcgen05.mma first moves its descriptors into uniform registers: measured
+// 62-87 cycles of issue per instruction, above the 64-72 cycles that a
+// 128 x 128 or 128 x 144 product takes, and 600 cycles of bookkeeping per k
+// tile; warp-uniform code issues one in 46.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(p));
+  return p != 0;
+}
+
 template <int CG>
 __device__ __forceinline__ void umma(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc,
                                      uint32_t acc) {
@@ -654,7 +667,7 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;
   // tile walk: by CTA (CG = 1) or by CTA pair (CG = 2)
   const int t0 = CG == 2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -693,9 +706,12 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     // ---------------- TMA producer (every CTA: its own tiles) ----------------
-    int it = 0;  // k tiles issued by this CTA
+    const bool el = elect_one();
+    int it = 0;               // k tiles issued by this CTA
+    int s = 0;                // stage of the next k tile
+    uint32_t ph = 1;          // parity of the `empty` phase it waits for
     bool stop = *(volatile int *)&g_tc_inject != 0;  // injected fault: issue nothing
     for (int t = t0; t < nTiles && !stop; t += tstep) {
       const TileRef T = decode_tile<CG, BN>(L, t);
@@ -704,36 +720,46 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
       int rA[kMaxSeg], rB[kMaxSeg];
       batch_rows(P, T.b, rA, rB);
       for (int kt = 0; kt < kTiles; ++kt) {
-        const int s = it % kStages;
-        if (it >= kStages && !mbar_wait_g<CG>(smem_u32(&empty[s]), ((it / kStages) - 1) & 1)) {
-          atomicExch(&g_tc_status, 1);
-          *(volatile int *)abort_flag = 1;
+        // (the first round of stages passes at once: parity 1 of a new barrier)
+        const bool w = mbar_wait_g<CG>(smem_u32(&empty[s]), ph);
+        if (!__all_sync(0xffffffffu, w)) {
+          if (el) {
+            atomicExch(&g_tc_status, 1);
+            *(volatile int *)abort_flag = 1;
+          }
           stop = true;
           break;
         }
-        if (*(volatile int *)abort_flag) {
+        if (__any_sync(0xffffffffu, *(volatile int *)abort_flag)) {
           stop = true;
           break;
         }
         const uint32_t fb = smem_u32(&full[s]);
         unsigned char *st = smem + s * kStage;
-        // a pair's stage completes on rank 0's barrier, armed with both halves
-        if (rank == 0) mbar_expect_tx(fb, CG * kStage);
         const StageAt sa = stage_at<CG, BN>(P, T, rA, rB, kt, rank);
         const int sg = sa.sg, kx = sa.kx, ya = sa.ya, yb = sa.yb;
-        if (CG == 1) {
-          tma_load_2d(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb);
-          tma_load_2d(smem_u32(st + TILE_A), &L.al[T.g][sg], kx, ya, fb);
-          tma_load_2d(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb);
-          tma_load_2d(smem_u32(st + 2 * TILE_A + kTileB), &L.bl[T.g][sg], kx, yb, fb);
-        } else {
-          const uint32_t fb0 = mapa_rank(fb, 0);
-          tma_load_2d_pair(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb0);
-          tma_load_2d_pair(smem_u32(st + TILE_A), &L.al[T.g][sg], kx, ya, fb0);
-          tma_load_2d_pair(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb0);
-          tma_load_2d_pair(smem_u32(st + 2 * TILE_A + kTileB), &L.bl[T.g][sg], kx, yb, fb0);
+        if (el) {
+          // a pair's stage completes on rank 0's barrier, armed with both halves
+          if (rank == 0) mbar_expect_tx(fb, CG * kStage);
+          if (CG == 1) {
+            tma_load_2d(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb);
+            tma_load_2d(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb);
+            tma_load_2d(smem_u32(st + 2 * TILE_A + kTileB), &L.bl[T.g][sg], kx, yb, fb);
+            tma_load_2d(smem_u32(st + TILE_A), &L.al[T.g][sg], kx, ya, fb);
+          } else {
+            const uint32_t fb0 = mapa_rank(fb, 0);
+            tma_load_2d_pair(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb0);
+            tma_load_2d_pair(smem_u32(st + TILE_A), &L.al[T.g][sg], kx, ya, fb0);
+            tma_load_2d_pair(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb0);
+            tma_load_2d_pair(smem_u32(st + 2 * TILE_A + kTileB), &L.bl[T.g][sg], kx, yb, fb0);
+          }
         }
+        __syncwarp();
         ++it;
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
+        }
       }
     }
     if (rank == 0) {
@@ -742,64 +768,76 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
       for (int k = first; k < it; ++k)
         if (!mbar_wait_g<CG>(smem_u32(&full[k % kStages]), (k / kStages) & 1))
           atomicExch(&g_tc_status, 2);
-      *(volatile int *)&peer_issued[1] = it;  // the stages this CTA armed
-    } else {
+      if (el) *(volatile int *)&peer_issued[1] = it;  // the stages this CTA armed
+    } else if (el) {
       // rank 0 accounts for this CTA's copies at teardown
       st_cluster_u32(mapa_rank(smem_u32(peer_issued), 0), (uint32_t)it);
     }
-  } else if (warp == 1 && lane == 0 && rank == 1) {
+  } else if (warp == 1 && rank == 1) {
     // rank 1 issues no products: its TMEM is released after rank 0's last one
     if (!mbar_wait_g<CG>(smem_u32(mma_done), 0)) atomicExch(&g_tc_status, 6);
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- MMA issuer (rank 0) ----------------
-    int it = 0, gc = 0;  // k tiles consumed, accumulation chunks started
+    const bool el = elect_one();  // one lane issues every product and commit
+    int s = 0, b = 0;             // stage, accumulator
+    uint32_t ph = 0, aph = 1;     // parities of their `full` / `acc_empty` phases
+    const uint64_t d0 = umma_desc(smem_u32(smem));
     bool stop = false;
     for (int t = t0; t < nTiles && !stop; t += tstep) {
       const TileRef T = decode_tile<CG, BN>(L, t);
       const int kTiles = T.kTiles, chunk = L.prob[T.g].chunk;
       const uint32_t idesc = idesc_for<CG, BN>(L.prob[T.g].N - T.n0);
+      int kin = 0;  // k tile inside the accumulation chunk
       for (int kt = 0; kt < kTiles; ++kt) {
-        const int kin = kt % chunk, b = gc % kNAcc;
-        if (kin == 0 && gc >= kNAcc &&
-            !mbar_wait_g<CG>(smem_u32(&acc_empty[b]), ((gc / kNAcc) - 1) & 1)) {
-          atomicExch(&g_tc_status, 5);
-          *(volatile int *)abort_flag = 1;
-          stop = true;
-          break;
+        bool w = true;
+        if (kin == 0) {  // a new chunk: its accumulator has been drained
+          w = __all_sync(0xffffffffu, mbar_wait_g<CG>(smem_u32(&acc_empty[b]), aph));
+          if (!w && el) atomicExch(&g_tc_status, 5);
         }
-        const int s = it % kStages;
-        if (!mbar_wait_g<CG>(smem_u32(&full[s]), (it / kStages) & 1)) {
-          atomicExch(&g_tc_status, 3);
-          *(volatile int *)abort_flag = 1;
+        if (w) {
+          w = __all_sync(0xffffffffu, mbar_wait_g<CG>(smem_u32(&full[s]), ph));
+          if (!w && el) atomicExch(&g_tc_status, 3);
+        }
+        if (!w) {
+          if (el) *(volatile int *)abort_flag = 1;
           stop = true;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t base = smem_u32(smem + s * kStage);
-        const uint32_t ah = base, al = base + TILE_A, bh = base + 2 * TILE_A, bl = bh + kTileB;
         const uint32_t acc_t = tmem + (uint32_t)(b * BN);
         // the start address is the descriptor's low field (address >> 4): the
         // 32-byte K step (16 BF16) inside a swizzled row adds 2 to it
-        const uint64_t dah = umma_desc(ah), dal = umma_desc(al), dbh = umma_desc(bh),
-                       dbl = umma_desc(bl);
+        const uint64_t dah = d0 + (uint64_t)(s * (kStage >> 4)), dal = dah + (TILE_A >> 4),
+                       dbh = dah + (2 * TILE_A >> 4), dbl = dbh + (kTileB >> 4);
+        const bool last = ++kin == chunk || kt == kTiles - 1;
+        if (el) {
 #pragma unroll
-        for (int kk = 0; kk < TBK / 16; ++kk) {
-          const uint64_t o = 2 * kk;
-          const uint32_t acc = (kin > 0 || kk > 0) ? 1u : 0u;
-          umma<CG>(acc_t, dah + o, dbh + o, idesc, acc);
-          umma<CG>(acc_t, dah + o, dbl + o, idesc, 1u);
-          umma<CG>(acc_t, dal + o, dbh + o, idesc, 1u);
+          for (int kk = 0; kk < TBK / 16; ++kk) {
+            const uint64_t o = 2 * kk;
+            const uint32_t acc = (kin > 1 || kk > 0) ? 1u : 0u;
+            umma<CG>(acc_t, dah + o, dbh + o, idesc, acc);
+            umma<CG>(acc_t, dah + o, dbl + o, idesc, 1u);
+            umma<CG>(acc_t, dal + o, dbh + o, idesc, 1u);
+          }
+          umma_commit<CG>(smem_u32(&empty[s]));
+          if (last) umma_commit<CG>(smem_u32(&acc_full[b]));
         }
-        umma_commit<CG>(smem_u32(&empty[s]));
-        ++it;
-        if (kin == chunk - 1 || kt == kTiles - 1) {
-          umma_commit<CG>(smem_u32(&acc_full[b]));
-          ++gc;
+        __syncwarp();
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
+        }
+        if (last) {
+          kin = 0;
+          if (++b == kNAcc) {
+            b = 0;
+            aph ^= 1;
+          }
         }
       }
     }
     // every product issued by this thread has retired before TMEM is released
-    umma_commit<CG>(smem_u32(mma_done));
+    if (el) umma_commit<CG>(smem_u32(mma_done));
     if (!mbar_wait_g<CG>(smem_u32(mma_done), 0)) atomicExch(&g_tc_status, 6);
   } else if (warp >= 2) {
     // ---------------- epilogue: FP64 accumulation of the chunks ----------------
