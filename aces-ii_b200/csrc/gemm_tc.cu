@@ -451,6 +451,10 @@ struct Problem {
   const BatchEntry *batch;
   int nbatch;
   int f32out;            // output elements are FP32
+  // tail split: tiles tail0, tail0 + 1, ... of the problem (numbered without
+  // split K) are computed in tailZ slices of tail_ktc k tiles (whole
+  // accumulation chunks), their sums going to part[slot]; tailZ 0: none
+  int tail0, tailZ, tail_ktc;
 };
 struct Launch {
   CUtensorMap ah[kMaxProb][kMaxSeg], al[kMaxProb][kMaxSeg];
@@ -463,6 +467,7 @@ struct Launch {
 };
 struct TileRef {
   int g, m0, n0, z, ktb, kTiles, b;
+  int slot;  // tail split: which part this slice's sums go to (else -1)
 };
 template <int CG, int BN>
 __device__ __forceinline__ TileRef decode_tile(const Launch &L, int t) {
@@ -470,9 +475,20 @@ __device__ __forceinline__ TileRef decode_tile(const Launch &L, int t) {
   r.g = 0;
   while (r.g + 1 < L.nprob && t >= L.prob[r.g + 1].tile0) ++r.g;
   const Problem &P = L.prob[r.g];
-  const int tl = t - P.tile0;
+  int tl = t - P.tile0;
   int tm, tn;
   r.b = 0;
+  r.slot = -1;
+  int tz = 0;
+  if (P.tailZ && tl >= P.tail0) {
+    // slice tz of tail tile i: the slices of one z run together (they share
+    // the rows of the tiles next to them)
+    const int n = P.tilesM * P.tilesN - P.tail0, u = tl - P.tail0;
+    tz = u / n;
+    const int i = u - tz * n;
+    tl = P.tail0 + i;
+    r.slot = i * P.tailZ + tz;
+  }
   if (P.batch) {
     // fewer-tiles side fastest, then the entry, then the other side
     if (P.mfast) {
@@ -502,6 +518,10 @@ __device__ __forceinline__ TileRef decode_tile(const Launch &L, int t) {
   r.n0 = tn * BN;
   r.ktb = r.z * P.ktc;
   r.kTiles = max(0, min(P.ktc, P.kTilesTotal - r.ktb));
+  if (r.slot >= 0) {
+    r.ktb = tz * P.tail_ktc;
+    r.kTiles = max(0, min(P.tail_ktc, P.kTilesTotal - r.ktb));
+  }
   return r;
 }
 
@@ -913,7 +933,13 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
           for (int j = 0; j < kCols; ++j, w.next())
             if (j < ncol) atomicAdd(cm + w.off, (float)(alpha * acc[j]));
         }
-      } else if (part) {
+      } else if (T.slot >= 0) {
+        // a tail slice: [slot][column][row], lanes write consecutive rows
+        double *pz = part + ((size_t)T.slot * BN + half * kCols) * TBM + row;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j)
+          if (j < ncol) pz[(size_t)j * TBM] = acc[j];
+      } else if (P.ktc < P.kTilesTotal) {
         // split-K partial, [z][n][m]: lanes write consecutive m
         double *pz = part + (size_t)z * M * N + m;
 #pragma unroll
@@ -983,6 +1009,49 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
                    "r"(kTmemCols));
   }
 }
+
+// The tail tiles' sums: C = alpha * sum_z part[tile][z] + beta * C, z in order.
+// One block per tile and 8 columns, one thread per row (consecutive rows of a
+// part are contiguous), two slices' loads of all columns in flight.
+constexpr int kTailCols = 8;
+__global__ void __launch_bounds__(TBM)
+    k_tail_reduce(CView C, const double *__restrict__ part, int M, int N, int tilesM, int tilesN,
+                  int mfast, int tail0, int Z, double alpha, double beta) {
+  const int i = blockIdx.x, tl = tail0 + i;
+  const int tm = mfast ? tl % tilesM : tl / tilesN, tn = mfast ? tl / tilesM : tl % tilesN;
+  const int m = tm * TBM + (int)threadIdx.x, n0 = tn * TBN_1 + blockIdx.y * kTailCols;
+  if (m >= M) return;
+  const int nc = min(kTailCols, N - n0);
+  constexpr size_t kPart = (size_t)TBN_1 * TBM;
+  const double *p = part + (size_t)i * Z * kPart + blockIdx.y * kTailCols * TBM + threadIdx.x;
+  double s[kTailCols];
+#pragma unroll
+  for (int j = 0; j < kTailCols; ++j) s[j] = 0.0;
+  int z = 0;
+  for (; z + 2 <= Z; z += 2, p += 2 * kPart) {
+    double x[kTailCols], y[kTailCols];
+#pragma unroll
+    for (int j = 0; j < kTailCols; ++j) {
+      x[j] = j < nc ? __ldcs(p + j * TBM) : 0.0;
+      y[j] = j < nc ? __ldcs(p + kPart + j * TBM) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kTailCols; ++j) s[j] = (s[j] + x[j]) + y[j];
+  }
+  if (z < Z) {
+#pragma unroll
+    for (int j = 0; j < kTailCols; ++j)
+      if (j < nc) s[j] += __ldcs(p + j * TBM);
+  }
+  double *const cm = C.p + cview_dim(C.mdiv, C.sm1, C.sm0, m);
+#pragma unroll
+  for (int j = 0; j < kTailCols; ++j)
+    if (j < nc) {
+      double *c = cm + cview_dim(C.ndiv, C.sn1, C.sn0, n0 + j);
+      *c = beta == 0.0 ? alpha * s[j] : alpha * s[j] + beta * *c;
+    }
+}
+static_assert(TBN_1 % kTailCols == 0, "column groups of a tail tile");
 
 // multiprocessor count of the current device (persistent grid size)
 int num_sms() {
@@ -1396,6 +1465,52 @@ int split_slices(long long tiles, int kTilesTotal, int nsm) {
   return Z;
 }
 
+// Split K for the last, partly filled wave only.  The persistent CTAs take
+// whole waves of tiles; the `tail` tiles left over would occupy `tail` of the
+// SMs for a whole tile time (16290 x 400 x 16290: 384 tiles are 2.6 waves but
+// took 3).  Cut into Z slices of whole accumulation chunks they fill the SMs:
+// the FP32 chunk values stay what they are, only the FP64 additions are
+// regrouped.  Costs, in us: 0.72 per k tile of a tile, 1.5 per slice (its
+// output), and the reduction, a launch and Z parts of 147 KB per tile.
+void plan_tail(Problem &P, long long tiles_before, int nsm) {
+  const long long tiles = (long long)P.tilesM * P.tilesN;
+  const int tail = (int)((tiles_before + tiles) % nsm);
+  const int nch = (P.kTilesTotal + P.chunk - 1) / P.chunk;
+  if (tail == 0 || tail > tiles || tiles_before + tiles <= nsm || nch < 2) return;
+  const double tau = 0.72 * P.kTilesTotal;
+  double best = tau - 4.0;
+  for (int z = 2; z <= std::min(nch, 8); ++z) {
+    const int per = (nch + z - 1) / z, zz = (nch + per - 1) / per;
+    if (zz != z) continue;
+    const double t = std::ceil((double)tail * z / nsm) * (0.72 * per * P.chunk + 1.5) + 5.0 +
+                     2.0 * tail * z * 0.147 / 5.0;
+    if (t < best) {
+      best = t;
+      P.tailZ = z;
+      P.tail_ktc = per * P.chunk;
+      P.tail0 = (int)(tiles - tail);
+    }
+  }
+}
+// tiles of a planned problem as scheduled, and the doubles of its parts
+long long tail_tiles(const Problem &P) {
+  const long long tiles = (long long)P.tilesM * P.tilesN;
+  return P.tailZ ? P.tail0 + (tiles - P.tail0) * P.tailZ : tiles;
+}
+size_t tail_doubles(const Problem &P) {
+  return P.tailZ ? (size_t)((long long)P.tilesM * P.tilesN - P.tail0) * P.tailZ * TBM * TBN_1 : 0;
+}
+int tail_reduce(const Problem &P, const double *part, double alpha, double beta,
+                cudaStream_t st) {
+  const int tail = P.tilesM * P.tilesN - P.tail0;
+  k_tail_reduce<<<dim3(tail, TBN_1 / kTailCols), TBM, 0, st>>>(P.C, part, P.M, P.N, P.tilesM,
+                                                              P.tilesN, P.mfast, P.tail0,
+                                                              P.tailZ, alpha, beta);
+  count_launch();
+  ACES_CUDA(cudaGetLastError());
+  return ACES_OK;
+}
+
 int multi_run(const TuneChoice &ch, const SplitOperand *A, const SplitOperand *B, int nseg,
               int M, int N, double alpha, double beta, const CView &C, cudaStream_t st) {
   Launch L;
@@ -1418,7 +1533,15 @@ int multi_run(const TuneChoice &ch, const SplitOperand *A, const SplitOperand *B
       return ACES_ERR_NOMEM;
     }
   }
-  const long long nTiles = tiles * Z;
+  if (Z == 1 && L.cg == 1) plan_tail(P, 0, nsm);
+  if (P.tailZ) {
+    part = splitk_workspace(tail_doubles(P));
+    if (!part) {
+      set_error("gemm_nt_bf16x3: split-K workspace allocation failed");
+      return ACES_ERR_NOMEM;
+    }
+  }
+  const long long nTiles = P.tailZ ? tail_tiles(P) : tiles * Z;
   if (nTiles > (1LL << 31) - 1) {
     set_error("gemm_nt_bf16x3: %lld output tiles exceed the scheduler range", nTiles);
     return ACES_ERR_ARG;
@@ -1426,6 +1549,7 @@ int multi_run(const TuneChoice &ch, const SplitOperand *A, const SplitOperand *B
   P.tile0 = 0;
   L.nTiles = (int)nTiles;
   ACES_TRY(launch_prepared(L, alpha, beta, part, st));
+  if (P.tailZ) return tail_reduce(P, part, alpha, beta, st);
   if (part) return splitk_reduce(C, part, M, N, Z, alpha, beta, st, true);
   return ACES_OK;
 }
@@ -1446,13 +1570,26 @@ int grouped_run(int cg, const GroupedProblem *probs, int nprob, double alpha, do
     ++n;
   }
   if (n == 0) return ACES_OK;
+  L.nprob = n;
+  // the launch's last tiles belong to its last problem
+  Problem &P = L.prob[n - 1];
+  double *part = nullptr;
+  if (L.cg == 1) plan_tail(P, P.tile0, num_sms());
+  if (P.tailZ) {
+    tiles = P.tile0 + tail_tiles(P);
+    part = splitk_workspace(tail_doubles(P));
+    if (!part) {
+      set_error("gemm_nt_bf16x3_grouped: split-K workspace allocation failed");
+      return ACES_ERR_NOMEM;
+    }
+  }
   if (tiles > (1LL << 31) - 1) {
     set_error("gemm_nt_bf16x3_grouped: %lld output tiles exceed the scheduler range", tiles);
     return ACES_ERR_ARG;
   }
-  L.nprob = n;
   L.nTiles = (int)tiles;
-  return launch_prepared(L, alpha, beta, nullptr, st);
+  ACES_TRY(launch_prepared(L, alpha, beta, part, st));
+  return P.tailZ ? tail_reduce(P, part, alpha, beta, st) : ACES_OK;
 }
 
 int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOperand *Bpar,
