@@ -412,6 +412,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
+// 16 rows x 32 columns as the fragments of 16 x 8 products: for column group g
+// of 8, lane l gets row l/4 (r[4g], r[4g+1]) and row l/4 + 8 (r[4g+2],
+// r[4g+3]) of the columns 2 (l%4) and 2 (l%4) + 1
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t *r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+      "%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
 
 // The MMA warp accumulates CHUNK K elements at a time in FP32 into one of two
 // TMEM accumulators (ping-pong); the epilogue warps drain every finished chunk
@@ -446,6 +458,8 @@ struct Problem {
   int mfast;             // tile order: m tile fastest (else n tile fastest)
   int nseg, chunk;
   int kt0[kMaxSeg + 1];  // segment s owns global k tiles [kt0[s], kt0[s+1])
+  int klast[kMaxSeg];    // 16-wide K steps of segment s's last k tile (1 .. TBK / 16)
+  int brows;             // rows of a B copy box: the tile width, less for a narrower output
   // batched problem: nbatch entries (row windows of the parents, output
   // offsets) in device memory, or nullptr
   const BatchEntry *batch;
@@ -565,78 +579,121 @@ __device__ __forceinline__ StageAt stage_at(const Problem &P, const TileRef &T,
   return s;
 }
 
-// Epilogue of the wide tiles (one accumulation chunk per tile, FP32 output):
-// each thread loads its row's 128 columns from TMEM (four 32-column loads),
-// hands the buffer back to the MMA thread, then writes them: plain stores for
-// beta = 0, one RED per element for beta = 1 (every element has one owner,
-// so the sum equals load + add + store).  Same arithmetic as the chunked
-// epilogue: (float)(alpha * (double)acc).
+// Epilogue of the wide tiles (one accumulation chunk per tile, FP32 output).
+// The live columns are divided between a quadrant's two warps in multiples of
+// 32; a warp loads its columns from TMEM, hands the buffer back to the MMA
+// thread, then writes: (float)(alpha * (double)acc), stores for beta = 0, one
+// RED per element for beta = 1 (every element has one owner, so the sum
+// equals load + add + store).
+// Unit m stride: a lane holds one row, so a column's 32 rows are one access.
+// Unit n stride (stores only): the columns are loaded as product fragments,
+// so an access covers 8 rows x 8 columns and writes whole 32-byte sectors (a
+// row per lane would touch 32 sectors with 4 or 16 bytes each).
+// This code was the bound of the (T) class launches: about 24 instructions
+// per column (the view walk, two conversions and an FP64 product, dead
+// columns) on 2 warps per SM sub-partition took 24k cycles per tile, the
+// tensor pipe busy for 8.7k of them (v = 170, o = 4: 440 us per accumulating
+// launch and 650 us for the storing one).
 template <int CG, int BN>
 __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep, uint32_t tmem,
                                               uint64_t *acc_full, uint64_t *acc_empty,
                                               int *abort_flag, double alpha, double beta,
                                               int q, int half, int lane) {
-  constexpr int kC = epi_cols<BN>();  // columns per thread
-  const int row = q * 32 + lane;
+  constexpr int kC = epi_cols<BN>();  // columns per thread, at most
+  static_assert(kC == 128, "two warps per quadrant, up to 128 columns each");
+  const bool unit = alpha == 1.0;
+  auto scaled = [&](uint32_t x) {
+    return unit ? __uint_as_float(x) : (float)(alpha * (double)__uint_as_float(x));
+  };
   int gc = 0;
   for (int t = t0; t < L.nTiles; t += tstep, ++gc) {
     const TileRef T = decode_tile<CG, BN>(L, t);
     const Problem &P = L.prob[T.g];
+    const CView &C = P.C;
     const int b = gc % kNAcc;
     const bool w = mbar_wait_g<CG>(smem_u32(&acc_full[b]), (gc / kNAcc) & 1);
     if (!w) atomicExch(&g_tc_status, 4);
     if (!__all_sync(0xffffffffu, w && !*(volatile int *)abort_flag)) return;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int nb = T.n0 + half * kC;
-    const int ncol = min(kC, P.N - nb);  // live columns (may be <= 0)
-    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + half * kC);
+    const int live = min(BN, P.N - T.n0), per = (live + 63) / 64 * 32;
+    const int c0 = half * per, ncol = min(per, live - c0);  // ncol may be <= 0
+    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c0);
+    const bool frag = C.sm0 != 1;  // unit n stride (checked by the host)
     uint32_t r[kC / 32][32];
+    if (frag) {
 #pragma unroll
-    for (int h = 0; h < kC / 32; ++h)
-      if (ncol > h * 32) tmem_ld32(tbase + h * 32, r[h]);  // warp-uniform condition
+      for (int h = 0; h < kC / 32; ++h)
+        if (ncol > h * 32) {  // warp-uniform condition
+          tmem_ld_frag32(tbase + h * 32, r[h]);
+          tmem_ld_frag32(tbase + (16u << 16) + h * 32, r[h] + 16);
+        }
+    } else {
+#pragma unroll
+      for (int h = 0; h < kC / 32; ++h)
+        if (ncol > h * 32) tmem_ld32(tbase + h * 32, r[h]);
+    }
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
-    const int m = T.m0 + row;
-    if (m >= P.M || ncol <= 0) continue;
-    const CView &C = P.C;
-    float *const cm = reinterpret_cast<float *>(C.p) +
-                      (P.batch ? __ldg(&P.batch[T.b].coff) : 0LL) +
-                      cview_dim(C.mdiv, C.sm1, C.sm0, m);
-    CViewNWalk wk(C, nb);
-    float *const c0 = cm + wk.off;  // column nb
-    if (beta == 0.0 && C.ndiv > 0x7fffffff && C.sn0 == 1 && ((uintptr_t)c0 & 15) == 0) {
-      // unit n stride: the thread's columns are contiguous, 16-byte stores
+    float *const base = reinterpret_cast<float *>(C.p) +
+                        (P.batch ? __ldg(&P.batch[T.b].coff) : 0LL);
+    const int nb = T.n0 + c0;
+    if (frag) {
+      const int rr = T.m0 + q * 32 + (lane >> 2), cc = 2 * (lane & 3);
 #pragma unroll
-      for (int h = 0; h < kC / 32; ++h)
+      for (int u = 0; u < 4; ++u) {  // rows rr, rr + 8, rr + 16, rr + 24
+        const int m = rr + 8 * u;
+        if (m >= P.M) break;
+        float *const row = base + cview_dim(C.mdiv, C.sm1, C.sm0, m) + nb + cc;
+        const bool pair = ((uintptr_t)row & 7) == 0;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const int c = h * 32 + j;
-          float x[4];
+        for (int h = 0; h < kC / 32; ++h)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) x[u] = (float)(alpha * (double)__uint_as_float(r[h][j + u]));
-          if (c + 3 < ncol) {
-            *reinterpret_cast<float4 *>(c0 + c) = make_float4(x[0], x[1], x[2], x[3]);
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (c + u < ncol) c0[c + u] = x[u];
+          for (int g = 0; g < 4; ++g) {
+            const int c = h * 32 + g * 8, k = (u >> 1) * 16 + 4 * g + 2 * (u & 1);
+            if (c + cc >= ncol) continue;
+            const float x = scaled(r[h][k]), y = scaled(r[h][k + 1]);
+            if (pair && c + cc + 1 < ncol) {
+              *reinterpret_cast<float2 *>(row + c) = make_float2(x, y);
+            } else {
+              row[c] = x;
+              if (c + cc + 1 < ncol) row[c + 1] = y;
+            }
           }
-        }
-    } else if (beta == 0.0) {
+      }
+      continue;
+    }
+    const int m = T.m0 + q * 32 + lane;
+    if (m >= P.M || ncol <= 0) continue;
+    float *const cm = base + cview_dim(C.mdiv, C.sm1, C.sm0, m);
+    if (C.ndiv > 0x7fffffff) {  // one column stride
+      float *p = cm + (long long)nb * C.sn0;
+      if (beta == 0.0) {
 #pragma unroll
-      for (int h = 0; h < kC / 32; ++h)
+        for (int h = 0; h < kC / 32; ++h)
 #pragma unroll
-        for (int j = 0; j < 32; ++j, wk.next())
-          if (h * 32 + j < ncol) cm[wk.off] = (float)(alpha * (double)__uint_as_float(r[h][j]));
+          for (int j = 0; j < 32; ++j, p += C.sn0)
+            if (h * 32 + j < ncol) *p = scaled(r[h][j]);
+      } else {
+#pragma unroll
+        for (int h = 0; h < kC / 32; ++h)
+#pragma unroll
+          for (int j = 0; j < 32; ++j, p += C.sn0)
+            if (h * 32 + j < ncol) atomicAdd(p, scaled(r[h][j]));
+      }
     } else {
+      CViewNWalk wk(C, nb);
 #pragma unroll
       for (int h = 0; h < kC / 32; ++h)
 #pragma unroll
         for (int j = 0; j < 32; ++j, wk.next())
-          if (h * 32 + j < ncol)
-            atomicAdd(cm + wk.off, (float)(alpha * (double)__uint_as_float(r[h][j])));
+          if (h * 32 + j < ncol) {
+            if (beta == 0.0)
+              cm[wk.off] = scaled(r[h][j]);
+            else
+              atomicAdd(cm + wk.off, scaled(r[h][j]));
+          }
     }
   }
 }
@@ -760,7 +817,8 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
         const int sg = sa.sg, kx = sa.kx, ya = sa.ya, yb = sa.yb;
         if (el) {
           // a pair's stage completes on rank 0's barrier, armed with both halves
-          if (rank == 0) mbar_expect_tx(fb, CG * kStage);
+          if (rank == 0)
+            mbar_expect_tx(fb, CG == 1 ? 2 * TILE_A + 2 * P.brows * kRowBytes : CG * kStage);
           if (CG == 1) {
             tma_load_2d(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb);
             tma_load_2d(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb);
@@ -806,8 +864,11 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
     for (int t = t0; t < nTiles && !stop; t += tstep) {
       const TileRef T = decode_tile<CG, BN>(L, t);
       const int kTiles = T.kTiles, chunk = L.prob[T.g].chunk;
-      const uint32_t idesc = idesc_for<CG, BN>(L.prob[T.g].N - T.n0);
+      const Problem &P = L.prob[T.g];
+      const uint32_t idesc = idesc_for<CG, BN>(P.N - T.n0);
       int kin = 0;  // k tile inside the accumulation chunk
+      int sg = 0;   // K segment of the k tile
+      while (sg + 1 < P.nseg && T.ktb >= P.kt0[sg + 1]) ++sg;
       for (int kt = 0; kt < kTiles; ++kt) {
         bool w = true;
         if (kin == 0) {  // a new chunk: its accumulator has been drained
@@ -830,14 +891,25 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
         const uint64_t dah = d0 + (uint64_t)(s * (kStage >> 4)), dal = dah + (TILE_A >> 4),
                        dbh = dah + (2 * TILE_A >> 4), dbl = dbh + (kTileB >> 4);
         const bool last = ++kin == chunk || kt == kTiles - 1;
+        // the K steps past the segment's end are zero in both operands
+        int steps = TBK / 16;
+        if (T.ktb + kt + 1 == P.kt0[sg + 1]) {
+          steps = P.klast[sg];
+          if (sg + 1 < P.nseg) ++sg;
+        }
         if (el) {
-#pragma unroll
-          for (int kk = 0; kk < TBK / 16; ++kk) {
+          auto product = [&](int kk) {
             const uint64_t o = 2 * kk;
-            const uint32_t acc = (kin > 1 || kk > 0) ? 1u : 0u;
-            umma<CG>(acc_t, dah + o, dbh + o, idesc, acc);
+            umma<CG>(acc_t, dah + o, dbh + o, idesc, (kin > 1 || kk > 0) ? 1u : 0u);
             umma<CG>(acc_t, dah + o, dbl + o, idesc, 1u);
             umma<CG>(acc_t, dal + o, dbh + o, idesc, 1u);
+          };
+          if (steps == TBK / 16) {
+#pragma unroll
+            for (int kk = 0; kk < TBK / 16; ++kk) product(kk);
+          } else {
+#pragma unroll 1
+            for (int kk = 0; kk < steps; ++kk) product(kk);
           }
           umma_commit<CG>(smem_u32(&empty[s]));
           if (last) umma_commit<CG>(smem_u32(&acc_full[b]));
@@ -1170,6 +1242,7 @@ int set_problem(Launch &L, int g, const SplitOperand *A, const SplitOperand *B, 
   P.N = N;
   P.nseg = nseg;
   P.kt0[0] = 0;
+  P.brows = cg == 1 ? std::min(bn, (N + 15) / 16 * 16) : bn;
   for (int s = 0; s < nseg; ++s) {
     const SplitOperand &a = A[s], &b = B[s];
     if (a.k_pad != b.k_pad || a.rows < M || b.rows < N || a.k_pad % TBK || a.rows_pad < M ||
@@ -1181,9 +1254,10 @@ int set_problem(Launch &L, int g, const SplitOperand *A, const SplitOperand *B, 
     const int kk = std::min(a.k, b.k) > 0 ? std::min(a.k, b.k) : a.k_pad;
     ACES_TRY(make_map(&L.ah[g][s], a.hi, a.rows_pad, a.k_pad, kk, TBM));
     ACES_TRY(make_map(&L.al[g][s], a.lo, a.rows_pad, a.k_pad, kk, TBM));
-    ACES_TRY(make_map(&L.bh[g][s], b.hi, b.rows_pad, b.k_pad, kk, bn / cg));
-    ACES_TRY(make_map(&L.bl[g][s], b.lo, b.rows_pad, b.k_pad, kk, bn / cg));
+    ACES_TRY(make_map(&L.bh[g][s], b.hi, b.rows_pad, b.k_pad, kk, P.brows / cg));
+    ACES_TRY(make_map(&L.bl[g][s], b.lo, b.rows_pad, b.k_pad, kk, P.brows / cg));
     P.kt0[s + 1] = P.kt0[s] + a.k_pad / TBK;
+    P.klast[s] = std::max(1, std::min(TBK / 16, (kk - (a.k_pad - TBK) + 15) / 16));
   }
   for (int s = nseg + 1; s <= kMaxSeg; ++s) P.kt0[s] = P.kt0[nseg];
   P.kTilesTotal = P.kt0[nseg];
