@@ -247,7 +247,7 @@ class Lib:
         self._chk("aces_set_tc_pairs", self.h.aces_set_tc_pairs(int(on)))
 
     def set_tc_wide(self, on):
-        """Tile width of the single-chunk FP32-output launches: 1 = 128 x 256
+        """Tile width of the single-chunk FP32-output launches: 1 = 256 x 192
         (aces_set_tc_wide, default), 0 = 128 x 144."""
         self._chk("aces_set_tc_wide", self.h.aces_set_tc_wide(int(on)))
 

@@ -207,10 +207,10 @@ int tc_set_wait_limit(unsigned long long ns);
 int tc_set_inject(int on);
 // launches of products with >= 256 rows on CTA pairs (process-wide)
 void tc_set_pairs(int on);
-// 128 x 256 tiles for the single-chunk FP32-output launches (process-wide)
+// 256 x 192 tiles for the single-chunk FP32-output launches (process-wide)
 void tc_set_wide(int on);
 // whether a batched FP32-output launch over these K segments with N output
-// columns runs on the 128 x 256 tiles (the knob is on, 144 < N <= 256 and
+// columns runs on the 256 x 192 tiles (the knob is on, 144 < N <= 192 and
 // the segments' k tiles form one chunk)
 bool bf16x3_wide_applies(const SplitOperand *A, int nseg, int N);
 // tile autotuner of the tensor-core launches (process-wide switch; choices

@@ -15,11 +15,11 @@
 //             thread one output row x 48, 64 or 128 columns, accumulated in
 //             FP64 across K chunks
 // Three variants: one CTA per 128 x 144 output tile (14 warps, 3-stage
-// mbarrier pipeline; the default), one CTA per 128 x 256 tile for launches
-// whose tiles are single FP32-output chunks (10 warps, 2 stages), and for
-// products of at least 256 rows a cluster pair of CTAs per 256 x 128 tile
-// (tcgen05 cta_group::2, 10 warps, 4 stages), which halves each CTA's share
-// of the B tile.  No copy uses cluster multicast.
+// mbarrier pipeline; the default), a cluster pair of CTAs (tcgen05
+// cta_group::2) per 256 x 192 tile for launches whose tiles are single
+// FP32-output chunks (10 warps, 4 stages), and for products of at least 256
+// rows a pair per 256 x 128 tile (10 warps, 4 stages; off by default).  A pair
+// halves each CTA's share of the B tile.  No copy uses cluster multicast.
 // Every mbarrier wait is bounded by a %globaltimer limit; on expiry the
 // kernel records an error code in g_tc_status, drains its own TMA copies,
 // waits for its issued products, releases TMEM and returns.
@@ -142,11 +142,11 @@ struct Geom {
   static constexpr int kBarArea = 512;
   static constexpr int kStages = (kSmemLimit - 1024 - kBarArea) / kStage;
   static constexpr int kSmem = kStages * kStage + 1024 + kBarArea;  // + alignment + barriers
-  static_assert(kSmem <= kSmemLimit && kStages >= (BN > 160 ? 2 : 3), "pipeline depth");
+  static_assert(kSmem <= kSmemLimit && kStages >= 3, "pipeline depth");
   static_assert(3 * kStages * 8 + 64 + 8 <= kBarArea, "barrier area");
 };
 // (3 stages at TBK 64 or 6/7 at TBK 32 for one CTA per tile, 4 at TBK 64 for
-// pairs, 2 of 96 KB for the 128 x 256 tiles)
+// both kinds of pairs)
 // k tiles per FP32 accumulation chunk, by the contraction length K: 512 K
 // elements up to K = 36864, 256 up to 73728, 128 beyond
 inline int chunk_for(int kTilesTotal) {
@@ -163,14 +163,18 @@ template <int BN>
 constexpr int epi_cols() { return 4 * BN / epi_warps<BN>(); }  // columns per epilogue thread
 template <int BN>
 constexpr int block_threads() { return 32 * (2 + epi_warps<BN>()); }
-static_assert(epi_cols<128>() == 64 && epi_cols<144>() == 48 && epi_cols<256>() == 128,
+// Wide tiles (256 x 192, a CTA pair): products whose every tile is a single
+// accumulation chunk with FP32 output (the batched (T) classes: one tile across
+// N = v <= 192).  No FP64 chunk sums to hold, so the epilogue streams the TMEM
+// columns straight to the output.  Their K is short (8 k tiles), so the copies'
+// latency bounds them: with one CTA per 128 x 256 tile only two stages of
+// 96 KB fit, and a k tile took 2600 cycles against the 1056 of its products; a
+// pair shares B, which leaves 56 KB per CTA and stage and four stages.
+constexpr int TBN_WIDE = 192;
+constexpr int kWideTag = 256;   // the wide variant in a launch's bn and in saved tile choices
+static_assert(epi_cols<TBN>() == 64 && epi_cols<TBN_1>() * epi_warps<TBN_1>() == 4 * TBN_1 &&
+                  epi_cols<TBN_WIDE>() == 96,
               "epilogue column spans");
-// Wide tiles (128 x 256, one CTA): products whose every tile is a single
-// accumulation chunk with FP32 output (the batched (T) classes) -- no FP64
-// chunk sums to hold, so the epilogue streams the 256 TMEM columns straight
-// to the output, and each tcgen05.mma carries N = 256 (half the instructions
-// of the 128-wide tile for the same products).
-constexpr int TBN_WIDE = 256;
 #ifndef ACES_TC_WIDE
 #define ACES_TC_WIDE 1
 #endif
@@ -459,7 +463,8 @@ struct Problem {
   int nseg, chunk;
   int kt0[kMaxSeg + 1];  // segment s owns global k tiles [kt0[s], kt0[s+1])
   int klast[kMaxSeg];    // 16-wide K steps of segment s's last k tile (1 .. TBK / 16)
-  int brows;             // rows of a B copy box: the tile width, less for a narrower output
+  int brows;             // rows of B a k tile copies (a pair: half per CTA): the tile
+                         // width, less for a narrower output
   // batched problem: nbatch entries (row windows of the parents, output
   // offsets) in device memory, or nullptr
   const BatchEntry *batch;
@@ -476,8 +481,8 @@ struct Launch {
   Problem prob[kMaxProb];
   int nprob, nTiles;
   int cg;  // CTAs per tile: 1, or 2 (a cluster pair on 256 x 128 tiles)
-  int bn;  // tile width: TBN_1 (one CTA), TBN (CTA pair), TBN_WIDE (one CTA,
-           // single-chunk FP32 output)
+  int bn;  // tile width: TBN_1 (one CTA), TBN (CTA pair), kWideTag (CTA pair,
+           // TBN_WIDE columns, single-chunk FP32 output)
 };
 struct TileRef {
   int g, m0, n0, z, ktb, kTiles, b;
@@ -598,9 +603,9 @@ template <int CG, int BN>
 __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep, uint32_t tmem,
                                               uint64_t *acc_full, uint64_t *acc_empty,
                                               int *abort_flag, double alpha, double beta,
-                                              int q, int half, int lane) {
+                                              int q, int half, int lane, uint32_t rank) {
   constexpr int kC = epi_cols<BN>();  // columns per thread, at most
-  static_assert(kC == 128, "two warps per quadrant, up to 128 columns each");
+  static_assert(kC % 32 == 0 && epi_warps<BN>() == 8, "two warps per quadrant");
   const bool unit = alpha == 1.0;
   auto scaled = [&](uint32_t x) {
     return unit ? __uint_as_float(x) : (float)(alpha * (double)__uint_as_float(x));
@@ -635,12 +640,18 @@ __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+    if (lane == 0) {
+      if constexpr (CG == 2)  // rank 0's barrier counts both CTAs' warps
+        mbar_arrive_cluster(mapa_rank(smem_u32(&acc_empty[b]), 0));
+      else
+        mbar_arrive(smem_u32(&acc_empty[b]));
+    }
+    const int m0 = T.m0 + (int)rank * TBM;
     float *const base = reinterpret_cast<float *>(C.p) +
                         (P.batch ? __ldg(&P.batch[T.b].coff) : 0LL);
     const int nb = T.n0 + c0;
     if (frag) {
-      const int rr = T.m0 + q * 32 + (lane >> 2), cc = 2 * (lane & 3);
+      const int rr = m0 + q * 32 + (lane >> 2), cc = 2 * (lane & 3);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {  // rows rr, rr + 8, rr + 16, rr + 24
         const int m = rr + 8 * u;
@@ -664,7 +675,7 @@ __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep
       }
       continue;
     }
-    const int m = T.m0 + q * 32 + lane;
+    const int m = m0 + q * 32 + lane;
     if (m >= P.M || ncol <= 0) continue;
     float *const cm = base + cview_dim(C.mdiv, C.sm1, C.sm0, m);
     if (C.ndiv > 0x7fffffff) {  // one column stride
@@ -717,14 +728,13 @@ __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep
 // any of them it did not arm itself (only after a wait gave up), so neither
 // CTA leaves while a copy of the pair is in flight.
 //
-// BN = 256 (one CTA, 128 x 256 tiles): the launch's every tile is a single
-// accumulation chunk with FP32 output; the epilogue streams each thread's 128
-// TMEM columns to the output (two stages of 96 KB in shared memory).
+// BN = TBN_WIDE: the launch's every tile is a single accumulation chunk with
+// FP32 output (epilogue_wide).
 template <int CG, int BN>
 __global__ void __launch_bounds__(block_threads<BN>(), 1)
     k_gemm_bf16x3(const __grid_constant__ Launch L, double alpha, double beta,
                   double *__restrict__ part) {
-  static_assert((CG == 2 && BN == TBN) || (CG == 1 && (BN == TBN_1 || BN == TBN_WIDE)),
+  static_assert((CG == 2 && (BN == TBN || BN == TBN_WIDE)) || (CG == 1 && BN == TBN_1),
                 "tile variants");
   constexpr int kEpiWarps = epi_warps<BN>(), kCols = epi_cols<BN>();
   constexpr int kPiece = kCols % 32 == 0 ? 32 : 16;  // columns per TMEM load
@@ -818,7 +828,7 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
         if (el) {
           // a pair's stage completes on rank 0's barrier, armed with both halves
           if (rank == 0)
-            mbar_expect_tx(fb, CG == 1 ? 2 * TILE_A + 2 * P.brows * kRowBytes : CG * kStage);
+            mbar_expect_tx(fb, CG * 2 * TILE_A + 2 * P.brows * kRowBytes);
           if (CG == 1) {
             tma_load_2d(smem_u32(st), &L.ah[T.g][sg], kx, ya, fb);
             tma_load_2d(smem_u32(st + 2 * TILE_A), &L.bh[T.g][sg], kx, yb, fb);
@@ -940,7 +950,7 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
     bool ok = true;
     if constexpr (BN == TBN_WIDE)
       epilogue_wide<CG, BN>(L, t0, tstep, tmem, acc_full, acc_empty, abort_flag, alpha, beta, q,
-                            half, lane);
+                            half, lane, rank);
     for (int t = t0; t < nTiles && ok && BN != TBN_WIDE; t += tstep) {
       const TileRef T = decode_tile<CG, BN>(L, t);
       const Problem &P = L.prob[T.g];
@@ -1062,7 +1072,7 @@ __global__ void __launch_bounds__(block_threads<BN>(), 1)
       const int theirs = (int)*(volatile uint32_t *)&peer_issued[0];
       for (int k = mine; k < theirs; ++k) {
         const uint32_t fb = smem_u32(&full[k % kStages]);
-        mbar_expect_tx(fb, kStage);
+        mbar_expect_tx(fb, 2 * TILE_A + 2 * (L.prob[0].brows / 2) * kRowBytes);
         if (!mbar_wait_g<CG>(fb, (k / kStages) & 1)) atomicExch(&g_tc_status, 8);
       }
     }
@@ -1231,7 +1241,7 @@ namespace {
 int set_problem(Launch &L, int g, const SplitOperand *A, const SplitOperand *B, int nseg, int M,
                 int N, const CView &C) {
   const int cg = L.cg == 2 ? 2 : 1;
-  const int bn = cg == 2 ? TBN : (L.bn == TBN_WIDE ? TBN_WIDE : TBN_1);
+  const int bn = L.bn == kWideTag ? TBN_WIDE : (cg == 2 ? TBN : TBN_1);
   if (nseg < 1 || nseg > kMaxSeg) {
     set_error("gemm_nt_bf16x3: %d K segments (1..%d)", nseg, kMaxSeg);
     return ACES_ERR_ARG;
@@ -1242,7 +1252,8 @@ int set_problem(Launch &L, int g, const SplitOperand *A, const SplitOperand *B, 
   P.N = N;
   P.nseg = nseg;
   P.kt0[0] = 0;
-  P.brows = cg == 1 ? std::min(bn, (N + 15) / 16 * 16) : bn;
+  // (a pair's teardown counts the bytes of one box height for every problem)
+  P.brows = cg == 1 || L.nprob == 1 ? std::min(bn, (N + 15) / 16 * 16) : bn;
   for (int s = 0; s < nseg; ++s) {
     const SplitOperand &a = A[s], &b = B[s];
     if (a.k_pad != b.k_pad || a.rows < M || b.rows < N || a.k_pad % TBK || a.rows_pad < M ||
@@ -1272,8 +1283,9 @@ int set_problem(Launch &L, int g, const SplitOperand *A, const SplitOperand *B, 
   return ACES_OK;
 }
 
-// CTA pairs the device keeps resident at once (the pair variant's grid is
+// CTA pairs of BN-wide tiles the device keeps resident at once (the grid is
 // twice that, at most the SM count)
+template <int BN>
 int max_pairs() {
   static int cached[64] = {0};
   int dev = 0;
@@ -1286,19 +1298,36 @@ int max_pairs() {
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(num_sms() & ~1));
-    cfg.blockDim = dim3(block_threads<TBN>());
-    cfg.dynamicSmemBytes = Geom<2>::kSmem;
+    cfg.blockDim = dim3(block_threads<BN>());
+    cfg.dynamicSmemBytes = Geom<2, BN>::kSmem;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16x3<2, TBN>, &cfg) != cudaSuccess ||
-        n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16x3<2, BN>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = num_sms() / 2;
     }
     cached[dev] = std::min(n, num_sms() / 2);
   }
   return cached[dev];
+}
+template <int BN>
+int launch_pairs(const Launch &L, double alpha, double beta, double *part, cudaStream_t st) {
+  const unsigned pairs = (unsigned)std::max(1, std::min(L.nTiles, max_pairs<BN>()));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(block_threads<BN>());
+  cfg.dynamicSmemBytes = Geom<2, BN>::kSmem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ACES_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_bf16x3<2, BN>, L, alpha, beta, part));
+  return ACES_OK;
 }
 
 // The pair variant passes the same tests as the 1-CTA kernel, but on B200 it
@@ -1327,33 +1356,17 @@ int launch_prepared(Launch &L, double alpha, double beta, double *part, cudaStre
                                    Geom<1, TBN_1>::kSmem));
     ACES_CUDA(cudaFuncSetAttribute(k_gemm_bf16x3<2, TBN>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Geom<2>::kSmem));
-    ACES_CUDA(cudaFuncSetAttribute(k_gemm_bf16x3<1, TBN_WIDE>,
+    ACES_CUDA(cudaFuncSetAttribute(k_gemm_bf16x3<2, TBN_WIDE>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   Geom<1, TBN_WIDE>::kSmem));
+                                   Geom<2, TBN_WIDE>::kSmem));
     int zero = 0;
     ACES_CUDA(cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(int)));
     attr[dev] = true;
   }
-  if (L.cg == 2) {
-    const unsigned pairs = (unsigned)std::max(1, std::min(L.nTiles, max_pairs()));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(block_threads<TBN>());
-    cfg.dynamicSmemBytes = Geom<2>::kSmem;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    ACES_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_bf16x3<2, TBN>, L, alpha, beta, part));
-  } else if (L.bn == TBN_WIDE) {
-    const unsigned grid = (unsigned)std::min(L.nTiles, num_sms());
-    k_gemm_bf16x3<1, TBN_WIDE>
-        <<<grid, block_threads<TBN_WIDE>(), Geom<1, TBN_WIDE>::kSmem, st>>>(L, alpha, beta,
-                                                                             part);
+  if (L.bn == kWideTag) {
+    ACES_TRY(launch_pairs<TBN_WIDE>(L, alpha, beta, part, st));
+  } else if (L.cg == 2) {
+    ACES_TRY(launch_pairs<TBN>(L, alpha, beta, part, st));
   } else {
     const unsigned grid = (unsigned)std::min(L.nTiles, num_sms());
     k_gemm_bf16x3<1, TBN_1>
@@ -1372,7 +1385,7 @@ namespace {
 // later products of the class launch the cached variant directly.  Variants:
 // one CTA per 128 x TBN_1 tile or CTA pairs (single and grouped products of
 // >= 256 rows), split K at the wave-efficiency slice count or none (single
-// products), and for batched FP32-output launches 128 x TBN_1 or 128 x 256
+// products), and for batched FP32-output launches 128 x TBN_1 or 256 x 192
 // tiles.  A class is the launch
 // kind, the K segment (or problem) count, FP32 output, eligibility for pairs,
 // and the output tile counts and k tile count rounded to two significant
@@ -1595,7 +1608,7 @@ int multi_run(const TuneChoice &ch, const SplitOperand *A, const SplitOperand *B
   Problem &P = L.prob[0];
   // split K when the output has too few tiles to fill the SMs (CTA pairs)
   const long long tiles = (long long)P.tilesN * P.tilesM;
-  const int nsm = L.cg == 2 ? max_pairs() : num_sms();
+  const int nsm = L.cg == 2 ? max_pairs<TBN>() : num_sms();
   int Z = ch.nosplit ? 1 : split_slices(tiles, P.kTilesTotal, nsm);
   double *part = nullptr;
   if (Z > 1) {
@@ -1674,21 +1687,20 @@ int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOpera
   L.nprob = 1;
   L.cg = ch.cg == 2 ? 2 : 1;
   // FP32 output whose every tile is one accumulation chunk, with 144 < N <=
-  // 256: one wide tile instead of a full and a ragged narrow one.  Where N
-  // fits one narrow tile or is much larger, the 3-stage narrow tiles win
-  // (o = 6, v = 128 class launches against 128-wide tiles: 32 % slower with
-  // N = 128 on wide tiles, 3 % slower with N = 16384)
+  // 192: one wide tile across N instead of a full and a ragged narrow one
+  // (where N fits one narrow tile those are faster: o = 6, v = 128 class
+  // launches ran 32 % slower on 128 x 256 tiles of one CTA)
+  int kt = 0;
+  for (int s = 0; s < nseg; ++s) kt += Apar[s].k_pad / TBK;
+  const bool fits = f32out && N <= TBN_WIDE && kt <= chunk_for(kt);
   if (L.cg == 2)
     L.bn = TBN;
   else if (ch.bn)
-    L.bn = f32out ? ch.bn : TBN_1;
+    L.bn = ch.bn == kWideTag && fits ? kWideTag : TBN_1;
   else
-    L.bn = f32out && N > TBN_1 && N <= TBN_WIDE && g_tc_wide.load() ? TBN_WIDE : TBN_1;
+    L.bn = fits && N > TBN_1 && g_tc_wide.load() ? kWideTag : TBN_1;
+  if (L.bn == kWideTag) L.cg = 2;
   ACES_TRY(set_problem(L, 0, Apar, Bpar, nseg, M, N, C));
-  if (L.bn == TBN_WIDE && L.prob[0].kTilesTotal > L.prob[0].chunk) {
-    L.bn = TBN_1;
-    ACES_TRY(set_problem(L, 0, Apar, Bpar, nseg, M, N, C));
-  }
   Problem &P = L.prob[0];
   P.batch = d_entries;
   P.nbatch = nbatch;
@@ -1863,7 +1875,7 @@ int gemm_nt_bf16x3_batched(const SplitOperand *Apar, const SplitOperand *Bpar, i
   const long long tm = (M + TBM - 1) / TBM, tn = (N + TBN_1 - 1) / TBN_1;
   const TuneKey key{current_device(), 2, nseg,
                     (M >= 2 * TBM ? 1 : 0) | (f32out ? 2 : 0) | (N > TBN_1 ? 4 : 0) |
-                        (N > TBN_WIDE ? 8 : 0),
+                        (N > kWideTag ? 8 : 0),
                     bucket2(tm * nbatch), bucket2(tn), bucket2(kt)};
   TuneChoice ch;
   if (tune_lookup(key, &ch))
@@ -1878,7 +1890,7 @@ int gemm_nt_bf16x3_batched(const SplitOperand *Apar, const SplitOperand *Bpar, i
   std::vector<TuneChoice> cands{def};
   if (def.cg == 1 && f32out && N > TBN_1 && N <= TBN_WIDE && kt <= chunk_for(kt)) {
     TuneChoice c;
-    c.bn = g_tc_wide.load() ? TBN_1 : TBN_WIDE;
+    c.bn = g_tc_wide.load() ? TBN_1 : kWideTag;
     cands.push_back(c);
   }
   if (cands.size() == 1) {
@@ -1990,7 +2002,7 @@ int tc_autotune_load(const char *path) {
         n == 10 && kind >= 0 && kind <= 2 && nseg >= 1 &&
         nseg <= (kind == 1 ? kMaxProb : kMaxSeg) && flags >= 0 && flags <= 15 && v[3] >= 0 &&
         v[4] >= 0 && v[5] >= 0 && (cg == 1 || (cg == 2 && (flags & 1))) &&
-        (bn == 0 || (kind == 2 && (flags & 2) && cg == 1 && (bn == TBN_1 || bn == TBN_WIDE))) &&
+        (bn == 0 || (kind == 2 && (flags & 2) && cg == 1 && (bn == TBN_1 || bn == kWideTag))) &&
         (nosplit == 0 || (nosplit == 1 && kind == 0 && cg == 1)) && (changed == 0 || changed == 1);
     if (!ok) {
       set_error("aces_autotune_load: %s line %d is not a valid tile choice", path, lineno);

@@ -428,7 +428,7 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
     const double budget = std::min(0.25 * (double)fr, 4.0e9);
     const int nb = (int)std::max(1.0, std::min((double)std::max(ntrip, 1), budget / slot));
     ACES_TRY(alloc(Wb, (size_t)((V3 * nb + 1) / 2)));  // FP32 slots in a double buffer
-    // class c runs transposed on the 128 x 256 tiles (M = (a,b), N = c: the
+    // class c runs transposed on the 256 x 192 tiles (M = (a,b), N = c: the
     // ragged side is the one whose MMA N is cut to the live columns, where on
     // 128-row tiles M = c = v would leave 256 - v rows idle), and stores W
     // rows of v contiguous floats

@@ -183,16 +183,16 @@ int aces_debug_inject(int mode);
  * error bound; process-wide. */
 int aces_set_tc_pairs(int on);
 /* Tile width of the tensor-core launches whose every output tile is one
- * accumulation chunk with FP32 output and 144 < N <= 256 (the batched (T)
+ * accumulation chunk with FP32 output and 144 < N <= 192 (the batched (T)
  * classes for 144 < v <= 192; no counterpart in the reference): 1 = one
- * 128 x 256 tile across N (the default), 0 = 128 x 144 tiles.  Same
+ * 256 x 192 tile of a CTA pair across N (the default), 0 = 128 x 144 tiles.  Same
  * arithmetic either way; process-wide. */
 int aces_set_tc_wide(int on);
 /* Tile autotuner of the tensor-core contractions (no counterpart in the
  * reference; the reference's XGEMM calls take whatever its BLAS does).
  * mode 1: the first product of each shape class on a device times the tile
  * variants that apply to it -- one CTA per tile or CTA pairs and split K or
- * not for single and grouped products, 144- or 256-wide tiles for the
+ * not for single and grouped products, 144- or 192-wide tiles for the
  * FP32-output batched (T) launches -- with CUDA
  * events on the product's stream (the call then waits for the device), and
  * later products of the class reuse the fastest; mode 0 (default): the
