@@ -4,7 +4,7 @@
 // For every occupied triplet i >= j >= k the connected triples
 //   W_ijk^abc = sum over the 6 simultaneous permutations of (ia)(jb)(kc) of
 //     X_ijk^abc = sum_d t(ij,ad) (bd|ck) - sum_l t(il,ab) (ck|jl)
-// are built in one v^3 FP64 buffer by three tensor-core launches (the 12
+// are built in a v^3 slot per triplet by three tensor-core launches (the 12
 // contractions grouped by output orientation, four K segments each) whose
 // outputs land in place through coalesced two-level views.  The energy kernel
 // then sums, for the distinct permutations of (i,j,k) and all orderings of
@@ -165,6 +165,8 @@ __device__ __forceinline__ void decode_set(int n, int &a, int &b, int &c) {
 // three distinct virtuals through the constant bilinear form, sets with a
 // repeated virtual through the general per-ordering sum.
 constexpr int kTile = 8;
+// triplets of one FP64 batch (the energy launch's grid.y holds 65535)
+constexpr int kMaxTasks = 32768;
 // kOrd[s][r] in device code: the first position is s / 2, the other two
 // follow in increasing order for even s and swapped for odd s
 __host__ __device__ __forceinline__ constexpr int ordpos(int s, int r) {
@@ -337,7 +339,8 @@ __global__ void __launch_bounds__(1024) k_sum_pairs(double *out, const double *p
 // share the large operand's rows: a window used by several triplets of the
 // batch (Gv[j] for every k of a pair (i,j), Gv[k] across pairs) is read from
 // DRAM about once per launch instead of once per triplet.  Four launches per
-// batch replace four per triplet.  The FP64 path keeps one triplet at a time.
+// batch replace four per triplet.  The FP64 path batches the same way (FP64
+// W slots, task tables of the FP64 contraction kernel).
 int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nranks) {
   const long long O = o, V = v;
   const long long V2 = V * V, V3 = V * V * V;
@@ -492,8 +495,20 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
     }
     nparts = (long long)ntrip * nblk;
   } else {
-    // FP64: one triplet at a time, W in FP64
-    ACES_TRY(alloc(Wb, V3));
+    // FP64: the triplets in batches as above, W in FP64 slots; a class of a
+    // batch is one launch over a table of tasks (four K segments each).  One
+    // triplet at a time took 13 launches of about 10 us each at o = 8, v = 70:
+    // 13.5 ms of kernels and 7 ms of gaps between them.
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+      cudaGetLastError();
+      fr = 0;
+    }
+    const double slot = (double)V3 * sizeof(double);
+    const double budget = std::min(0.25 * (double)fr, 4.0e9);
+    const int nb = (int)std::max(
+        1.0, std::min({(double)std::max(ntrip, 1), budget / slot, (double)kMaxTasks}));
+    ACES_TRY(alloc(Wb, V3 * nb));
     const int nt = (v + kTile - 1) / kTile;
     const int nblk = nt * (nt + 1) * (nt + 2) / 6;
     ACES_TRY(alloc(part, (size_t)std::max(ntrip, 1) * nblk * 2));
@@ -503,43 +518,52 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
     auto GTp = [&](int z) { return GvT.p + (long long)z * V2 * V; };
     auto Pp = [&](int x) { return t2P.p + (long long)x * V2 * O; };
     auto Qp = [&](int x) { return t2Q.p + (long long)x * V2 * O; };
-    // one class: C(view) = beta C + sum_s A_s B_s^T (K = v for the t2 x (bd|ck)
-    // segments, o for the others)
-    auto run_class = [&](const double *const (&A)[4], const double *const (&B)[4], int M, int N,
-                         const CView &cv, double beta) -> int {
+    // C(view) = beta C + sum_s A_s B_s^T (K = v for the t2 x (bd|ck) segments, o
+    // for the others)
+    auto task = [&](const double *const (&A)[4], const double *const (&B)[4], int M, int N,
+                    const CView &view, double *W) {
+      F64Task t{};
+      t.nseg = 4;
+      t.M = M;
+      t.N = N;
+      t.C = view;
+      t.C.p = W;
       for (int g = 0; g < 4; ++g) {
         const int K = g < 2 ? v : o;
-        ACES_TRY(gemm_nt_f64(M, N, K, 1.0, A[g], K, B[g], K, g == 0 ? beta : 1.0, cv, st));
+        t.seg[g] = F64Seg{A[g], B[g], K, K, K};
       }
-      return ACES_OK;
+      return t;
     };
-    for (int t = 0; t < ntrip; ++t) {
-      const int i = trip[3 * t], j = trip[3 * t + 1], k = trip[3 * t + 2];
-      CView cv = vc;
-      cv.p = Wb.p;
-      {
-        const double *const A[4] = {T2p(k, i), T2p(k, j), Hp(j, k), Hp(i, k)};
-        const double *const B[4] = {Gp(j), GTp(i), Pp(i), Qp(j)};
-        ACES_TRY(run_class(A, B, v, v * v, cv, 0.0));
+    std::vector<F64Task> tasks;
+    ACES_TRY(alloc(dent, ((size_t)3 * nb * sizeof(F64Task) + 7) / 8));
+    F64Task *d_tasks = reinterpret_cast<F64Task *>(dent.p);
+    for (int t0b = 0; t0b < ntrip; t0b += nb) {
+      const int n = std::min(nb, ntrip - t0b);
+      tasks.resize((size_t)3 * n);
+      for (int e = 0; e < n; ++e) {
+        const int *x = &trip[3 * (size_t)(t0b + e)], i = x[0], j = x[1], k = x[2];
+        double *W = Wb.p + (size_t)e * V3;
+        tasks[e] = task({T2p(k, i), T2p(k, j), Hp(j, k), Hp(i, k)}, {Gp(j), GTp(i), Pp(i), Qp(j)},
+                        v, v * v, vc, W);
+        tasks[n + e] = task({Gp(k), GTp(j), Pp(j), Qp(k)}, {T2p(i, j), T2p(i, k), Hp(k, i), Hp(j, i)},
+                            v * v, v, va, W);
+        tasks[2 * n + e] = task({Gp(k), GTp(i), Pp(i), Qp(k)},
+                                {T2p(j, i), T2p(j, k), Hp(k, j), Hp(i, j)}, v * v, v, vb, W);
       }
-      cv = va;
-      cv.p = Wb.p;
-      {
-        const double *const A[4] = {Gp(k), GTp(j), Pp(j), Qp(k)};
-        const double *const B[4] = {T2p(i, j), T2p(i, k), Hp(k, i), Hp(j, i)};
-        ACES_TRY(run_class(A, B, v * v, v, cv, 1.0));
-      }
-      cv = vb;
-      cv.p = Wb.p;
-      {
-        const double *const A[4] = {Gp(k), GTp(i), Pp(i), Qp(k)};
-        const double *const B[4] = {T2p(j, i), T2p(j, k), Hp(k, j), Hp(i, j)};
-        ACES_TRY(run_class(A, B, v * v, v, cv, 1.0));
-      }
-      k_triples_energy_tiled<double><<<dim3(nblk, 1), 128, 0, st>>>(
-          Wb.p, 0, d_trip + 3 * t, t1(), I_oovv.p, eo.p, ev.p, o, v,
-          part.p + (size_t)t * nblk * 2);
+      F64TaskPlan plan[3];
+      for (int q = 0; q < 3; ++q)
+        ACES_TRY(f64_tasks_plan(tasks.data() + (size_t)q * n, n, &plan[q]));
+      // the table is read by this batch's launches only: the copy waits for the
+      // previous batch's (stream order), and the host vector is copied out
+      ACES_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(F64Task),
+                                cudaMemcpyHostToDevice, st));
+      for (int q = 0; q < 3; ++q)
+        ACES_TRY(f64_tasks_run(d_tasks + (size_t)q * n, n, plan[q], 1.0, q ? 1.0 : 0.0, st));
+      k_triples_energy_tiled<double><<<dim3(nblk, n), 128, 0, st>>>(
+          Wb.p, V3, d_trip + 3 * (size_t)t0b, t1(), I_oovv.p, eo.p, ev.p, o, v,
+          part.p + (size_t)t0b * nblk * 2);
       count_launch();
+      ACES_CUDA(cudaGetLastError());
     }
     nparts = (long long)ntrip * nblk;
   }
