@@ -15,11 +15,90 @@
 // the adjoints of the Fock blocks recorded in the residual, plus dE/df_ia =
 // 2 t_i^a, plus the denominator terms of the diagonal, so that for a
 // one-electron perturbation f -> f + x h' the derivative dE/dx = Tr(D h').
+#include <algorithm>
 #include <cmath>
 
 #include "engine.cuh"
 
 namespace acesb200 {
+
+namespace {
+// Sums of x = l2 * t2 over one pair block [i,j]: rs[ij][a] = sum_b x[a,b] and
+// cs[ij][b] = sum_a x[a,b].  One block per (ij): its warps take the rows a in
+// turn (rs by a shuffle tree), and every thread keeps the column sums of its
+// columns b = lane + 32 k over the warp's rows, added over the warps in order
+// at the end: all orders are fixed.  Memory bound (two passes of the host
+// loop's 2 o^2 v^2 doubles, which took 38 ms with its copies at o = 16,
+// v = 130).
+constexpr int kDensWarps = 8, kDensCols = 16;   // up to 512 columns per sweep
+__global__ void __launch_bounds__(32 * kDensWarps)
+    k_density_sums(double *__restrict__ rs, double *__restrict__ cs,
+                   const double *__restrict__ l2, const double *__restrict__ t2, int v) {
+  __shared__ double sh[kDensWarps][32 * kDensCols];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long base = (long long)blockIdx.x * v * v;
+  for (int b0 = 0; b0 < v; b0 += 32 * kDensCols) {
+    double col[kDensCols];
+#pragma unroll
+    for (int k = 0; k < kDensCols; ++k) col[k] = 0.0;
+    for (int a = wid; a < v; a += kDensWarps) {
+      double row = 0.0;
+#pragma unroll
+      for (int k = 0; k < kDensCols; ++k) {
+        const int b = b0 + lane + 32 * k;
+        if (b < v) {
+          const long long e = base + (long long)a * v + b;
+          const double x = l2[e] * t2[e];
+          row += x;
+          col[k] += x;
+        }
+      }
+      for (int off = 16; off; off >>= 1) row += __shfl_down_sync(0xffffffffu, row, off);
+      if (lane == 0) {
+        double *r = rs + (long long)blockIdx.x * v + a;
+        *r = b0 == 0 ? row : *r + row;
+      }
+    }
+    __syncthreads();  // the previous sweep's reads are done
+#pragma unroll
+    for (int k = 0; k < kDensCols; ++k) sh[wid][lane + 32 * k] = col[k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < 32 * kDensCols && b0 + c < v; c += 32 * kDensWarps) {
+      double t = 0.0;
+      for (int w = 0; w < kDensWarps; ++w) t += sh[w][c];
+      cs[(long long)blockIdx.x * v + b0 + c] = t;
+    }
+  }
+}
+
+// diag[a] = sum_ij rs[ij][a] + cs[ij][a] (a < v; one block each), and
+// diag[v + i] = -sum_ja (rs[ij][a] + rs[ji][a]) (i < o)
+__global__ void __launch_bounds__(256)
+    k_density_diag(double *__restrict__ diag, const double *__restrict__ rs,
+                   const double *__restrict__ cs, int o, int v) {
+  __shared__ double sh[8];
+  double t = 0.0;
+  if ((int)blockIdx.x < v) {
+    const int a = blockIdx.x;
+    for (int ij = threadIdx.x; ij < o * o; ij += 256)
+      t += rs[(long long)ij * v + a] + cs[(long long)ij * v + a];
+  } else {
+    const int i = blockIdx.x - v;
+    for (int e = threadIdx.x; e < o * v; e += 256) {
+      const int j = e / v, a = e - j * v;
+      t -= rs[((long long)i * o + j) * v + a] + rs[((long long)j * o + i) * v + a];
+    }
+  }
+  for (int off = 16; off; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t = 0.0;
+    for (int w = 0; w < 8; ++w) t += sh[w];
+    diag[blockIdx.x] = t;
+  }
+}
+}  // namespace
 
 int CCEngine::record_residual(bool fock_active) {
   // the forward values the previous tape's backward pass cached may change
@@ -66,14 +145,29 @@ int CCEngine::density(std::vector<double> &D) {
   launch_axpy(z1b, L.p, 1.0, ov, st);
   launch_axpy(z2b, L.p + ov, 1.0, len - ov, st);
   ACES_TRY(backward());
+  // doubles part of the diagonal, -lambda . d(D o T)/d e_p, on the device
+  DBuf sums;
+  struct Release {
+    DBuf &b;
+    ~Release() { if (b.p) dev_free(b.p); }
+  } release{sums};
+  const size_t nsum = (size_t)o * o * v;
+  ACES_TRY(alloc(sums, 2 * nsum + o + v));
+  double *rs = sums.p, *cs = rs + nsum, *dg = cs + nsum;
+  k_density_sums<<<o * o, 32 * kDensWarps, 0, st>>>(rs, cs, L.p + ov, X.p + ov, v);
+  count_launch();
+  k_density_diag<<<o + v, 256, 0, st>>>(dg, rs, cs, o, v);
+  count_launch();
+  ACES_CUDA(cudaGetLastError());
   std::vector<double> aoo((size_t)o * o), avv((size_t)v * v), aov((size_t)ov), avo((size_t)ov),
-      t(len), l(len);
+      t((size_t)ov), l((size_t)ov), diag((size_t)(o + v));
   ACES_CUDA(cudaMemcpyAsync(aoo.data(), adj(offo.p), aoo.size() * 8, cudaMemcpyDeviceToHost, st));
   ACES_CUDA(cudaMemcpyAsync(avv.data(), adj(offv.p), avv.size() * 8, cudaMemcpyDeviceToHost, st));
   ACES_CUDA(cudaMemcpyAsync(aov.data(), adj(fov.p), aov.size() * 8, cudaMemcpyDeviceToHost, st));
   ACES_CUDA(cudaMemcpyAsync(avo.data(), adj(fovT.p), avo.size() * 8, cudaMemcpyDeviceToHost, st));
-  ACES_CUDA(cudaMemcpyAsync(t.data(), X.p, len * 8, cudaMemcpyDeviceToHost, st));
-  ACES_CUDA(cudaMemcpyAsync(l.data(), L.p, len * 8, cudaMemcpyDeviceToHost, st));
+  ACES_CUDA(cudaMemcpyAsync(t.data(), X.p, ov * 8, cudaMemcpyDeviceToHost, st));
+  ACES_CUDA(cudaMemcpyAsync(l.data(), L.p, ov * 8, cudaMemcpyDeviceToHost, st));
+  ACES_CUDA(cudaMemcpyAsync(diag.data(), dg, diag.size() * 8, cudaMemcpyDeviceToHost, st));
   ACES_CUDA(cudaStreamSynchronize(st));
   D.assign((size_t)nmo * nmo, 0.0);
   auto at = [&](int p, int q) -> double & { return D[(size_t)p * nmo + q]; };
@@ -86,26 +180,14 @@ int CCEngine::density(std::vector<double> &D) {
   for (int i = 0; i < o; ++i)
     for (int a = 0; a < v; ++a)
       at(i, o + a) = aov[(size_t)i * v + a] + avo[(size_t)a * o + i] + 2.0 * t[(size_t)i * v + a];
-  // diagonal: -lambda . d(D o T)/d e_p
-  const double *t1 = t.data(), *l1 = l.data(), *t2 = t.data() + ov, *l2 = l.data() + ov;
-  std::vector<double> occ(o, 0.0), vir(v, 0.0);
+  // diagonal: the singles' part on top of the doubles'
+  std::vector<double> occ(diag.begin() + v, diag.end()), vir(diag.begin(), diag.begin() + v);
   for (int i = 0; i < o; ++i)
     for (int a = 0; a < v; ++a) {
-      double x = l1[(size_t)i * v + a] * t1[(size_t)i * v + a];
+      const double x = l[(size_t)i * v + a] * t[(size_t)i * v + a];
       occ[i] -= x;
       vir[a] += x;
     }
-  for (int i = 0; i < o; ++i)
-    for (int j = 0; j < o; ++j)
-      for (int a = 0; a < v; ++a)
-        for (int b = 0; b < v; ++b) {
-          size_t k = (((size_t)i * o + j) * v + a) * v + b;
-          double x = l2[k] * t2[k];
-          occ[i] -= x;
-          occ[j] -= x;
-          vir[a] += x;
-          vir[b] += x;
-        }
   for (int i = 0; i < o; ++i) at(i, i) = occ[i];
   for (int a = 0; a < v; ++a) at(o + a, o + a) = vir[a];
   return ACES_OK;
