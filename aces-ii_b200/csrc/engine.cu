@@ -59,6 +59,10 @@ void CCEngine::release() {
     if (t.hi) dev_free(t.hi);
     t = SplitOperand();
   }
+  for (SplitOperand *t : {&sUp, &sUm}) {
+    if (t->hi) dev_free(t->hi);
+    *t = SplitOperand();
+  }
   split_tmpA = SplitOperand();
   split_tmpB = SplitOperand();
   for (auto &m : memo)
@@ -1107,7 +1111,10 @@ int CCEngine::ladder_packed_blocks(const double *in, double *out) {
 int CCEngine::ladder_packed(const double *in, double *out) {
   if (state().sym.nirrep > 1) return ladder_packed_blocks(in, out);
   const int np = v * (v + 1) / 2, nm = v * (v - 1) / 2, oo = o * o;
-  if (!Up.p) {
+  // both products on the tensor cores: U+- and tau+- go straight into the
+  // planes of their operands
+  const bool sp = nm > 0 && splits(np, oo, np) && splits(nm, oo, nm);
+  if (!ladpairs.p) {
     // pair tables: p(c,d) = d(d+1)/2 + c (c <= d), m(c,d) = d(d-1)/2 + c (c < d)
     std::vector<int> pr((size_t)2 * (np + nm));
     for (int d = 0; d < v; ++d)
@@ -1124,6 +1131,40 @@ int CCEngine::ladder_packed(const double *in, double *out) {
     ACES_TRY(alloc(ladpairs, (pr.size() + 1) / 2));
     ACES_CUDA(cudaMemcpyAsync(ladpairs.p, pr.data(), pr.size() * sizeof(int),
                               cudaMemcpyHostToDevice, st));
+    ACES_CUDA(cudaStreamSynchronize(st));
+  }
+  auto planes_of = [](const SplitOperand &p, const SplitOperand &m) {
+    LadderPlanes pl;
+    pl.hi_p = (__nv_bfloat16 *)p.hi;
+    pl.lo_p = (__nv_bfloat16 *)p.lo;
+    pl.hi_m = (__nv_bfloat16 *)m.hi;
+    pl.lo_m = (__nv_bfloat16 *)m.lo;
+    pl.kp_p = p.k_pad;
+    pl.kp_m = m.k_pad;
+    return pl;
+  };
+  if (sp && !sUm.hi) {
+    // (the tensor maps end at the true K, so the K padding is never read)
+    for (int q = 0; q < 2; ++q) {
+      SplitOperand &u = q ? sUm : sUp;
+      const int n = q ? nm : np, kp = (n + kSplitKPad - 1) / kSplitKPad * kSplitKPad;
+      if (!u.hi) {
+        const size_t bytes = (size_t)n * kp * 2 * 2;
+        if (dev_alloc(&u.hi, bytes) != cudaSuccess) {
+          u.hi = nullptr;
+          set_error("engine: device allocation of %zu bytes failed", bytes);
+          return ACES_ERR_NOMEM;
+        }
+        u.cap = bytes;
+      }
+      u.rows = u.rows_pad = u.k = n;
+      u.k_pad = kp;
+      u.lo = (char *)u.hi + (size_t)n * kp * 2;
+    }
+    const LadderPlanes pl = planes_of(sUp, sUm);
+    launch_ladder_pack_v(nullptr, nullptr, I_vvvv.p, (const int *)ladpairs.p, v, st, &pl);
+    ACES_CUDA(cudaGetLastError());
+  } else if (!sp && !Up.p) {
     ACES_TRY(alloc(Up, (size_t)np * np));
     ACES_TRY(alloc(Um, (size_t)std::max(nm, 1) * std::max(nm, 1)));
     launch_ladder_pack_v(Up.p, Um.p, I_vvvv.p, (const int *)ladpairs.p, v, st);
@@ -1135,29 +1176,38 @@ int CCEngine::ladder_packed(const double *in, double *out) {
   ACES_TRY(alloc(Ald, (size_t)oo * std::max(nm, 1)));
   memo_written(taup.p, (long long)oo * np);
   memo_written(taum.p, (long long)oo * std::max(nm, 1));
-  if (memo_on && nm > 0 && splits(np, oo, np) && splits(nm, oo, nm)) {
-    // inside a residual pass whose grouped launch splits: tau+- straight
-    // into the planes of its B operands, no FP64 copy
-    MemoEntry *mp = nullptr, *mm = nullptr;
-    ACES_TRY(memo_planes(taup.p, oo, np, &mp));
-    ACES_TRY(memo_planes(taum.p, oo, nm, &mm));
-    LadderPlanes pl;
-    pl.hi_p = (__nv_bfloat16 *)mp->op.hi;
-    pl.lo_p = (__nv_bfloat16 *)mp->op.lo;
-    pl.hi_m = (__nv_bfloat16 *)mm->op.hi;
-    pl.lo_m = (__nv_bfloat16 *)mm->op.lo;
-    pl.kp_p = mp->op.k_pad;
-    pl.kp_m = mm->op.k_pad;
-    launch_ladder_pack_tau(taup.p, taum.p, in, v, oo, st, &pl);
-    mp->valid = mm->valid = true;
-    mp->fp64 = mm->fp64 = false;
+  // both products in one grouped launch (their tiles fill each other's last wave)
+  if (sp) {
+    const SplitOperand *tp = &split_tmpG[1], *tm = &split_tmpG[3];
+    if (memo_on) {
+      MemoEntry *mp = nullptr, *mm = nullptr;
+      ACES_TRY(memo_planes(taup.p, oo, np, &mp));
+      ACES_TRY(memo_planes(taum.p, oo, nm, &mm));
+      const LadderPlanes pl = planes_of(mp->op, mm->op);
+      launch_ladder_pack_tau(taup.p, taum.p, in, v, oo, st, &pl);
+      mp->valid = mm->valid = true;
+      mp->fp64 = mm->fp64 = false;
+      tp = &mp->op;
+      tm = &mm->op;
+    } else {
+      launch_ladder_pack_tau(taup.p, taum.p, in, v, oo, st);
+      ACES_TRY(split_pack(split_tmpG[1], taup.p, np, oo, np, st));
+      ACES_TRY(split_pack(split_tmpG[3], taum.p, nm, oo, nm, st));
+    }
+    memo_written(Sld.p, (long long)oo * np);
+    memo_written(Ald.p, (long long)oo * nm);
+    gemm_calls += 2;
+    gemm_flops += 2.0 * oo * ((double)np * np + (double)nm * nm);
+    const GroupedProblem pr[2] = {{&sUp, tp, 1, np, oo, cview_colmajor(Sld.p, np)},
+                                  {&sUm, tm, 1, nm, oo, cview_colmajor(Ald.p, nm)}};
+    ACES_TRY(gemm_nt_bf16x3_grouped(pr, 2, 1.0, 0.0, st));
   } else {
     launch_ladder_pack_tau(taup.p, taum.p, in, v, oo, st);
+    const GArgs g[2] = {
+        {np, oo, np, Up.p, np, taup.p, np, cview_colmajor(Sld.p, np), true, false},
+        {nm, oo, nm, Um.p, nm, taum.p, nm, cview_colmajor(Ald.p, nm), true, false}};
+    ACES_TRY(Ggroup(g, nm > 0 ? 2 : 1, 0.0));
   }
-  // both products in one grouped launch (their tiles fill each other's last wave)
-  const GArgs g[2] = {{np, oo, np, Up.p, np, taup.p, np, cview_colmajor(Sld.p, np), true, false},
-                      {nm, oo, nm, Um.p, nm, taum.p, nm, cview_colmajor(Ald.p, nm), true, false}};
-  ACES_TRY(Ggroup(g, nm > 0 ? 2 : 1, 0.0));
   memo_written(out, (long long)o * o * v * v);
   launch_ladder_unpack(out, Sld.p, Ald.p, v, oo, st);
   ACES_CUDA(cudaGetLastError());

@@ -64,6 +64,7 @@ class CCEngine {
       WmnT, t1T, Fae, Fmi, Fme, Fp, Fpp, FmiT, FppT, FmeT, tmp4;
   // packed particle-particle ladder (symmetric / antisymmetric pair combinations)
   DBuf Up, Um, taup, taum, Sld, Ald, ladpairs;
+  SplitOperand sUp, sUm;  // U+- of the one-irrep ladder in split precision (no FP64 copy)
   // out[ij,ab] += <ab|cd> in[ij,cd] at half the dense flops
   int ladder_packed(const double *in, double *out);
   // the same on irrep blocks (more than one irrep): pair irrep g of (a,b) and

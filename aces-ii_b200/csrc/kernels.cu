@@ -1041,11 +1041,15 @@ void launch_scatter(const double *dense, const DpdMap &m, cudaStream_t st) {
 // m(c,d) = d(d-1)/2 + c.  One block per (row a <= b, 32 x 32 tile pair of
 // (c, d) with the c tile <= the d tile): the [c][d] and [d][c] tiles of the
 // row's v x v block are read coalesced, the second through a shared-memory
-// transpose, and the packed outputs (consecutive c for one d) coalesce.
+// transpose, and the packed outputs (consecutive c for one d) coalesce.  S: the
+// outputs are the BF16 planes of the ladder's A operands (rows k_pad apart)
+// instead of FP64 arrays: 12 bytes per packed pair of elements instead of 16
+// written and then 16 + 8 for the split (o = 24, v = 220: 3.9 + 4.7 ms before).
+template <bool S>
 __global__ void __launch_bounds__(256)
     k_ladder_pack_v(double *__restrict__ Up, double *__restrict__ Um,
                     const double *__restrict__ V, const int *__restrict__ pairs, int v,
-                    int ntile) {
+                    int ntile, LadderPlanes pl) {
   __shared__ double t1[32][33];  // [c][d]
   __shared__ double t2[32][33];  // [c][d] = V[ab][d][c]
   const int np = v * (v + 1) / 2, nm = v * (v - 1) / 2;
@@ -1079,7 +1083,20 @@ __global__ void __launch_bounds__(256)
       const int c = c0 + cl, d = d0 + dl;
       if (c >= v || d >= v || c > d) continue;
       const double x = t1[cl][dl], y = t2[cl][dl];
-      if (c == d) {
+      if (S) {
+        __nv_bfloat16 h, l;
+        split_bf16(c == d ? x : 0.5 * (x + y), h, l);
+        const size_t ap = (size_t)r * pl.kp_p + (size_t)d * (d + 1) / 2 + c;
+        pl.hi_p[ap] = h;
+        pl.lo_p[ap] = l;
+        if (a < b && c < d) {
+          split_bf16(0.5 * (x - y), h, l);
+          const size_t am =
+              (size_t)(b * (b - 1) / 2 + a) * pl.kp_m + (size_t)d * (d - 1) / 2 + c;
+          pl.hi_m[am] = h;
+          pl.lo_m[am] = l;
+        }
+      } else if (c == d) {
         Up[(size_t)r * np + (size_t)d * (d + 1) / 2 + c] = x;
       } else {
         Up[(size_t)r * np + (size_t)d * (d + 1) / 2 + c] = 0.5 * (x + y);
@@ -1091,11 +1108,14 @@ __global__ void __launch_bounds__(256)
 }
 
 void launch_ladder_pack_v(double *Up, double *Um, const double *V, const int *pairs, int v,
-                          cudaStream_t st) {
+                          cudaStream_t st, const LadderPlanes *planes) {
   const int ntile = (v + 31) / 32;
   const long long blocks = (long long)(v * (v + 1) / 2) * (ntile * (ntile + 1) / 2);
-  k_ladder_pack_v<<<(unsigned)std::min<long long>(blocks, 148 * 64), 256, 0, st>>>(
-      Up, Um, V, pairs, v, ntile);
+  const unsigned grid = (unsigned)std::min<long long>(blocks, 148 * 64);
+  if (planes)
+    k_ladder_pack_v<true><<<grid, 256, 0, st>>>(Up, Um, V, pairs, v, ntile, *planes);
+  else
+    k_ladder_pack_v<false><<<grid, 256, 0, st>>>(Up, Um, V, pairs, v, ntile, LadderPlanes());
   count_launch();
 }
 

@@ -92,13 +92,15 @@ void launch_scatter_rpsq(const double *X, const DpdMap &m, cudaStream_t st);
 // packed particle-particle ladder (engine.cu, ladder_packed): pairs[2p], pairs[2p+1]
 // = (c, d) of the symmetric pair p (np = v(v+1)/2 of them) followed by the
 // antisymmetric pairs (c < d)
-void launch_ladder_pack_v(double *Up, double *Um, const double *V, const int *pairs, int v,
-                          cudaStream_t st);
-// BF16 planes (hi, lo; rows ij k_pad apart) of the packed tau+ / tau- operands
+// BF16 planes (hi, lo; rows k_pad apart) of the packed U+ / U- or tau+ / tau-
+// operands
 struct LadderPlanes {
   __nv_bfloat16 *hi_p = nullptr, *lo_p = nullptr, *hi_m = nullptr, *lo_m = nullptr;
   int kp_p = 0, kp_m = 0;
 };
+// with planes: U+- written only as the planes (Up, Um untouched)
+void launch_ladder_pack_v(double *Up, double *Um, const double *V, const int *pairs, int v,
+                          cudaStream_t st, const LadderPlanes *planes = nullptr);
 // tau+ / tau- of the C1 ladder in the packed order p(c,d) = d(d+1)/2 + c,
 // m(c,d) = d(d-1)/2 + c (the order of `pairs` in launch_ladder_pack_v); with
 // planes: written only as the planes (tp, tm untouched)
