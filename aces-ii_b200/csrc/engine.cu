@@ -24,7 +24,7 @@ std::vector<DBuf *> CCEngine::registry() {
   return {&eo, &ev, &foo, &fvv, &fov, &offo, &offv, &fovT, &I_oooo, &I_ooov, &I_oovv,
           &I_ovov, &I_ovvv, &I_vvvv, &L_oovv, &LF, &LovP, &LooP, &LmeP, &I1, &I2, &IvP,
           &IvP2, &IX, &IX2, &WA0, &WB0, &IoP3, &IvT, &IooT, &LT1, &X, &Xn, &Z1,
-          &Z2, &tau, &taut, &tautP, &tauT, &U, &Tp, &Tpp, &uT, &wP, &t2P, &Y1, &Y2, &XnP,
+          &Z2, &tau, &taut, &tautP, &tauT, &U, &Tp, &Tpp, &uT, &wP, &t2P, &Y2, &XnP,
           &WA, &WB, &ZT, &XP, &Xmn, &Wmnij, &WmnT, &t1T, &Fae, &Fmi, &Fme, &Fp, &Fpp,
           &FmiT, &FppT, &FmeT, &tmp4, &scratch, &dev_small, &Bmat, &dvec, &L, &Ln, &gE,
           &lrhs, &bwdA, &bwdB, &bwdC, &bwdD, &Up, &Um, &taup, &taum, &Sld, &Ald, &ladpairs, &Ic, &I1n};
@@ -78,7 +78,7 @@ void CCEngine::release() {
   st = 0;
 }
 
-int CCEngine::alloc(DBuf &b, size_t n) {
+int CCEngine::alloc(DBuf &b, size_t n, bool zero) {
   if (b.p && b.n >= n) return ACES_OK;
   if (b.borrowed) {
     set_error("engine: a borrowed list buffer cannot be reallocated");
@@ -94,7 +94,7 @@ int CCEngine::alloc(DBuf &b, size_t n) {
     return ACES_ERR_NOMEM;
   }
   b.n = n;
-  ACES_CUDA(cudaMemsetAsync(b.p, 0, bytes, st));
+  if (zero) ACES_CUDA(cudaMemsetAsync(b.p, 0, bytes, st));
   return ACES_OK;
 }
 
@@ -502,6 +502,25 @@ int make_map(DevMap &dm, int list, int typeL, int typeR, const std::vector<int> 
   return ACES_OK;
 }
 
+// Without symmetry a list of FULL pair types is one dense column-major block:
+// element (p,q | r,s) at p + q np + (r + s nr) np nq, read and written in place
+// by the resorts (no index tables, no gathered copy).  *out = nullptr with
+// irreps; the dimensions are checked as make_map checks them.
+int c1_list(int list, int typeL, int typeR, double **out) {
+  *out = nullptr;
+  const SymInfo &s = state().sym;
+  if (s.nirrep != 1) return ACES_OK;
+  int nc = 0, nr = 0;
+  aces_list_dims(1, list, &nc, &nr);
+  if (nc != s.irpdpd[0][typeR - 1] || nr != s.irpdpd[0][typeL - 1]) {
+    set_error("list %d irrep %d has %dx%d, expected %dx%d (types %d,%d)", list, 1, nr, nc,
+              s.irpdpd[0][typeL - 1], s.irpdpd[0][typeR - 1], typeL, typeR);
+    return ACES_ERR_NOLIST;
+  }
+  *out = aces_list_devptr(1, list);
+  return ACES_OK;
+}
+
 int CCEngine::load_from_lists() {
   State &stt = state();
   const SymInfo &s = stt.sym;
@@ -569,51 +588,73 @@ int CCEngine::load_from_lists() {
   ACES_TRY(h2d(offo, hofo)); ACES_TRY(h2d(offv, hofv)); ACES_TRY(h2d(fovT, hfovT));
   ACES_CUDA(cudaStreamSynchronize(st));
 
+  // lists put with aces_putlst_dev are complete (stream 0; this one does not wait for it)
+  ACES_CUDA(cudaStreamSynchronize(0));
   const long long O = o, V = v;
+  double *lp = nullptr;
   // list 13 (14,14): <Ij|Kl>  -> I_oooo[i,j,k,l]
-  {
+  ACES_TRY(alloc(I_oooo, O * O * O * O, false));
+  ACES_TRY(c1_list(13, 14, 14, &lp));
+  if (lp) {
+    ACES_TRY(perm(I_oooo.p, o, o, o, o, 0.0, {PT(lp, 1.0, 1, O, O * O, O * O * O)}));
+  } else {
     DevMap dm;
     ACES_TRY(make_map(dm, 13, 14, 14, irr_o, irr_v, false));
-    ACES_TRY(alloc(I_oooo, O * O * O * O));
     launch_gather(I_oooo.p, dm.m, st);
     ACES_CUDA(cudaStreamSynchronize(st));
   }
   // list 10 (14,18): <Ij|Ka>  -> I_ooov[i,j,k,a]
-  {
+  ACES_TRY(alloc(I_ooov, O * O * O * V, false));
+  ACES_TRY(c1_list(10, 14, 18, &lp));
+  if (lp) {
+    ACES_TRY(perm(I_ooov.p, o, o, o, v, 0.0, {PT(lp, 1.0, 1, O, O * O, O * O * O)}));
+  } else {
     DevMap dm;
     ACES_TRY(make_map(dm, 10, 14, 18, irr_o, irr_v, false));
-    ACES_TRY(alloc(I_ooov, O * O * O * V));
     launch_gather(I_ooov.p, dm.m, st);
     ACES_CUDA(cudaStreamSynchronize(st));
   }
-  // list 16 (13,14): <Ab|Ij> -> dense [a,b,i,j] -> I_oovv[i,j,a,b]
-  ACES_TRY(alloc(tmp4, std::max(O * O * V * V, O * V * V * V)));
-  {
+  if (s.nirrep != 1) ACES_TRY(alloc(tmp4, std::max(O * O * V * V, O * V * V * V), false));
+  // list 16 (13,14): <Ab|Ij> at a + b v + i v^2 + j v^2 o, or gathered to dense
+  // [a,b,i,j] -> I_oovv[i,j,a,b]
+  ACES_TRY(alloc(I_oovv, O * O * V * V, false));
+  ACES_TRY(c1_list(16, 13, 14, &lp));
+  if (lp) {
+    ACES_TRY(perm(I_oovv.p, o, o, v, v, 0.0, {PT(lp, 1.0, V * V, V * V * O, 1, V)}));
+  } else {
     DevMap dm;
     ACES_TRY(make_map(dm, 16, 13, 14, irr_o, irr_v, false));
     launch_gather(tmp4.p, dm.m, st);
-    ACES_TRY(alloc(I_oovv, O * O * V * V));
     // out (i,j,a,b) <- tmp[a,b,i,j]
     ACES_TRY(perm(I_oovv.p, o, o, v, v, 0.0, {PT(tmp4.p, 1.0, O, 1, V * O * O, O * O)}));
     ACES_CUDA(cudaStreamSynchronize(st));
   }
-  // list 25 (11,11): <Ai|Bj> -> dense [a,i,b,j] = <ai|bj>; I_ovov[m,b,j,e] = <mb|je> = <bm|ej> = d[b,m,e,j]
-  {
+  // list 25 (11,11): <Ai|Bj> at a + i v + (b + j v) v o, or gathered to dense
+  // [a,i,b,j] = <ai|bj>; I_ovov[m,b,j,e] = <mb|je> = <bm|ej> = d[b,m,e,j]
+  ACES_TRY(alloc(I_ovov, O * O * V * V, false));
+  ACES_TRY(c1_list(25, 11, 11, &lp));
+  if (lp) {
+    ACES_TRY(perm(I_ovov.p, o, v, o, v, 0.0, {PT(lp, 1.0, V, 1, V * V * O, V * O)}));
+  } else {
     DevMap dm;
     ACES_TRY(make_map(dm, 25, 11, 11, irr_o, irr_v, false));
     launch_gather(tmp4.p, dm.m, st);
-    ACES_TRY(alloc(I_ovov, O * O * V * V));
     // d strides: [a,i,b,j] -> a: O*V*O, i: V*O, b: O, j: 1 ; out (m,b,j,e) = d[b,m,e,j]
     ACES_TRY(perm(I_ovov.p, o, v, o, v, 0.0,
                   {PT(tmp4.p, 1.0, V * O, O * V * O, 1, O)}));
     ACES_CUDA(cudaStreamSynchronize(st));
   }
-  // list 30 (13,11): <Ab|Ci> -> dense [a,b,c,i]; I_ovvv[m,a,e,f] = <ma|ef> = <fe|am> = d[f,e,a,m]
-  {
+  // list 30 (13,11): <Ab|Ci> at a + b v + c v^2 + i v^3, or gathered to dense
+  // [a,b,c,i]; I_ovvv[m,a,e,f] = <ma|ef> = <fe|am> = d[f,e,a,m], the list block's
+  // own order
+  ACES_TRY(alloc(I_ovvv, O * V * V * V, false));
+  ACES_TRY(c1_list(30, 13, 11, &lp));
+  if (lp) {
+    ACES_TRY(copy(I_ovvv.p, lp, (size_t)(O * V * V * V)));
+  } else {
     DevMap dm;
     ACES_TRY(make_map(dm, 30, 13, 11, irr_o, irr_v, false));
     launch_gather(tmp4.p, dm.m, st);
-    ACES_TRY(alloc(I_ovvv, O * V * V * V));
     // d strides [a,b,c,i]: a: V*V*O, b: V*O, c: O, i: 1; out (m,a,e,f) = d[f,e,a,m]
     ACES_TRY(perm(I_ovvv.p, o, v, v, v, 0.0, {PT(tmp4.p, 1.0, 1, O, V * O, V * V * O)}));
     ACES_CUDA(cudaStreamSynchronize(st));
@@ -625,7 +666,7 @@ int CCEngine::load_from_lists() {
   // list's device memory instead of gathering a second copy (42.5 GB at
   // o = 30, v = 270).
   if (s.nirrep == 1 && aces_isytyp(1, 233) == 13 && aces_isytyp(2, 233) == 13) {
-    double *lp = aces_list_devptr(1, 233);
+    lp = aces_list_devptr(1, 233);
     int nc = 0, nr = 0;
     if (lp && aces_list_dims(1, 233, &nc, &nr) == ACES_OK && (long long)nr == V * V &&
         (long long)nc == V * V) {
@@ -638,7 +679,7 @@ int CCEngine::load_from_lists() {
   {
     DevMap dm;
     ACES_TRY(make_map(dm, 233, 13, 13, irr_o, irr_v, false));
-    ACES_TRY(alloc(I_vvvv, V * V * V * V));
+    ACES_TRY(alloc(I_vvvv, V * V * V * V, false));
     launch_gather(I_vvvv.p, dm.m, st);
     ACES_CUDA(cudaStreamSynchronize(st));
   }
@@ -658,79 +699,80 @@ int CCEngine::setup_intermediates() {
   const long long sv[4] = {V * V * V, V * V, V, 1};
   const long long s3[4] = {O * O * V, O * V, V, 1};
   const long long sj[4] = {V * O * V, O * V, V, 1};
-  ACES_TRY(alloc(L_oovv, OOVV));
+  // (no zero fill: every array below is written whole before it is read)
+  ACES_TRY(alloc(L_oovv, OOVV, false));
   ACES_TRY(perm(L_oovv.p, o, o, v, v, 0.0,
                 {PT(I_oovv.p, 2.0, so[0], so[1], so[2], so[3]),
                  PT(I_oovv.p, -1.0, so[0], so[1], so[3], so[2])}));
   // LF[a,e,m,f] = 2 I_ovvv[m,a,f,e] - I_ovvv[m,a,e,f]
-  ACES_TRY(alloc(LF, OVVV));
+  ACES_TRY(alloc(LF, OVVV, false));
   ACES_TRY(perm(LF.p, v, v, o, v, 0.0,
                 {PT(I_ovvv.p, 2.0, sv[1], sv[3], sv[0], sv[2]),
                  PT(I_ovvv.p, -1.0, sv[1], sv[2], sv[0], sv[3])}));
   // LovP[e,m,n,f] = L_oovv[m,n,e,f]
-  ACES_TRY(alloc(LovP, OOVV));
+  ACES_TRY(alloc(LovP, OOVV, false));
   ACES_TRY(perm(LovP.p, v, o, o, v, 0.0, {PT(L_oovv.p, 1.0, so[2], so[0], so[1], so[3])}));
   // LooP[m,i,n,e] = 2 I_ooov[m,n,i,e] - I_ooov[n,m,i,e]
-  ACES_TRY(alloc(LooP, OOOV));
+  ACES_TRY(alloc(LooP, OOOV, false));
   ACES_TRY(perm(LooP.p, o, o, o, v, 0.0,
                 {PT(I_ooov.p, 2.0, s3[0], s3[2], s3[1], s3[3]),
                  PT(I_ooov.p, -1.0, s3[1], s3[2], s3[0], s3[3])}));
   // LmeP[m,e,n,f] = L_oovv[m,n,e,f]
-  ACES_TRY(alloc(LmeP, OOVV));
+  ACES_TRY(alloc(LmeP, OOVV, false));
   ACES_TRY(perm(LmeP.p, o, v, o, v, 0.0, {PT(L_oovv.p, 1.0, so[0], so[2], so[1], so[3])}));
   // I1[m,e,n,f] = I_oovv[m,n,e,f];  I2[m,e,n,f] = I_oovv[m,n,f,e]
-  ACES_TRY(alloc(I1, OOVV));
+  ACES_TRY(alloc(I1, OOVV, false));
   ACES_TRY(perm(I1.p, o, v, o, v, 0.0, {PT(I_oovv.p, 1.0, so[0], so[2], so[1], so[3])}));
-  ACES_TRY(alloc(I2, OOVV));
+  ACES_TRY(alloc(I2, OOVV, false));
   ACES_TRY(perm(I2.p, o, v, o, v, 0.0, {PT(I_oovv.p, 1.0, so[0], so[3], so[1], so[2])}));
   // Ic = I1 - I2 / 2, I1n = -I1: W(mbej) += Y2 Ic^T + XnP I1n^T (one launch)
-  ACES_TRY(alloc(Ic, OOVV));
+  ACES_TRY(alloc(Ic, OOVV, false));
   ACES_TRY(perm(Ic.p, o, v, o, v, 0.0,
                 {PT(I_oovv.p, 1.0, so[0], so[2], so[1], so[3]),
                  PT(I_oovv.p, -0.5, so[0], so[3], so[1], so[2])}));
-  ACES_TRY(alloc(I1n, OOVV));
+  ACES_TRY(alloc(I1n, OOVV, false));
   ACES_TRY(perm(I1n.p, o, v, o, v, 0.0, {PT(I_oovv.p, -1.0, so[0], so[2], so[1], so[3])}));
   // IvP[b,m,e,f] = I_ovvv[m,b,e,f]; IvP2[b,m,e,f] = I_ovvv[m,b,f,e]
-  ACES_TRY(alloc(IvP, OVVV));
+  ACES_TRY(alloc(IvP, OVVV, false));
   ACES_TRY(perm(IvP.p, v, o, v, v, 0.0, {PT(I_ovvv.p, 1.0, sv[1], sv[0], sv[2], sv[3])}));
-  ACES_TRY(alloc(IvP2, OVVV));
+  ACES_TRY(alloc(IvP2, OVVV, false));
   ACES_TRY(perm(IvP2.p, v, o, v, v, 0.0, {PT(I_ovvv.p, 1.0, sv[1], sv[0], sv[3], sv[2])}));
   // IX[j,m,e,n] = I_ooov[n,m,j,e]; IX2[j,m,e,n] = I_ooov[m,n,j,e]
-  ACES_TRY(alloc(IX, OOOV));
+  ACES_TRY(alloc(IX, OOOV, false));
   ACES_TRY(perm(IX.p, o, o, v, o, 0.0, {PT(I_ooov.p, 1.0, s3[2], s3[1], s3[3], s3[0])}));
-  ACES_TRY(alloc(IX2, OOOV));
+  ACES_TRY(alloc(IX2, OOOV, false));
   ACES_TRY(perm(IX2.p, o, o, v, o, 0.0, {PT(I_ooov.p, 1.0, s3[2], s3[0], s3[3], s3[1])}));
   // WA0[j,b,m,e] = <mb|ej> = I_oovv[m,j,e,b];  WB0[j,b,m,e] = -<mb|je> = -I_ovov[m,b,j,e]
-  ACES_TRY(alloc(WA0, OOVV));
+  ACES_TRY(alloc(WA0, OOVV, false));
   ACES_TRY(perm(WA0.p, o, v, o, v, 0.0, {PT(I_oovv.p, 1.0, so[1], so[3], so[0], so[2])}));
-  ACES_TRY(alloc(WB0, OOVV));
+  ACES_TRY(alloc(WB0, OOVV, false));
   ACES_TRY(perm(WB0.p, o, v, o, v, 0.0, {PT(I_ovov.p, -1.0, sj[2], sj[1], sj[0], sj[3])}));
   // IoP3[i,j,b,m] = I_ooov[i,j,m,b]
-  ACES_TRY(alloc(IoP3, OOOV));
+  ACES_TRY(alloc(IoP3, OOOV, false));
   ACES_TRY(perm(IoP3.p, o, o, v, o, 0.0, {PT(I_ooov.p, 1.0, s3[0], s3[1], s3[3], s3[2])}));
   // IvT[j,a,b,e] = I_ovvv[j,e,b,a]
-  ACES_TRY(alloc(IvT, OVVV));
+  ACES_TRY(alloc(IvT, OVVV, false));
   ACES_TRY(perm(IvT.p, o, v, v, v, 0.0, {PT(I_ovvv.p, 1.0, sv[0], sv[3], sv[2], sv[1])}));
   // IooT[i,m,n,e] = I_ooov[m,n,i,e]
-  ACES_TRY(alloc(IooT, OOOV));
+  ACES_TRY(alloc(IooT, OOOV, false));
   ACES_TRY(perm(IooT.p, o, o, o, v, 0.0, {PT(I_ooov.p, 1.0, s3[2], s3[0], s3[1], s3[3])}));
   // LT1[i,a,n,f] = 2<na|fi> - <na|if> = 2 I_oovv[n,i,f,a] - I_ovov[n,a,i,f]
-  ACES_TRY(alloc(LT1, OOVV));
+  ACES_TRY(alloc(LT1, OOVV, false));
   ACES_TRY(perm(LT1.p, o, v, o, v, 0.0,
                 {PT(I_oovv.p, 2.0, so[1], so[3], so[0], so[2]),
                  PT(I_ovov.p, -1.0, sj[2], sj[1], sj[0], sj[3])}));
   // working storage
-  ACES_TRY(alloc(X, OV + OOVV));
-  ACES_TRY(alloc(Xn, OV + OOVV));
-  ACES_TRY(alloc(Z1, OV));
-  ACES_TRY(alloc(Z2, OOVV));
+  ACES_TRY(alloc(X, OV + OOVV, false));
+  ACES_TRY(alloc(Xn, OV + OOVV, false));
+  ACES_TRY(alloc(Z1, OV, false));
+  ACES_TRY(alloc(Z2, OOVV, false));
   DBuf *big[] = {&tau, &taut, &tautP, &tauT, &U, &Tp, &Tpp, &uT, &wP, &t2P,
-                 &Y1, &Y2, &XnP, &WA, &WB, &XP};
-  for (DBuf *b : big) ACES_TRY(alloc(*b, OOVV));
-  ACES_TRY(alloc(ZT, OOOV));
-  ACES_TRY(alloc(Xmn, O * O * O * O));
-  ACES_TRY(alloc(Wmnij, O * O * O * O));
-  ACES_TRY(alloc(WmnT, O * O * O * O));
+                 &Y2, &XnP, &WA, &WB, &XP};
+  for (DBuf *b : big) ACES_TRY(alloc(*b, OOVV, false));
+  ACES_TRY(alloc(ZT, OOOV, false));
+  ACES_TRY(alloc(Xmn, O * O * O * O, false));
+  ACES_TRY(alloc(Wmnij, O * O * O * O, false));
+  ACES_TRY(alloc(WmnT, O * O * O * O, false));
   ACES_TRY(alloc(t1T, OV));
   ACES_TRY(alloc(Fae, V * V)); ACES_TRY(alloc(Fp, V * V));
   ACES_TRY(alloc(Fmi, O * O)); ACES_TRY(alloc(Fpp, O * O));
@@ -1165,15 +1207,15 @@ int CCEngine::ladder_packed(const double *in, double *out) {
     launch_ladder_pack_v(nullptr, nullptr, I_vvvv.p, (const int *)ladpairs.p, v, st, &pl);
     ACES_CUDA(cudaGetLastError());
   } else if (!sp && !Up.p) {
-    ACES_TRY(alloc(Up, (size_t)np * np));
-    ACES_TRY(alloc(Um, (size_t)std::max(nm, 1) * std::max(nm, 1)));
+    ACES_TRY(alloc(Up, (size_t)np * np, false));
+    ACES_TRY(alloc(Um, (size_t)std::max(nm, 1) * std::max(nm, 1), false));
     launch_ladder_pack_v(Up.p, Um.p, I_vvvv.p, (const int *)ladpairs.p, v, st);
     ACES_CUDA(cudaStreamSynchronize(st));
   }
-  ACES_TRY(alloc(taup, (size_t)oo * np));
-  ACES_TRY(alloc(taum, (size_t)oo * std::max(nm, 1)));
-  ACES_TRY(alloc(Sld, (size_t)oo * np));
-  ACES_TRY(alloc(Ald, (size_t)oo * std::max(nm, 1)));
+  ACES_TRY(alloc(taup, (size_t)oo * np, false));
+  ACES_TRY(alloc(taum, (size_t)oo * std::max(nm, 1), false));
+  ACES_TRY(alloc(Sld, (size_t)oo * np, false));
+  ACES_TRY(alloc(Ald, (size_t)oo * std::max(nm, 1), false));
   memo_written(taup.p, (long long)oo * np);
   memo_written(taum.p, (long long)oo * std::max(nm, 1));
   // both products in one grouped launch (their tiles fill each other's last wave)
@@ -1287,8 +1329,8 @@ int CCEngine::iteration(int icycle, int exporder, double *e3, double *res, doubl
   // cycle waits on the allocator
   for (int k = 0; k < exporder; ++k)
     if (!hx[k].p) {
-      ACES_TRY(alloc(hx[k], len));
-      ACES_TRY(alloc(he[k], len));
+      ACES_TRY(alloc(hx[k], len, false));
+      ACES_TRY(alloc(he[k], len, false));
     }
   ACES_TRY(copy(hx[idimr].p, cur, len));
   std::vector<const double *> hp(ndimr);
@@ -1324,7 +1366,7 @@ int CCEngine::iteration(int icycle, int exporder, double *e3, double *res, doubl
   // DIIS residual dvec = sum_i c_i e_i (vcc/dodiis0.F:131-146)
   std::vector<const double *> pe(ndimr);
   for (int k = 0; k < ndimr; ++k) pe[k] = he[k].p;
-  ACES_TRY(alloc(dvec, len));
+  ACES_TRY(alloc(dvec, len, false));
   launch_lincomb_absmax(dvec.p, d + 40, pe.data(), ndimr, o, v, scratch.p, d + 4, st);
   int hstat = 0;
   ACES_CUDA(cudaMemcpyAsync(&hstat, status, 4, cudaMemcpyDeviceToHost, st));
@@ -1360,10 +1402,18 @@ int CCEngine::write_amplitudes(const double *a1, const double *a2, int list1, in
   const SymInfo &s = state().sym;
   // doubles (AB) -> list2ab (13,14): dense [a,b,i,j] = a2[i,j,a,b]
   DBuf tmpb;
-  ACES_TRY(alloc(tmpb, O * O * V * V));
+  ACES_TRY(alloc(tmpb, O * O * V * V, false));
   const long long st2[4] = {O * V * V, V * V, V, 1};
-  ACES_TRY(perm(tmpb.p, v, v, o, o, 0.0, {PT(a2, 1.0, st2[2], st2[3], st2[0], st2[1])}));
-  {
+  double *lp = nullptr;
+  ACES_CUDA(cudaStreamSynchronize(0));  // pending device reads of the old contents
+  if (s.nirrep == 1) {
+    ACES_TRY(list_inipck(1, 13, 14, list2ab, 1, false));
+    ACES_TRY(c1_list(list2ab, 13, 14, &lp));
+  }
+  if (lp) {  // a + b v + i v^2 + j v^2 o
+    ACES_TRY(perm(lp, o, o, v, v, 0.0, {PT(a2, 1.0, st2[1], st2[0], st2[3], st2[2])}));
+  } else {
+    ACES_TRY(perm(tmpb.p, v, v, o, o, 0.0, {PT(a2, 1.0, st2[2], st2[3], st2[0], st2[1])}));
     DevMap dm;
     ACES_TRY(make_map(dm, list2ab, 13, 14, irr_o, irr_v, true));
     launch_scatter(tmpb.p, dm.m, st);

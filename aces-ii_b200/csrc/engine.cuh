@@ -60,7 +60,7 @@ class CCEngine {
   double *t2n() { return Xn.p + (size_t)o * v; }
 
   // temporaries
-  DBuf tau, taut, tautP, tauT, U, Tp, Tpp, uT, wP, t2P, Y1, Y2, XnP, WA, WB, ZT, XP, Xmn, Wmnij,
+  DBuf tau, taut, tautP, tauT, U, Tp, Tpp, uT, wP, t2P, Y2, XnP, WA, WB, ZT, XP, Xmn, Wmnij,
       WmnT, t1T, Fae, Fmi, Fme, Fp, Fpp, FmiT, FppT, FmeT, tmp4;
   // packed particle-particle ladder (symmetric / antisymmetric pair combinations)
   DBuf Up, Um, taup, taum, Sld, Ald, ladpairs;
@@ -184,7 +184,9 @@ class CCEngine {
   cudaEvent_t ev_lad0 = nullptr, ev_lad1 = nullptr;  // around the pp-ladder contraction
 
   ~CCEngine();
-  int alloc(DBuf &b, size_t n);
+  // b holds at least n doubles afterwards; a new buffer is zeroed unless its
+  // first use writes all of it (zero = false)
+  int alloc(DBuf &b, size_t n, bool zero = true);
   int load_from_lists();
   int setup_intermediates();
   int mp2_guess();
