@@ -150,6 +150,9 @@ __device__ __forceinline__ void split_bf16(double x, __nv_bfloat16 &h, __nv_bflo
 
 // Fill a split operand from an FP64 K-contiguous matrix (src[r*ld + k]).
 int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int k, cudaStream_t st);
+// ... and from a column-major one (src[r + k*ld])
+int split_pack_t(SplitOperand &op, const double *src, long long ld, int rows, int k,
+                 cudaStream_t st);
 
 // BF16x3 contraction on tcgen05: A, B split operands with equal k_pad.
 // acc = A_hi B_hi + A_hi B_lo + A_lo B_hi in FP32 (TMEM), C = alpha*acc + beta*C (FP64).

@@ -69,8 +69,47 @@ __global__ void k_split_pack(__nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__
   }
 }
 
-int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int k,
-               cudaStream_t st) {
+// The same from a column-major source (src[r + c * ld], element (r, c) of the
+// operand): 64 x 64 tiles read with lanes along r and written with lanes along
+// c through shared memory.  Bandwidth bound: 12 bytes per element, where a
+// transposed FP64 copy and a split moved 28 (3600 x 3600: 72 us before).
+__global__ void __launch_bounds__(256)
+    k_split_pack_t(__nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo,
+                   const double *__restrict__ src, long long ld, int rows, int k, int kp) {
+  __shared__ double T[64][65];   // [r][c]
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long r0 = blockIdx.x * 64LL;
+  const int c0 = blockIdx.y * 64;
+  double x[8][2];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long r = r0 + tx + 32 * h;
+      const int c = c0 + ty + 8 * q;
+      x[q][h] = r < rows && c < k ? src[r + (long long)c * ld] : 0.0;
+    }
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) T[tx + 32 * h][ty + 8 * q] = x[q][h];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int rl = ty + 8 * q;
+    const long long r = r0 + rl;
+    if (r >= rows) break;
+    __nv_bfloat16 h0, l0, h1, l1;
+    split_bf16(T[rl][2 * tx], h0, l0);
+    split_bf16(T[rl][2 * tx + 1], h1, l1);
+    const long long e = r * (kp / 2) + c0 / 2 + tx;
+    hi[e] = __halves2bfloat162(h0, h1);
+    lo[e] = __halves2bfloat162(l0, l1);
+  }
+}
+
+// planes of a rows x k operand: allocated or reused, dimensions set
+static int split_planes(SplitOperand &op, int rows, int k) {
   int rp = rows;
   int kp = (k + kSplitKPad - 1) / kSplitKPad * kSplitKPad;
   size_t need = (size_t)rp * kp * 2 * 2;
@@ -92,7 +131,14 @@ int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int 
   op.rows_pad = rp;
   op.k_pad = kp;
   op.lo = (char *)op.hi + (size_t)rp * kp * 2;
-  const long long pairs = (long long)rp * (kp / 2);
+  return ACES_OK;
+}
+
+int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int k,
+               cudaStream_t st) {
+  ACES_TRY(split_planes(op, rows, k));
+  const int kp = op.k_pad;
+  const long long pairs = (long long)rows * (kp / 2);
   long long nb = (pairs + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
   const FastDiv fp((unsigned)(kp / 2));
@@ -103,6 +149,22 @@ int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int 
     k_split_pack<true><<<(unsigned)nb, 256, 0, st>>>(
         (__nv_bfloat162 *)op.hi, (__nv_bfloat162 *)op.lo, src, ld, k, pairs, fp);
   count_launch();
+  ACES_CUDA(cudaGetLastError());
+  return ACES_OK;
+}
+
+int split_pack_t(SplitOperand &op, const double *src, long long ld, int rows, int k,
+                 cudaStream_t st) {
+  ACES_TRY(split_planes(op, rows, k));
+  const int ct = op.k_pad / 64;
+  // column tiles in grid.y (at most 65535 = 4.2 M columns) per launch
+  for (int t0 = 0; t0 < ct; t0 += 65535) {
+    const int n = std::min(65535, ct - t0);
+    k_split_pack_t<<<dim3((unsigned)((rows + 63LL) / 64), n), 256, 0, st>>>(
+        (__nv_bfloat162 *)op.hi + (size_t)t0 * 32, (__nv_bfloat162 *)op.lo + (size_t)t0 * 32,
+        src + (long long)t0 * 64 * ld, ld, rows, k - t0 * 64, op.k_pad);
+    count_launch();
+  }
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
 }

@@ -49,29 +49,30 @@ extern "C" int aces_xgemm(char transa, char transb, int m, int n, int k, double 
   long long ldak = lda, ldbk = ldb;
   double *tA = nullptr, *tB = nullptr;
   int status = ACES_OK;
-  if (ta == 'N') {  // op(A)(i,l) = A[i + l*lda]
-    status = to_kmajor(&tA, A, m, k, lda, st);
-    Ak = tA;
-    ldak = k;
-  }
-  if (status == ACES_OK && tb == 'T') {  // op(B)(l,j) = B[j + l*ldb]
-    status = to_kmajor(&tB, B, n, k, ldb, st);
-    Bk = tB;
-    ldbk = k;
-  }
-  if (status == ACES_OK) {
-    CView C = cview_colmajor(Cm, ldc);
-    if (precision == ACES_PREC_BF16X3 && k > 0) {
-      SplitOperand sa, sb;
-      status = split_pack(sa, Ak, ldak, m, k, st);
-      if (status == ACES_OK) status = split_pack(sb, Bk, ldbk, n, k, st);
-      if (status == ACES_OK) status = gemm_nt_bf16x3(sa, sb, m, n, alpha, beta, C, st);
-      cudaStreamSynchronize(st);
-      if (sa.hi) dev_free(sa.hi);
-      if (sb.hi) dev_free(sb.hi);
-    } else {
-      status = gemm_nt_f64(m, n, k, alpha, Ak, ldak, Bk, ldbk, beta, C, st);
+  const CView C = cview_colmajor(Cm, ldc);
+  if (precision == ACES_PREC_BF16X3 && k > 0) {
+    // the planes straight from either storage order
+    SplitOperand sa, sb;
+    status = ta == 'N' ? split_pack_t(sa, A, lda, m, k, st) : split_pack(sa, A, lda, m, k, st);
+    if (status == ACES_OK)
+      status = tb == 'T' ? split_pack_t(sb, B, ldb, n, k, st) : split_pack(sb, B, ldb, n, k, st);
+    if (status == ACES_OK) status = gemm_nt_bf16x3(sa, sb, m, n, alpha, beta, C, st);
+    cudaStreamSynchronize(st);
+    if (sa.hi) dev_free(sa.hi);
+    if (sb.hi) dev_free(sb.hi);
+  } else {
+    if (ta == 'N') {  // op(A)(i,l) = A[i + l*lda]
+      status = to_kmajor(&tA, A, m, k, lda, st);
+      Ak = tA;
+      ldak = k;
     }
+    if (status == ACES_OK && tb == 'T') {  // op(B)(l,j) = B[j + l*ldb]
+      status = to_kmajor(&tB, B, n, k, ldb, st);
+      Bk = tB;
+      ldbk = k;
+    }
+    if (status == ACES_OK)
+      status = gemm_nt_f64(m, n, k, alpha, Ak, ldak, Bk, ldbk, beta, C, st);
   }
   cudaError_t e = cudaStreamSynchronize(st);
   if (tA) dev_free(tA);
