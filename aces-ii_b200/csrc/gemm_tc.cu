@@ -233,6 +233,7 @@ constexpr int block_threads() { return 32 * (2 + epi_warps<BN>()); }
 // 96 KB fit, and a k tile took 2600 cycles against the 1056 of its products; a
 // pair shares B, which leaves 56 KB per CTA and stage and four stages.
 constexpr int TBN_WIDE = 192;
+constexpr int kWideMinN = 128;
 constexpr int kWideTag = 256;   // the wide variant in a launch's bn and in saved tile choices
 static_assert(epi_cols<TBN>() == 64 && epi_cols<TBN_1>() * epi_warps<TBN_1>() == 4 * TBN_1 &&
                   epi_cols<TBN_WIDE>() == 96,
@@ -1748,10 +1749,11 @@ int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOpera
   memset(&L, 0, sizeof(L));
   L.nprob = 1;
   L.cg = ch.cg == 2 ? 2 : 1;
-  // FP32 output whose every tile is one accumulation chunk, with 144 < N <=
-  // 192: one wide tile across N instead of a full and a ragged narrow one
-  // (where N fits one narrow tile those are faster: o = 6, v = 128 class
-  // launches ran 32 % slower on 128 x 256 tiles of one CTA)
+  // FP32 output whose every tile is one accumulation chunk, 128 <= N <= 192:
+  // one wide tile across N.  (T), o = 10 at v = 128 / 136 / 144 / 145: 5.9 / 8.0
+  // / 8.8 / 10.7 ms on wide tiles, 6.4 / 9.4 / 10.4 / 15.4 on 144-wide ones;
+  // o = 8, v = 192: 11.3 against 15.3 (smaller N was not measured: (T) takes
+  // this path from v = 128 on)
   int kt = 0;
   for (int s = 0; s < nseg; ++s) kt += Apar[s].k_pad / TBK;
   const bool fits = f32out && N <= TBN_WIDE && kt <= chunk_for(kt);
@@ -1760,7 +1762,7 @@ int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOpera
   else if (ch.bn)
     L.bn = ch.bn == kWideTag && fits ? kWideTag : TBN_1;
   else
-    L.bn = fits && N > TBN_1 && g_tc_wide.load() ? kWideTag : TBN_1;
+    L.bn = fits && N >= kWideMinN && g_tc_wide.load() ? kWideTag : TBN_1;
   if (L.bn == kWideTag) L.cg = 2;
   ACES_TRY(set_problem(L, 0, Apar, Bpar, nseg, M, N, C));
   Problem &P = L.prob[0];
@@ -1950,7 +1952,7 @@ int gemm_nt_bf16x3_batched(const SplitOperand *Apar, const SplitOperand *Bpar, i
   // both widths of the one-CTA tile (cands[0] keeps the default rule); the
   // CTA pairs stay with the aces_set_tc_pairs switch here
   std::vector<TuneChoice> cands{def};
-  if (def.cg == 1 && f32out && N > TBN_1 && N <= TBN_WIDE && kt <= chunk_for(kt)) {
+  if (def.cg == 1 && f32out && N >= kWideMinN && N <= TBN_WIDE && kt <= chunk_for(kt)) {
     TuneChoice c;
     c.bn = g_tc_wide.load() ? TBN_1 : kWideTag;
     cands.push_back(c);
@@ -2115,7 +2117,7 @@ void tc_set_pairs(int on) { g_tc_pairs.store(on ? 1 : 0); }
 void tc_set_wide(int on) { g_tc_wide.store(on ? 1 : 0); }
 
 bool bf16x3_wide_applies(const SplitOperand *A, int nseg, int N) {
-  if (!g_tc_wide.load() || pairs_for(1 << 30) || N <= TBN_1 || N > TBN_WIDE || nseg < 1 ||
+  if (!g_tc_wide.load() || pairs_for(1 << 30) || N < kWideMinN || N > TBN_WIDE || nseg < 1 ||
       nseg > kMaxSeg)
     return false;
   int kt = 0;

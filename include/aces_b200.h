@@ -183,8 +183,8 @@ int aces_debug_inject(int mode);
  * error bound; process-wide. */
 int aces_set_tc_pairs(int on);
 /* Tile width of the tensor-core launches whose every output tile is one
- * accumulation chunk with FP32 output and 144 < N <= 192 (the batched (T)
- * classes for 144 < v <= 192; no counterpart in the reference): 1 = one
+ * accumulation chunk with FP32 output and 128 <= N <= 192 (the batched (T)
+ * classes for 128 <= v <= 192; no counterpart in the reference): 1 = one
  * 256 x 192 tile of a CTA pair across N (the default), 0 = 128 x 144 tiles.  Same
  * arithmetic either way; process-wide. */
 int aces_set_tc_wide(int on);

@@ -1,5 +1,5 @@
 """GPU test of the wide tiles of the batched (T) class launches at the
-edges of their range against the 144-wide tiles: v = 145 and 192 (one tile
+edges of their range against the 144-wide tiles: v = 128 and 192 (one tile
 across N, the narrowest and the widest), odd v (rows of W that start on
 4-byte boundaries), v = 170 and 176 (8- and 16-byte boundaries), nocc with
 partial K steps (3, 16, 17) and v^2 ragged against the tile rows.
@@ -24,7 +24,7 @@ def lib():
     return lib
 
 
-@pytest.mark.parametrize("o,v", [(3, 145), (3, 151), (4, 170), (3, 176), (3, 192), (16, 146),
+@pytest.mark.parametrize("o,v", [(3, 128), (3, 129), (3, 145), (3, 151), (4, 170), (3, 176), (3, 192), (16, 146),
                                  (17, 145)])
 def test_wide_tiles_match_narrow_tiles(lib, o, v):
     ham = synthetic(o, v, 40, seed=o + v, bscale=0.5)
