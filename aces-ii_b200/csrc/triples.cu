@@ -29,111 +29,17 @@ namespace {
 // W at (x[kOrd[s][0]], x[kOrd[s][1]], x[kOrd[s][2]]).
 constexpr int kOrd[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
 
-constexpr int ord_index(int a, int b, int c) {
-  for (int s = 0; s < 6; ++s)
-    if (kOrd[s][0] == a && kOrd[s][1] == b && kOrd[s][2] == c) return s;
-  return -1;
-}
-
-// kT.v[q][p][m]: for the triplet permutation p and the set ordering q, the
-// ordering of the set that supplies W_abc, W_bca, W_cab and W_cba (m = 0..3)
-// of the closed-shell energy expression.  Built at compile time so the
-// energy kernel indexes its six W values with constants (registers).
-struct TripleTable {
-  int v[6][6][4];
-};
-constexpr TripleTable make_triple_table() {
-  TripleTable t{};
-  const int args[4][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-  int S[6][4] = {};
-  int comp[6][6] = {};
-  for (int p = 0; p < 6; ++p)
-    for (int m = 0; m < 4; ++m) {
-      int pos[3] = {0, 0, 0};
-      for (int r = 0; r < 3; ++r) pos[kOrd[p][r]] = args[m][r];
-      S[p][m] = ord_index(pos[0], pos[1], pos[2]);
-    }
-  for (int q = 0; q < 6; ++q)
-    for (int s = 0; s < 6; ++s)
-      comp[q][s] = ord_index(kOrd[q][kOrd[s][0]], kOrd[q][kOrd[s][1]], kOrd[q][kOrd[s][2]]);
-  for (int q = 0; q < 6; ++q)
-    for (int p = 0; p < 6; ++p)
-      for (int m = 0; m < 4; ++m) t.v[q][p][m] = comp[q][S[p][m]];
-  return t;
-}
-constexpr TripleTable kT = make_triple_table();
-
-// the table entries as template constants (usable in device code)
-template <int Q, int P, int M>
-struct TT {
-  static constexpr int value = kT.v[Q][P][M];
-};
-template <int Q, int P>
-__device__ __forceinline__ void accum_orders(const double (&u)[6], const double (&vd)[6],
-                                             double &g4, double &g5) {
-  constexpr int s0 = TT<Q, P, 0>::value, s1 = TT<Q, P, 1>::value, s2 = TT<Q, P, 2>::value,
-                s3 = TT<Q, P, 3>::value;
-  const double Z = 4.0 * u[s0] + u[s1] + u[s2];
-  g4 += Z * (u[s0] - u[s3]);
-  g5 += Z * (vd[s0] - vd[s3]);
-  if constexpr (P < 5) accum_orders<Q, P + 1>(u, vd, g4, g5);
-}
-template <int Q>
-__device__ __forceinline__ void accum_sets(const bool (&use)[6], const double (&u)[6],
-                                           const double (&vd)[6], double &g4, double &g5) {
-  if (use[Q]) accum_orders<Q, 0>(u, vd, g4, g5);
-  if constexpr (Q < 5) accum_sets<Q + 1>(use, u, vd, g4, g5);
-}
-
-// For a set of three distinct virtuals every ordering q is used, and the
-// energy terms above form a fixed bilinear form in the six W values:
-//   g4 = sum_{q,p} (4 u_s0 + u_s1 + u_s2)(u_s0 - u_s3) = u^T M u,
-//   g5 = sum_{q,p} (4 u_s0 + u_s1 + u_s2)(vd_s0 - vd_s3) = u^T M vd,
-// with integer M[a][b] = sum_{q,p} r_qp[a] c_qp[b], r = 4 e_s0 + e_s1 + e_s2,
-// c = e_s0 - e_s3 (s_m = kT.v[q][p][m]).  Built at compile time.
-struct FormTable {
-  int m[6][6];
-};
-constexpr FormTable make_form_table() {
-  FormTable f{};
-  for (int q = 0; q < 6; ++q)
-    for (int p = 0; p < 6; ++p) {
-      const int s0 = kT.v[q][p][0], s1 = kT.v[q][p][1], s2 = kT.v[q][p][2],
-                s3 = kT.v[q][p][3];
-      const int r[3] = {s0, s1, s2}, rw[3] = {4, 1, 1};
-      for (int k = 0; k < 3; ++k) {
-        f.m[r[k]][s0] += rw[k];
-        f.m[r[k]][s3] -= rw[k];
-      }
-    }
-  return f;
-}
-constexpr FormTable kM = make_form_table();
-template <int A, int B>
-struct MM {
-  static constexpr int value = kM.m[A][B];
-};
-// y[B] = sum_A M[A][B] u[A] (zero coefficients fold away)
-template <int B, int A = 0>
-__device__ __forceinline__ double form_col(const double (&u)[6]) {
-  if constexpr (A == 6) {
-    return 0.0;
-  } else {
-    constexpr int c = MM<A, B>::value;
-    if constexpr (c == 0) return form_col<B, A + 1>(u);
-    else return (double)c * u[A] + form_col<B, A + 1>(u);
-  }
-}
-template <int B = 0>
-__device__ __forceinline__ void form_apply(const double (&u)[6], const double (&vd)[6], double &g4,
-                                           double &g5) {
-  if constexpr (B < 6) {
-    const double y = form_col<B>(u);
-    g4 += y * u[B];
-    g5 += y * vd[B];
-    form_apply<B + 1>(u, vd, g4, g5);
-  }
-}
+// The energy of a virtual set.  With the ordering s of the set read as an
+// element of the permutation group, the terms of E[4]T over all orderings of
+// the set and all permutations of (i,j,k),
+//   sum_{q,p} (4 u_s0 + u_s1 + u_s2)(u_s0 - u_s3)
+// (s0..s3: the orderings of W_abc, W_bca, W_cab, W_cba under q and p), are the
+// bilinear form u^T M u with M[s][s] = 24, M[s][s'] = 6 where s' is a cyclic
+// permutation of s (the orderings 0, 3, 4 and 1, 2, 5) and -12 otherwise, and
+// E[5]ST is u^T M vd.  So (M u)_s = 18 u_s + 6 E - 12 O on the even orderings
+// and 18 u_s + 6 O - 12 E on the odd ones, E and O the sums over 0, 3, 4 and
+// 1, 2, 5.  A repeated virtual makes orderings coincide in pairs (or all six):
+// their distinct ones contribute half (a sixth) of the form.
 
 // a >= b >= c from the flat index n of the set in the order
 // (a, then b <= a, then c <= b): n = a(a+1)(a+2)/6 + b(b+1)/2 + c
@@ -151,19 +57,18 @@ __device__ __forceinline__ void decode_set(int n, int &a, int &b, int &c) {
 }
 
 // One batch entry's contribution to E[4]T and E[5]ST, every set {a >= b >= c}
-// of virtuals evaluated once with all six of its orderings, the distinct
-// orderings q of repeated virtuals counted once (a = b keeps q = 0, 1, 4;
-// b = c keeps q = 0, 2, 3; a = b = c keeps q = 0).  The loads are staged
-// through shared memory.  Block
-// (blockIdx.x, blockIdx.y = e) takes one tile triple A >= B >= C of 8-wide
-// virtual tiles (decoded like a set) of triplet e and loads, with sector-
-// complete row reads, the six permuted 8x8x8 cubes of W (tiles (A,B,C),
-// (A,C,B), ..., one per ordering), the 8x8 tiles of the <jk|..>, <ik|..>,
-// <ij|..> slabs for every ordered pair of the three tiles, and the t1 rows and
-// orbital energies of the three tiles.  Each of its 128 threads then
-// evaluates four sets {a >= b >= c} of the cube from shared memory: sets of
-// three distinct virtuals through the constant bilinear form, sets with a
-// repeated virtual through the general per-ordering sum.
+// of virtuals evaluated once.  Block (blockIdx.x, blockIdx.y = e) takes one
+// tile triple A >= B >= C of 8-wide virtual tiles (decoded like a set) of
+// triplet e and stages in shared memory, with sector-complete row reads, the
+// six permuted 8x8x8 cubes of W (tiles (A,B,C), (A,C,B), ..., one per
+// ordering), the 8x8 tiles of the <jk|..>, <ik|..>, <ij|..> slabs for every
+// ordered pair of the three tiles, and the t1 rows and orbital energies of the
+// three tiles.  Each of its 128 threads then evaluates four sets that share
+// (b, c): what depends on these alone is read once.
+// Instruction bound (W is read once, at 10 % of the DRAM rate): index splits
+// per staged element, 36 shared-memory reads and a general 6 x 6 form per set,
+// and a per-ordering sum for repeated virtuals took 1830 instructions per warp
+// (o = 14, v = 170: 14.0 ms; with the form above and these loop orders 8.3).
 constexpr int kTile = 8;
 // triplets of one FP64 batch (the energy launch's grid.y holds 65535)
 constexpr int kMaxTasks = 32768;
@@ -177,6 +82,10 @@ static_assert(ordpos(0, 2) == kOrd[0][2] && ordpos(3, 1) == kOrd[3][1] &&
                   ordpos(4, 2) == kOrd[4][2] && ordpos(5, 0) == kOrd[5][0] &&
                   ordpos(1, 1) == kOrd[1][1] && ordpos(2, 1) == kOrd[2][1],
               "ordpos restates kOrd");
+// index of the ordered pair (x, y) of tile positions, x != y
+__host__ __device__ __forceinline__ constexpr int pairpos(int x, int y) {
+  return x * 2 + (y > x ? y - 1 : y);
+}
 template <typename TW>
 __global__ void __launch_bounds__(128)
     k_triples_energy_tiled(const TW *__restrict__ Wbase, long long wstride,
@@ -194,33 +103,39 @@ __global__ void __launch_bounds__(128)
   const TW *__restrict__ W = Wbase + (long long)e * wstride;
   const int mult = (i == j && j == k) ? 6 : ((i == j || j == k) ? 2 : 1);
   const double scale = 1.0 / (3.0 * mult);
-  const long long v2 = (long long)v * v;
+  const int v2 = v * v;
   int T[3];
   decode_set((int)blockIdx.x, T[0], T[1], T[2]);
   const int b0[3] = {T[0] * kTile, T[1] * kTile, T[2] * kTile};
   const int tid = threadIdx.x;
-  // six cubes: cube s spans tiles (T[kOrd[s][0]], T[kOrd[s][1]], T[kOrd[s][2]])
+  // this thread's place in an 8 x 8 tile and which half of the third index
+  const int half = tid >> 6, l1 = (tid >> 3) & 7, l2 = tid & 7;
+  // six cubes: cube s spans tiles (T[kOrd[s][0]], T[kOrd[s][1]], T[kOrd[s][2]]);
+  // the thread loads (x, y, z) = (half + 2 q, l1, l2)
 #pragma unroll
   for (int s = 0; s < 6; ++s) {
-    const int c0 = b0[ordpos(s, 0)], c1 = b0[ordpos(s, 1)], c2 = b0[ordpos(s, 2)];
+    const int gx = b0[ordpos(s, 0)] + half, gy = b0[ordpos(s, 1)] + l1,
+              gz = b0[ordpos(s, 2)] + l2;
+    const TW *w = W + ((long long)gx * v2 + (gy * v + gz));
+    const bool in = gy < v && gz < v;
+    TW x[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = tid + 128 * q;
-      const int x = idx >> 6, y = (idx >> 3) & 7, z = idx & 7;
-      const int gx = c0 + x, gy = c1 + y, gz = c2 + z;
-      cube[s][x][y][z] = (gx < v && gy < v && gz < v) ? W[gx * v2 + (long long)gy * v + gz]
-                                                      : (TW)0;
-    }
+    for (int q = 0; q < 4; ++q) x[q] = in && gx + 2 * q < v ? w[(long long)(2 * q) * v2] : (TW)0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cube[s][half + 2 * q][l1][l2] = x[q];
   }
-  // integral tiles: slab 0 = <jk|..>, 1 = <ik|..>, 2 = <ij|..>; ordered pair
-  // (x, y) of tile positions -> index x * 2 + (y > x ? y - 1 : y)
+  // integral tiles: slab 0 = <jk|..>, 1 = <ik|..>, 2 = <ij|..>; the two halves
+  // of the block take the two pairs (x, .) of each x
   const double *slab[3] = {Ioovv + ((long long)j * o + k) * v2, Ioovv + ((long long)i * o + k) * v2,
                            Ioovv + ((long long)i * o + j) * v2};
-  for (int idx = tid; idx < 3 * 6 * 64; idx += 128) {
-    const int sl = idx / 384, pr = (idx / 64) % 6, r = (idx >> 3) & 7, c = idx & 7;
-    const int x = pr >> 1, yy = pr & 1, y = yy < x ? yy : yy + 1;
-    const int gr = b0[x] + r, gc = b0[y] + c;
-    It[sl][pr][r][c] = (gr < v && gc < v) ? slab[sl][(long long)gr * v + gc] : 0.0;
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    const int y = half < x ? half : half + 1;
+    const int gr = b0[x] + l1, gc = (y == 0 ? b0[0] : (y == 1 ? b0[1] : b0[2])) + l2;
+    const bool in = gr < v && gc < v;
+    const int at = gr * v + gc;
+#pragma unroll
+    for (int sl = 0; sl < 3; ++sl) It[sl][2 * x + half][l1][l2] = in ? slab[sl][at] : 0.0;
   }
   if (tid < 72) {
     const int w = tid / 24, pos = (tid / 8) % 3, l = tid & 7;
@@ -231,38 +146,54 @@ __global__ void __launch_bounds__(128)
     es[pos][l] = g < v ? ev[g] : 0.0;
   }
   __syncthreads();
-  const double eijk = eo[i] + eo[j] + eo[k];
   double s4 = 0.0, s5 = 0.0;
+  const int b = b0[1] + l1, c = b0[2] + l2;
+  if (b < v && c <= b) {
+    // t1 values by [occupied][tile position] and integrals by [slab][pair]
+    double t[3][3], I[3][6];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int n = tid + 128 * q;
-    const int l[3] = {n >> 6, (n >> 3) & 7, n & 7};
-    const int a = b0[0] + l[0], b = b0[1] + l[1], c = b0[2] + l[2];
-    if (a >= v || b >= v || c >= v || a < b || b < c) continue;
-    double u[6], vd[6];
-#pragma unroll
-    for (int s = 0; s < 6; ++s) {
-      const int P0 = ordpos(s, 0), P1 = ordpos(s, 1), P2 = ordpos(s, 2);
-      u[s] = (double)cube[s][l[P0]][l[P1]][l[P2]];
-      const int p12 = P1 * 2 + (P2 > P1 ? P2 - 1 : P2), p02 = P0 * 2 + (P2 > P0 ? P2 - 1 : P2),
-                p01 = P0 * 2 + (P1 > P0 ? P1 - 1 : P1);
-      // V - W at (p0,p1,p2): t_i^p0 <jk|p1p2> + t_j^p1 <ik|p0p2> + t_k^p2 <ij|p0p1>
-      vd[s] = ts[0][P0][l[P0]] * It[0][p12][l[P1]][l[P2]] +
-              ts[1][P1][l[P1]] * It[1][p02][l[P0]][l[P2]] +
-              ts[2][P2][l[P2]] * It[2][p01][l[P0]][l[P1]];
+    for (int w = 0; w < 3; ++w) {
+      t[w][1] = ts[w][1][l1];
+      t[w][2] = ts[w][2][l2];
+      I[w][pairpos(1, 2)] = It[w][pairpos(1, 2)][l1][l2];
+      I[w][pairpos(2, 1)] = It[w][pairpos(2, 1)][l2][l1];
     }
-    const double D = eijk - es[0][l[0]] - es[1][l[1]] - es[2][l[2]];
-    double g4 = 0.0, g5 = 0.0;
-    if (a > b && b > c) {
-      form_apply(u, vd, g4, g5);
-    } else {
+    const double dbc = eo[i] + eo[j] + eo[k] - es[1][l1] - es[2][l2];
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      const int l0 = half + 2 * q, a = b0[0] + l0;
+      if (a >= v || a < b) continue;
+      const int l[3] = {l0, l1, l2};
+#pragma unroll
+      for (int w = 0; w < 3; ++w) {
+        t[w][0] = ts[w][0][l0];
+        I[w][pairpos(0, 1)] = It[w][pairpos(0, 1)][l0][l1];
+        I[w][pairpos(0, 2)] = It[w][pairpos(0, 2)][l0][l2];
+        I[w][pairpos(1, 0)] = It[w][pairpos(1, 0)][l1][l0];
+        I[w][pairpos(2, 0)] = It[w][pairpos(2, 0)][l2][l0];
+      }
+      double u[6];
+#pragma unroll
+      for (int s = 0; s < 6; ++s)
+        u[s] = (double)cube[s][l[ordpos(s, 0)]][l[ordpos(s, 1)]][l[ordpos(s, 2)]];
+      const double E = u[0] + u[3] + u[4], O = u[1] + u[2] + u[5];
+      const double pe = 6.0 * E - 12.0 * O, po = 6.0 * O - 12.0 * E;
+      double g4 = 0.0, g5 = 0.0;
+#pragma unroll
+      for (int s = 0; s < 6; ++s) {
+        const int P0 = ordpos(s, 0), P1 = ordpos(s, 1), P2 = ordpos(s, 2);
+        // V - W at (p0,p1,p2): t_i^p0 <jk|p1p2> + t_j^p1 <ik|p0p2> + t_k^p2 <ij|p0p1>
+        const double vd = t[0][P0] * I[0][pairpos(P1, P2)] + t[1][P1] * I[1][pairpos(P0, P2)] +
+                          t[2][P2] * I[2][pairpos(P0, P1)];
+        const double y = 18.0 * u[s] + (s == 0 || s == 3 || s == 4 ? pe : po);
+        g4 += y * u[s];
+        g5 += y * vd;
+      }
       const bool ab = a == b, bc = b == c;
-      const bool use[6] = {true, !bc, !ab, !ab, !bc, !(ab || bc)};
-      accum_sets<0>(use, u, vd, g4, g5);
+      const double inv = (ab && bc ? 1.0 / 6.0 : (ab || bc ? 0.5 : 1.0)) / (dbc - es[0][l0]);
+      s4 += g4 * inv;
+      s5 += g5 * inv;
     }
-    const double inv = 1.0 / D;
-    s4 += g4 * inv;
-    s5 += g5 * inv;
   }
   for (int off = 16; off; off >>= 1) {
     s4 += __shfl_down_sync(0xffffffffu, s4, off);
