@@ -8,6 +8,7 @@
 namespace acesb200 {
 
 namespace {
+constexpr int kZeroBufs = 64;
 __device__ __forceinline__ long long view_off(const CView &C, long long m, long long n) {
   return cview_off(C, (int)m, (int)n);
 }
@@ -57,6 +58,21 @@ __global__ void k_scale(double *__restrict__ y, double a, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = a == 0.0 ? 0.0 : a * y[i];
+}
+
+// zeroes up to kZeroBufs buffers in one launch (blockIdx.y selects one):
+// 16-byte stores, the pool's blocks being aligned to 512 bytes
+struct ZeroList {
+  double *p[kZeroBufs];
+  long long n[kZeroBufs];
+};
+__global__ void k_zero_many(ZeroList z) {
+  double *p = z.p[blockIdx.y];
+  const long long n = z.n[blockIdx.y], n2 = n / 2;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2;
+       i += (long long)gridDim.x * blockDim.x)
+    reinterpret_cast<double2 *>(p)[i] = make_double2(0.0, 0.0);
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) p[n - 1] = 0.0;
 }
 
 // t1_bar[i,a] += c * sum_jb taub[i,j,a,b] t1[j,b] + c * sum_jb taub[j,i,b,a] t1[j,b]
@@ -341,9 +357,76 @@ int CCEngine::backward() {
   return ACES_OK;
 }
 
+// one launch per 64 buffers (a backward pass of a small system starts with some
+// 45 of them: as many memsets took 75 us of its 1.2 ms)
 void CCEngine::zero_adjoints() {
-  for (auto &kv : adjoint)
-    if (kv.second.p) cudaMemsetAsync(kv.second.p, 0, kv.second.n * 8, st);
+  ZeroList z;
+  int n = 0;
+  long long most = 0;
+  auto flush = [&] {
+    if (n == 0) return;
+    const long long nb = std::min<long long>((most / 2 + 255) / 256 + 1, 148 * 8);
+    k_zero_many<<<dim3((unsigned)nb, n), 256, 0, st>>>(z);
+    count_launch();
+    n = 0;
+    most = 0;
+  };
+  for (auto &kv : adjoint) {
+    if (!kv.second.p) continue;
+    z.p[n] = kv.second.p;
+    z.n[n] = (long long)kv.second.n;
+    most = std::max(most, z.n[n]);
+    if (++n == kZeroBufs) flush();
+  }
+  flush();
+}
+
+void CCEngine::drop_backward_graph() {
+  if (backward_exec) cudaGraphExecDestroy(backward_exec);
+  backward_exec = nullptr;
+  backward_passes = 0;
+}
+
+// The reverse replay, directly or through its captured graph: every Lambda
+// iteration and EOM product replays the same tape on the same buffers (some
+// 200 launches; from the host they leave gaps as long as the kernels of a
+// small system).  The first pass allocates and fills the caches, the second
+// is captured; a new tape or another symmetry of the replayed vector starts
+// over.
+int CCEngine::backward_run() {
+  if (backward_sym != ladder_sym) {
+    drop_backward_graph();
+    backward_sym = ladder_sym;
+  }
+  if (backward_exec) {
+    ACES_CUDA(cudaGraphLaunch(backward_exec, st));
+    g_launches.fetch_add(backward_launches, std::memory_order_relaxed);
+    return ACES_OK;
+  }
+  if (backward_passes++ == 0) return backward();
+  const long long l0 = g_launches.load();
+  cudaGraph_t graph = nullptr;
+  ACES_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  const int s = backward();
+  const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+  if (s != ACES_OK) {
+    if (graph) cudaGraphDestroy(graph);
+    return s;
+  }
+  if (ce != cudaSuccess) {
+    set_error("backward graph capture failed: %s", cudaGetErrorString(ce));
+    return ACES_ERR_CUDA;
+  }
+  backward_launches = g_launches.load() - l0;
+  const cudaError_t ie = cudaGraphInstantiate(&backward_exec, graph, 0);
+  cudaGraphDestroy(graph);
+  if (ie != cudaSuccess) {
+    backward_exec = nullptr;
+    set_error("backward graph instantiation failed: %s", cudaGetErrorString(ie));
+    return ACES_ERR_CUDA;
+  }
+  ACES_CUDA(cudaGraphLaunch(backward_exec, st));
+  return ACES_OK;
 }
 
 }  // namespace acesb200

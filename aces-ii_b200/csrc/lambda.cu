@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(256)
 
 int CCEngine::record_residual(bool fock_active) {
   // the forward values the previous tape's backward pass cached may change
+  drop_backward_graph();
   tape_cache_clear();
   tape.clear();
   active.clear();
@@ -127,7 +128,7 @@ int CCEngine::lambda_rhs() {
   if (!z1b || !z2b) return ACES_ERR_NOMEM;
   launch_axpy(z1b, L.p, 1.0, ov, st);
   launch_axpy(z2b, L.p + ov, 1.0, len - ov, st);
-  ACES_TRY(backward());
+  ACES_TRY(backward_run());
   double *xb = adj(X.p);
   ACES_TRY(alloc(lrhs, len));
   ACES_CUDA(cudaMemcpyAsync(lrhs.p, gE.p, len * 8, cudaMemcpyDeviceToDevice, st));
