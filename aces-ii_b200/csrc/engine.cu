@@ -438,20 +438,9 @@ void pair_table(const SymInfo &s, int type, const std::vector<int> &irr_p,
     }
 }
 
-template <class T>
-int upload(T **d, const std::vector<T> &h) {
-  ACES_CUDA(dev_alloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(T)));
-  if (!h.empty()) ACES_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return ACES_OK;
-}
-
 }  // namespace
 
-DevMap::~DevMap() {
-  dev_free(d_rowidx); dev_free(d_colidx); dev_free(d_rowsgn); dev_free(d_colsgn);
-  for (int k = 0; k < 4; ++k) dev_free(d_irr[k]);
-  dev_free(d_base); dev_free(d_nrows);
-}
+DevMap::~DevMap() { dev_free(d_tab); }
 
 int make_map(DevMap &dm, int list, int typeL, int typeR, const std::vector<int> &irr_o,
              const std::vector<int> &irr_v, bool create) {
@@ -483,21 +472,36 @@ int make_map(DevMap &dm, int list, int typeL, int typeR, const std::vector<int> 
     base[h] = aces_list_devptr(h + 1, list);
     nrows[h] = nr;
   }
-  ACES_TRY(upload(&dm.d_rowidx, hm.rowidx));
-  ACES_TRY(upload(&dm.d_colidx, hm.colidx));
-  ACES_TRY(upload(&dm.d_rowsgn, hm.rowsgn));
-  ACES_TRY(upload(&dm.d_colsgn, hm.colsgn));
-  ACES_TRY(upload(&dm.d_irr[0], ip));
-  ACES_TRY(upload(&dm.d_irr[1], iq));
-  ACES_TRY(upload(&dm.d_irr[2], ir));
-  ACES_TRY(upload(&dm.d_irr[3], is));
-  ACES_TRY(upload(&dm.d_base, base));
-  ACES_TRY(upload(&dm.d_nrows, nrows));
-  dm.m.rowidx = dm.d_rowidx; dm.m.colidx = dm.d_colidx;
-  dm.m.rowsgn = dm.d_rowsgn; dm.m.colsgn = dm.d_colsgn;
-  dm.m.irr_p = dm.d_irr[0]; dm.m.irr_q = dm.d_irr[1];
-  dm.m.irr_r = dm.d_irr[2]; dm.m.irr_s = dm.d_irr[3];
-  dm.m.base = dm.d_base; dm.m.nrows = dm.d_nrows;
+  // the tables as one upload (a copy each were ten synchronous ones per list)
+  std::vector<char> tab;
+  auto put = [&](const void *src, size_t bytes) {
+    const size_t at = (tab.size() + 15) / 16 * 16;
+    tab.resize(at + bytes);
+    if (bytes) memcpy(tab.data() + at, src, bytes);
+    return at;
+  };
+  const size_t a_ri = put(hm.rowidx.data(), hm.rowidx.size() * sizeof(int)),
+               a_ci = put(hm.colidx.data(), hm.colidx.size() * sizeof(int)),
+               a_rs = put(hm.rowsgn.data(), hm.rowsgn.size()),
+               a_cs = put(hm.colsgn.data(), hm.colsgn.size()),
+               a_ip = put(ip.data(), ip.size() * sizeof(int)),
+               a_iq = put(iq.data(), iq.size() * sizeof(int)),
+               a_ir = put(ir.data(), ir.size() * sizeof(int)),
+               a_is = put(is.data(), is.size() * sizeof(int)),
+               a_b = put(base.data(), base.size() * sizeof(double *)),
+               a_n = put(nrows.data(), nrows.size() * sizeof(int));
+  ACES_CUDA(dev_alloc(&dm.d_tab, tab.size()));
+  // cudaMemcpy from pageable memory may return while its last transfer is in
+  // flight on stream 0, and the kernels that read the tables run on another
+  // stream: wait for it
+  ACES_CUDA(cudaMemcpyAsync(dm.d_tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, 0));
+  ACES_CUDA(cudaStreamSynchronize(0));
+  const char *d = (const char *)dm.d_tab;
+  dm.m.rowidx = (const int *)(d + a_ri); dm.m.colidx = (const int *)(d + a_ci);
+  dm.m.rowsgn = (const signed char *)(d + a_rs); dm.m.colsgn = (const signed char *)(d + a_cs);
+  dm.m.irr_p = (const int *)(d + a_ip); dm.m.irr_q = (const int *)(d + a_iq);
+  dm.m.irr_r = (const int *)(d + a_ir); dm.m.irr_s = (const int *)(d + a_is);
+  dm.m.base = (double *const *)(d + a_b); dm.m.nrows = (const int *)(d + a_n);
   dm.m.np = (int)ip.size(); dm.m.nq = (int)iq.size();
   dm.m.nr = (int)ir.size(); dm.m.ns = (int)is.size();
   return ACES_OK;

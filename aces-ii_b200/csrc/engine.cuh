@@ -221,11 +221,7 @@ constexpr long long kHugeView = 1LL << 62;  // CView divisor meaning "no split"
 // Device tables mapping the dense [p,q,r,s] index space of one DPD list onto
 // its irrep blocks (pair indices, signs, orbital irreps, block pointers).
 struct DevMap {
-  int *d_rowidx = nullptr, *d_colidx = nullptr;
-  signed char *d_rowsgn = nullptr, *d_colsgn = nullptr;
-  int *d_irr[4] = {nullptr, nullptr, nullptr, nullptr};
-  double **d_base = nullptr;
-  int *d_nrows = nullptr;
+  void *d_tab = nullptr;  // every table, one allocation
   DpdMap m;
   DevMap() = default;
   DevMap(const DevMap &) = delete;
