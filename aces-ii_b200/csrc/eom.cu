@@ -140,9 +140,18 @@ __global__ void __launch_bounds__(256)
 
 __global__ void k_multidot_final(double *__restrict__ c, const double *__restrict__ part, int m,
                                  double alpha) {
+  // every load in flight before the first addition
+  constexpr int kPer = (kDotBlocks + 31) / 32;
   const int r = blockIdx.x;
+  double v[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int b = threadIdx.x + 32 * u;
+    v[u] = b < kDotBlocks ? part[(long long)b * kMaxRows + r] : 0.0;
+  }
   double s = 0.0;
-  for (int b = threadIdx.x; b < kDotBlocks; b += 32) s += part[(long long)b * kMaxRows + r];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) s += v[u];
   for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
   if (threadIdx.x == 0) c[r] = alpha * s;
 }

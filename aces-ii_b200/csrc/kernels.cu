@@ -589,11 +589,20 @@ __global__ void __launch_bounds__(kPbThreads)
   block_reduce<3>(s, part + 3 * blockIdx.x);
 }
 
-__global__ void k_final_sum(double *out, const double *part, int nblk, int nv) {
-  // single warp per value, fixed order
-  int k = blockIdx.x;
+// out[k] = sum of the kRedBlocks partials of value k: a warp per value, every
+// load in flight before the first addition, fixed order
+constexpr int kPerLane = (kRedBlocks + 31) / 32;
+__global__ void k_final_sum(double *out, const double *part, int nv) {
+  const int k = blockIdx.x;
+  double v[kPerLane];
+#pragma unroll
+  for (int u = 0; u < kPerLane; ++u) {
+    const int b = threadIdx.x + 32 * u;
+    v[u] = b < kRedBlocks ? part[(long long)b * nv + k] : 0.0;
+  }
   double x = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += 32) x += part[(long long)b * nv + k];
+#pragma unroll
+  for (int u = 0; u < kPerLane; ++u) x += v[u];
   for (int off = 16; off; off >>= 1) x += __shfl_down_sync(0xffffffff, x, off);
   if (threadIdx.x == 0) out[k] = x;
 }
@@ -603,7 +612,7 @@ void launch_energy(double *out3, const double *t2, const double *t1, const doubl
   const PairBlocks P = pair_blocks(o, v, true);
   k_energy<<<kRedBlocks, kPbThreads, 0, st>>>(scratch, t2, t1, voovv, fov, P);
   count_launch();
-  k_final_sum<<<3, 32, 0, st>>>(out3, scratch, kRedBlocks, 3); count_launch();
+  k_final_sum<<<3, 32, 0, st>>>(out3, scratch, 3); count_launch();
 }
 
 // xn = x + damp (xn - x), two loads and a store per element
@@ -632,12 +641,22 @@ __device__ inline void amax_merge(double &bv, long long &bi, double v, long long
   }
 }
 
-// one warp; amax_merge orders candidates by (|value| descending, index
-// ascending), a total order, so the merge order does not change the result
-__global__ void k_absmax_final(double *out, const double *pv, const long long *pi, int nb) {
+// one warp over the kRedBlocks candidates, every load in flight first;
+// amax_merge orders candidates by (|value| descending, index ascending), a
+// total order, so the merge order does not change the result
+__global__ void k_absmax_final(double *out, const double *pv, const long long *pi) {
+  double v[kPerLane];
+  long long w[kPerLane];
+#pragma unroll
+  for (int u = 0; u < kPerLane; ++u) {
+    const int b = threadIdx.x + 32 * u;
+    v[u] = b < kRedBlocks ? pv[b] : 0.0;
+    w[u] = b < kRedBlocks ? pi[b] : 0x7fffffffffffffffLL;
+  }
   double bv = 0.0;
   long long bi = 0x7fffffffffffffffLL;
-  for (int b = threadIdx.x; b < nb; b += 32) amax_merge(bv, bi, pv[b], pi[b]);
+#pragma unroll
+  for (int u = 0; u < kPerLane; ++u) amax_merge(bv, bi, v[u], w[u]);
   for (int off = 16; off; off >>= 1) {
     double ov = __shfl_down_sync(0xffffffff, bv, off);
     long long oi = __shfl_down_sync(0xffffffff, bi, off);
@@ -795,9 +814,9 @@ int launch_diff_stats(double *e, const double *xnew, const double *xold,
   const PairBlocks P = pair_blocks(o, v, true);
   k_diff_stats<<<kRedBlocks, kPbThreads, 0, st>>>(e, xnew, xold, h, nh, self, P, part, pv, pi);
   count_launch();
-  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi, kRedBlocks);
+  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi);
   count_launch();
-  k_final_sum<<<nh, 32, 0, st>>>(dots_out, part, kRedBlocks, 25);
+  k_final_sum<<<nh, 32, 0, st>>>(dots_out, part, 25);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -872,7 +891,7 @@ void launch_lincomb_absmax(double *out, const double *c, const double *const *p,
   const PairBlocks P = pair_blocks(o, v, true);
   k_lincomb_absmax<<<kRedBlocks, kPbThreads, 0, st>>>(out, c, a, n, P, pv, pi);
   count_launch();
-  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi, kRedBlocks);
+  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi);
   count_launch();
 }
 
