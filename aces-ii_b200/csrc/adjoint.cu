@@ -14,6 +14,7 @@ __device__ __forceinline__ long long view_off(const CView &C, long long m, long 
 }
 
 __global__ void k_view_gather(double *__restrict__ dense, CView C, int M, int N, double scale) {
+  after_previous();
   long long total = (long long)M * N;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -23,6 +24,7 @@ __global__ void k_view_gather(double *__restrict__ dense, CView C, int M, int N,
 }
 
 __global__ void k_view_scale(CView C, int M, int N, double value) {
+  after_previous();
   long long total = (long long)M * N;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -35,6 +37,7 @@ __global__ void k_view_scale(CView C, int M, int N, double value) {
 __global__ void k_perm_scatter_add(double *__restrict__ src_bar, const double *__restrict__ out_bar,
                                    double alpha, long long s0, long long s1, long long s2,
                                    long long s3, int n0, int n1, int n2, int n3) {
+  after_previous();
   long long total = (long long)n0 * n1 * n2 * n3;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -49,12 +52,14 @@ __global__ void k_perm_scatter_add(double *__restrict__ src_bar, const double *_
 }
 
 __global__ void k_axpy(double *__restrict__ y, const double *__restrict__ x, double a, long long n) {
+  after_previous();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] += a * x[i];
 }
 
 __global__ void k_scale(double *__restrict__ y, double a, long long n) {
+  after_previous();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     y[i] = a == 0.0 ? 0.0 : a * y[i];
@@ -67,6 +72,7 @@ struct ZeroList {
   long long n[kZeroBufs];
 };
 __global__ void k_zero_many(ZeroList z) {
+  after_previous();
   double *p = z.p[blockIdx.y];
   const long long n = z.n[blockIdx.y], n2 = n / 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2;
@@ -79,6 +85,7 @@ __global__ void k_zero_many(ZeroList z) {
 // one block per (i,a)
 __global__ void k_tau_adj_t1(double *__restrict__ t1_bar, const double *__restrict__ taub,
                              const double *__restrict__ t1, double c, int o, int v) {
+  after_previous();
   int ia = blockIdx.x;
   int i = ia / v, a = ia % v;
   double s = 0.0;
@@ -108,26 +115,26 @@ unsigned blocks_for(long long n) {
 
 void launch_view_gather(double *dense, const CView &C, int M, int N, double scale,
                         cudaStream_t st) {
-  k_view_gather<<<blocks_for((long long)M * N), 256, 0, st>>>(dense, C, M, N, scale);
+  launch_after(k_view_gather, blocks_for((long long)M * N), 256, 0, st, dense, C, M, N, scale);
   count_launch();
 }
 void launch_view_scale(const CView &C, int M, int N, double value, cudaStream_t st) {
-  k_view_scale<<<blocks_for((long long)M * N), 256, 0, st>>>(C, M, N, value);
+  launch_after(k_view_scale, blocks_for((long long)M * N), 256, 0, st, C, M, N, value);
   count_launch();
 }
 void launch_perm_scatter_add(double *src_bar, const double *out_bar, const PermTerm &t,
                              const int n[4], cudaStream_t st) {
   long long total = (long long)n[0] * n[1] * n[2] * n[3];
-  k_perm_scatter_add<<<blocks_for(total), 256, 0, st>>>(src_bar, out_bar, t.alpha, t.s[0], t.s[1],
-                                                        t.s[2], t.s[3], n[0], n[1], n[2], n[3]);
+  launch_after(k_perm_scatter_add, blocks_for(total), 256, 0, st, src_bar, out_bar, t.alpha, t.s[0],
+               t.s[1], t.s[2], t.s[3], n[0], n[1], n[2], n[3]);
   count_launch();
 }
 void launch_axpy(double *y, const double *x, double a, long long n, cudaStream_t st) {
-  k_axpy<<<blocks_for(n), 256, 0, st>>>(y, x, a, n);
+  launch_after(k_axpy, blocks_for(n), 256, 0, st, y, x, a, n);
   count_launch();
 }
 void launch_scale(double *y, double a, long long n, cudaStream_t st) {
-  k_scale<<<blocks_for(n), 256, 0, st>>>(y, a, n);
+  launch_after(k_scale, blocks_for(n), 256, 0, st, y, a, n);
   count_launch();
 }
 void launch_tau_adjoint(double *t2_bar, double *t1_bar, const double *tau_bar, const double *t1,
@@ -135,7 +142,7 @@ void launch_tau_adjoint(double *t2_bar, double *t1_bar, const double *tau_bar, c
   long long n = (long long)o * o * v * v;
   if (t2_bar) launch_axpy(t2_bar, tau_bar, 1.0, n, st);
   if (t1_bar) {
-    k_tau_adj_t1<<<o * v, 256, 0, st>>>(t1_bar, tau_bar, t1, c, o, v);
+    launch_after(k_tau_adj_t1, o * v, 256, 0, st, t1_bar, tau_bar, t1, c, o, v);
     count_launch();
   }
 }
@@ -366,7 +373,7 @@ void CCEngine::zero_adjoints() {
   auto flush = [&] {
     if (n == 0) return;
     const long long nb = std::min<long long>((most / 2 + 255) / 256 + 1, 148 * 8);
-    k_zero_many<<<dim3((unsigned)nb, n), 256, 0, st>>>(z);
+    launch_after(k_zero_many, dim3((unsigned)nb, n), 256, 0, st, z);
     count_launch();
     n = 0;
     most = 0;

@@ -48,6 +48,7 @@ __global__ void k_eom_combine(double *out, const double *g,
                               const double *__restrict__ ev, const int *__restrict__ irr_o,
                               const int *__restrict__ irr_v, int h, int o, int v,
                               long long len) {
+  after_previous();
   const long long ov = (long long)o * v;
   for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < len;
        n += (long long)gridDim.x * blockDim.x) {
@@ -77,6 +78,7 @@ __global__ void k_eom_precond(double *__restrict__ dvec, const double *__restric
                               const double *__restrict__ ev, const int *__restrict__ irr_o,
                               const int *__restrict__ irr_v, int h, int o, int v,
                               long long len) {
+  after_previous();
   const long long ov = (long long)o * v;
   for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < len;
        n += (long long)gridDim.x * blockDim.x) {
@@ -110,6 +112,7 @@ constexpr int kMaxRows = 64, kDotBlocks = 592;
 __global__ void __launch_bounds__(256)
     k_multidot(double *__restrict__ part, const double *__restrict__ A, long long lda,
                const double *__restrict__ y, long long len, int m) {
+  after_previous();
   __shared__ double sh[kMaxRows][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0)
@@ -140,6 +143,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void k_multidot_final(double *__restrict__ c, const double *__restrict__ part, int m,
                                  double alpha) {
+  after_previous();
   // every load in flight before the first addition
   constexpr int kPer = (kDotBlocks + 31) / 32;
   const int r = blockIdx.x;
@@ -191,8 +195,8 @@ int CCEngine::eom_sigma(const double *x, double *out, int h, const int *d_irr_o,
   ps.t[0] = PermTerm{g + ov, 0.5, {s2[0], s2[1], s2[2], s2[3]}};
   ps.t[1] = PermTerm{g + ov, 0.5, {s2[1], s2[0], s2[3], s2[2]}};
   ACES_TRY(permute(out + ov, ps, st));
-  k_eom_combine<<<grid_for(len), 256, 0, st>>>(out, out, x, eo.p, ev.p, d_irr_o, d_irr_v, h, o,
-                                               v, len);
+  launch_after(k_eom_combine, grid_for(len), 256, 0, st, out, out, x, eo.p, ev.p, d_irr_o, d_irr_v,
+               h, o, v, len);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -265,9 +269,10 @@ extern "C" int xvee_run(aces_eom_config *cfg) {
     // c[k] = alpha sum_n A[k*len + n] y[n] for k < m, m <= kMaxRows at a time
     for (int r0 = 0; r0 < m; r0 += kMaxRows) {
       const int mr = std::min(kMaxRows, m - r0);
-      k_multidot<<<kDotBlocks, 256, 0, E.st>>>(dpart.p, A + (size_t)r0 * len, len, y, len, mr);
+      launch_after(k_multidot, kDotBlocks, 256, 0, E.st, dpart.p, A + (size_t)r0 * len, len, y, len,
+                   mr);
       count_launch();
-      k_multidot_final<<<mr, 32, 0, E.st>>>(c + r0, dpart.p, mr, alpha);
+      launch_after(k_multidot_final, mr, 32, 0, E.st, c + r0, dpart.p, mr, alpha);
       count_launch();
     }
     ACES_CUDA(cudaGetLastError());
@@ -380,8 +385,8 @@ extern "C" int xvee_run(aces_eom_config *cfg) {
         if (rn[r] > tol || std::fabs(wsel[r] - w_old[r]) > tol) {
           done = false;
           if (m < maxdim) {
-            k_eom_precond<<<grid_for(len), 256, 0, E.st>>>(dv.p, rv.p, wsel[r], E.eo.p, E.ev.p,
-                                                           d_irr_o, d_irr_v, h, o, v, len);
+            launch_after(k_eom_precond, grid_for(len), 256, 0, E.st, dv.p, rv.p, wsel[r], E.eo.p,
+                         E.ev.p, d_irr_o, d_irr_v, h, o, v, len);
             count_launch();
             ACES_CUDA(cudaGetLastError());
             // Gram-Schmidt against the subspace, twice

@@ -132,6 +132,7 @@ struct F64Launch {
 template <class T, int VEC>
 __global__ void __launch_bounds__(T::kThreads, T::OCC)
     k_gemm_f64(const __grid_constant__ F64Launch L) {
+  after_previous();
   constexpr int BM = T::BM, BN = T::BN, MI = T::MI, NI = T::NI;
   extern __shared__ __align__(128) unsigned char f64_smem[];
   int t = blockIdx.x;
@@ -319,7 +320,7 @@ int launch_tile(const F64Launch &L, unsigned tiles, unsigned z, cudaStream_t st)
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
     attr_set[dev] = true;
   }
-  k_gemm_f64<T, VEC><<<dim3(tiles, z), T::kThreads, T::kSmem, st>>>(L);
+  launch_after(k_gemm_f64<T, VEC>, dim3(tiles, z), T::kThreads, T::kSmem, st, L);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -333,6 +334,7 @@ int launch_tile(const F64Launch &L, unsigned tiles, unsigned z, cudaStream_t st)
 template <bool Wide>
 __global__ void k_splitk_reduce(CView C, const double *__restrict__ part, int M, int N, int Z,
                                 double alpha, double beta, bool mfast, FastDiv fd) {
+  after_previous();
   const long long total = (long long)M * N;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -369,6 +371,7 @@ __global__ void k_splitk_reduce(CView C, const double *__restrict__ part, int M,
 __global__ void k_gemv_f64(int M, int K, double alpha, const double *__restrict__ A,
                            long long lda, const double *__restrict__ x, double beta, CView C,
                            bool transpose_out) {
+  after_previous();
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int m = warp; m < M; m += nwarps) {
@@ -401,6 +404,7 @@ __global__ void k_gemv_f64(int M, int K, double alpha, const double *__restrict_
 __global__ void k_gemv_part(int M, int K, int W, int kc, const double *__restrict__ A,
                             long long lda, const double *__restrict__ x,
                             double *__restrict__ part) {
+  after_previous();
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= (long long)M * W) return;  // warp-uniform
@@ -424,6 +428,7 @@ __global__ void k_gemv_part(int M, int K, int W, int kc, const double *__restric
 // y[m] = alpha * sum_c part[m * W + c] + beta * y[m], the chunks summed in order
 __global__ void k_gemv_final(int M, int W, double alpha, const double *__restrict__ part,
                              double beta, CView C, bool transpose_out) {
+  after_previous();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   double t = 0.0;
@@ -444,6 +449,7 @@ constexpr long long kTinyOut = 8192;
 __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double *__restrict__ A,
                                 long long lda, const double *__restrict__ B, long long ldb,
                                 double beta, CView C) {
+  after_previous();
   const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= M * N) return;  // warp-uniform
@@ -478,6 +484,7 @@ __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double 
 // part[z][m][n], or part[z][n][m] with mfast.
 __global__ void k_reduce_warp(CView C, const double *__restrict__ part, int M, int N, int Z,
                               double alpha, double beta, bool mfast) {
+  after_previous();
   const long long total = (long long)M * N;
   const int lane = threadIdx.x & 31;
   for (long long idx = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; idx < total;
@@ -501,7 +508,7 @@ static void launch_reduce_warp(const CView &C, const double *part, int M, int N,
   const long long total = (long long)M * N;
   long long nb = (total + 7) / 8;  // 8 warps per block
   if (nb > 148 * 32) nb = 148 * 32;
-  k_reduce_warp<<<(unsigned)nb, 256, 0, st>>>(C, part, M, N, Z, alpha, beta, mfast);
+  launch_after(k_reduce_warp, (unsigned)nb, 256, 0, st, C, part, M, N, Z, alpha, beta, mfast);
   count_launch();
 }
 
@@ -521,6 +528,7 @@ __global__ void __launch_bounds__(LR_F)
     k_gemm_lowrank_f64(int M, int N, int K, double alpha, const double *__restrict__ A,
                        long long lda, const double *__restrict__ B, long long ldb, double beta,
                        CView C, bool fast_is_m, int tiles_f) {
+  after_previous();
   extern __shared__ double lr_smem[];
   const int ks = K | 1;  // odd row stride: column reads across threads are conflict free
   double *Fs = lr_smem;              // [LR_F][ks]
@@ -606,8 +614,8 @@ static int launch_lowrank(int M, int N, int K, double alpha, const double *A, lo
     return ACES_ERR_ARG;
   }
   const size_t smem = (size_t)(LR_F + LR_S) * (K | 1) * sizeof(double);
-  k_gemm_lowrank_f64<<<(unsigned)nb, LR_F, smem, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C,
-                                                       fast_is_m, tiles_f);
+  launch_after(k_gemm_lowrank_f64, (unsigned)nb, LR_F, smem, st, M, N, K, alpha, A, lda, B, ldb,
+               beta, C, fast_is_m, tiles_f);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -659,9 +667,11 @@ int splitk_reduce(const CView &C, const double *part, int M, int N, int Z, doubl
   if (nb > 148 * 16) nb = 148 * 16;
   const FastDiv fd((unsigned)std::max(1, mfast ? M : N));
   if (total < (1LL << 31))
-    k_splitk_reduce<false><<<(unsigned)nb, 256, 0, st>>>(C, part, M, N, Z, alpha, beta, mfast, fd);
+    launch_after(k_splitk_reduce<false>, (unsigned)nb, 256, 0, st, C, part, M, N, Z, alpha, beta,
+                 mfast, fd);
   else
-    k_splitk_reduce<true><<<(unsigned)nb, 256, 0, st>>>(C, part, M, N, Z, alpha, beta, mfast, fd);
+    launch_after(k_splitk_reduce<true>, (unsigned)nb, 256, 0, st, C, part, M, N, Z, alpha, beta,
+                 mfast, fd);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -684,11 +694,11 @@ int gemv_f64(int M, int K, double alpha, const double *A, long long lda, const d
         return ACES_ERR_NOMEM;
       }
       const long long nw = (long long)M * W;
-      k_gemv_part<<<(unsigned)((nw * 32 + 255) / 256), 256, 0, st>>>(M, K, W, kc, A, lda, x,
-                                                                      part);
+      launch_after(k_gemv_part, (unsigned)((nw * 32 + 255) / 256), 256, 0, st, M, K, W, kc, A, lda,
+                   x, part);
       count_launch();
-      k_gemv_final<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(M, W, alpha, part, beta, C,
-                                                                transpose_out);
+      launch_after(k_gemv_final, (unsigned)((M + 255) / 256), 256, 0, st, M, W, alpha, part, beta,
+                   C, transpose_out);
       count_launch();
       ACES_CUDA(cudaGetLastError());
       return ACES_OK;
@@ -697,7 +707,8 @@ int gemv_f64(int M, int K, double alpha, const double *A, long long lda, const d
   long long warps = M;
   long long nb = (warps * 32 + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
-  k_gemv_f64<<<(unsigned)nb, 256, 0, st>>>(M, K, alpha, A, lda, x, beta, C, transpose_out);
+  launch_after(k_gemv_f64, (unsigned)nb, 256, 0, st, M, K, alpha, A, lda, x, beta, C,
+               transpose_out);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -799,8 +810,8 @@ int gemm_dispatch(int M, int N, int K, double alpha, const double *A, long long 
   if (M <= 0 || N <= 0) return ACES_OK;
   // a few thousand outputs: one warp each (no tiles, no split K)
   if ((long long)M * N <= kTinyOut && K > 0 && K <= 8192) {
-    k_gemm_tiny_f64<<<(unsigned)(((long long)M * N * 32 + 255) / 256), 256, 0, st>>>(
-        M, N, K, alpha, A, lda, B, ldb, beta, C);
+    launch_after(k_gemm_tiny_f64, (unsigned)(((long long)M * N * 32 + 255) / 256), 256, 0, st, M, N,
+                 K, alpha, A, lda, B, ldb, beta, C);
     count_launch();
     ACES_CUDA(cudaGetLastError());
     return ACES_OK;

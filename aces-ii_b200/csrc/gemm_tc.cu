@@ -47,6 +47,7 @@ template <bool Wide>
 __global__ void k_split_pack(__nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo,
                              const double *__restrict__ src, long long ld, int k,
                              long long total_pairs, FastDiv fpairs) {
+  after_previous();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total_pairs;
        idx += (long long)gridDim.x * blockDim.x) {
     long long r;
@@ -76,6 +77,7 @@ __global__ void k_split_pack(__nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__
 __global__ void __launch_bounds__(256)
     k_split_pack_t(__nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo,
                    const double *__restrict__ src, long long ld, int rows, int k, int kp) {
+  after_previous();
   __shared__ double T[64][65];   // [r][c]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long r0 = blockIdx.x * 64LL;
@@ -143,11 +145,11 @@ int split_pack(SplitOperand &op, const double *src, long long ld, int rows, int 
   if (nb > 148 * 32) nb = 148 * 32;
   const FastDiv fp((unsigned)(kp / 2));
   if (pairs < (1LL << 31))
-    k_split_pack<false><<<(unsigned)nb, 256, 0, st>>>(
-        (__nv_bfloat162 *)op.hi, (__nv_bfloat162 *)op.lo, src, ld, k, pairs, fp);
+    launch_after(k_split_pack<false>, (unsigned)nb, 256, 0, st, (__nv_bfloat162 *)op.hi,
+                 (__nv_bfloat162 *)op.lo, src, ld, k, pairs, fp);
   else
-    k_split_pack<true><<<(unsigned)nb, 256, 0, st>>>(
-        (__nv_bfloat162 *)op.hi, (__nv_bfloat162 *)op.lo, src, ld, k, pairs, fp);
+    launch_after(k_split_pack<true>, (unsigned)nb, 256, 0, st, (__nv_bfloat162 *)op.hi,
+                 (__nv_bfloat162 *)op.lo, src, ld, k, pairs, fp);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -160,9 +162,10 @@ int split_pack_t(SplitOperand &op, const double *src, long long ld, int rows, in
   // column tiles in grid.y (at most 65535 = 4.2 M columns) per launch
   for (int t0 = 0; t0 < ct; t0 += 65535) {
     const int n = std::min(65535, ct - t0);
-    k_split_pack_t<<<dim3((unsigned)((rows + 63LL) / 64), n), 256, 0, st>>>(
-        (__nv_bfloat162 *)op.hi + (size_t)t0 * 32, (__nv_bfloat162 *)op.lo + (size_t)t0 * 32,
-        src + (long long)t0 * 64 * ld, ld, rows, k - t0 * 64, op.k_pad);
+    launch_after(k_split_pack_t, dim3((unsigned)((rows + 63LL) / 64), n), 256, 0, st,
+                 (__nv_bfloat162 *)op.hi + (size_t)t0 * 32,
+                 (__nv_bfloat162 *)op.lo + (size_t)t0 * 32, src + (long long)t0 * 64 * ld, ld, rows,
+                 k - t0 * 64, op.k_pad);
     count_launch();
   }
   ACES_CUDA(cudaGetLastError());
@@ -797,6 +800,7 @@ template <int CG, int BN>
 __global__ void __launch_bounds__(block_threads<BN>(), 1)
     k_gemm_bf16x3(const __grid_constant__ Launch L, double alpha, double beta,
                   double *__restrict__ part) {
+  after_previous();
   static_assert((CG == 2 && (BN == TBN || BN == TBN_WIDE)) || (CG == 1 && BN == TBN_1),
                 "tile variants");
   constexpr int kEpiWarps = epi_warps<BN>(), kCols = epi_cols<BN>();
@@ -1162,6 +1166,7 @@ constexpr int kTailCols = 8;
 __global__ void __launch_bounds__(TBM)
     k_tail_reduce(CView C, const double *__restrict__ part, int M, int N, int tilesM, int tilesN,
                   int mfast, int tail0, int Z, double alpha, double beta) {
+  after_previous();
   const int i = blockIdx.x, tl = tail0 + i;
   const int tm = mfast ? tl % tilesM : tl / tilesN, tn = mfast ? tl / tilesM : tl % tilesN;
   const int m = tm * TBM + (int)threadIdx.x, n0 = tn * TBN_1 + blockIdx.y * kTailCols;
@@ -1432,8 +1437,8 @@ int launch_prepared(Launch &L, double alpha, double beta, double *part, cudaStre
     ACES_TRY(launch_pairs<TBN>(L, alpha, beta, part, st));
   } else {
     const unsigned grid = (unsigned)std::min(L.nTiles, num_sms());
-    k_gemm_bf16x3<1, TBN_1>
-        <<<grid, block_threads<TBN_1>(), Geom<1, TBN_1>::kSmem, st>>>(L, alpha, beta, part);
+    launch_after(k_gemm_bf16x3<1, TBN_1>, grid, block_threads<TBN_1>(), Geom<1, TBN_1>::kSmem, st,
+                 L, alpha, beta, part);
   }
   count_launch();
   ACES_CUDA(cudaGetLastError());
@@ -1653,9 +1658,8 @@ size_t tail_doubles(const Problem &P) {
 int tail_reduce(const Problem &P, const double *part, double alpha, double beta,
                 cudaStream_t st) {
   const int tail = P.tilesM * P.tilesN - P.tail0;
-  k_tail_reduce<<<dim3(tail, TBN_1 / kTailCols), TBM, 0, st>>>(P.C, part, P.M, P.N, P.tilesM,
-                                                              P.tilesN, P.mfast, P.tail0,
-                                                              P.tailZ, alpha, beta);
+  launch_after(k_tail_reduce, dim3(tail, TBN_1 / kTailCols), TBM, 0, st, P.C, part, P.M, P.N,
+               P.tilesM, P.tilesN, P.mfast, P.tail0, P.tailZ, alpha, beta);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;

@@ -56,6 +56,7 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
 __global__ void __launch_bounds__(256)
     k_factor_stats(const double *__restrict__ B, int naux, int n,
                    unsigned long long *__restrict__ stats) {
+  after_previous();
   __shared__ double T[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int tiles = (n + 31) / 32;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_factor_pack(double *__restrict__ F, const double *__restrict__ B,
                   const int2 *__restrict__ rows, int nrows, int naux, int kp, int n) {
+  after_previous();
   __shared__ double T[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int r0 = blockIdx.x * 32, L0 = blockIdx.y * 32;
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256)
     k_expand_pairs(double *__restrict__ out, const double *__restrict__ G, long long ldg,
                    const int2 *__restrict__ rows, int x0, int y0, int n, long long sx,
                    long long sy, long long sc, int swap) {
+  after_previous();
   __shared__ double X[32][33];   // [c local][a local]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int2 pr = rows[blockIdx.x];
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(256)
     k_expand_irrep(double *__restrict__ out, GBlocks g, const int2 *__restrict__ rowtab,
                    const int2 *__restrict__ coltab, int nrows, int ncols,
                    const int *__restrict__ pidx, const int *__restrict__ irr, int n) {
+  after_previous();
   const int ri = blockIdx.x * 256 + threadIdx.x;
   if (ri >= nrows) return;
   const int2 pq = rowtab[ri];
@@ -272,7 +276,8 @@ int produce_packed(const double *dB, int naux, const std::vector<int> &irr_o,
   auto *d_stats = (unsigned long long *)mem.get(16);
   if (!d_stats) return ACES_OK;
   ACES_CUDA(cudaMemsetAsync(d_stats, 0, 16, st));
-  k_factor_stats<<<dim3(tri_tiles(n), std::min(naux, 64)), 256, 0, st>>>(dB, naux, n, d_stats);
+  launch_after(k_factor_stats, dim3(tri_tiles(n), std::min(naux, 64)), 256, 0, st, dB, naux, n,
+               d_stats);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   double stats[2];
@@ -340,8 +345,8 @@ int produce_packed(const double *dB, int naux, const std::vector<int> &irr_o,
   ACES_CUDA(cudaMemcpyAsync(d_ints, ints.data(), ints.size() * 4, cudaMemcpyHostToDevice, st));
   ACES_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(F64Task),
                             cudaMemcpyHostToDevice, st));
-  k_factor_pack<<<dim3((nrows + 31) / 32, (kp + 31) / 32), 256, 0, st>>>(F, dB, d_tab, nrows,
-                                                                        naux, kp, n);
+  launch_after(k_factor_pack, dim3((nrows + 31) / 32, (kp + 31) / 32), 256, 0, st, F, dB, d_tab,
+               nrows, naux, kp, n);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   // ---- one irrep: list offset of (pair (x,y) of the row, matrix (c,a) of the columns)
@@ -361,9 +366,8 @@ int produce_packed(const double *dB, int naux, const std::vector<int> &irr_o,
       const int R = cnt[P.R][0], tp = tri_tiles(m);
       // enough blocks for the machine, few tile pairs each when there are many rows
       const int ny = std::max(1, std::min(tp, (148 * 16 + R - 1) / R));
-      k_expand_pairs<<<dim3(R, ny), 256, 0, st>>>(base[k], G + goff[k][0], cnt[P.C][0],
-                                                  d_tab + off[P.R][0], x0, y0, m, sx, sy, sc,
-                                                  P.R != 1);
+      launch_after(k_expand_pairs, dim3(R, ny), 256, 0, st, base[k], G + goff[k][0], cnt[P.C][0],
+                   d_tab + off[P.R][0], x0, y0, m, sx, sy, sc, P.R != 1);
       count_launch();
     } else {
       GBlocks gb{};
@@ -379,9 +383,9 @@ int produce_packed(const double *dB, int naux, const std::vector<int> &irr_o,
         int nc = 0, nr = 0;
         aces_list_dims(h + 1, P.list, &nc, &nr);
         if (nc > 0 && nr > 0) {
-          k_expand_irrep<<<dim3((nr + 255) / 256, std::min(nc, 32768)), 256, 0, st>>>(
-              aces_list_devptr(h + 1, P.list), gb, d_tab + ra, d_tab + ca, nr, nc, d_ints,
-              d_ints + (size_t)n * n, n);
+          launch_after(k_expand_irrep, dim3((nr + 255) / 256, std::min(nc, 32768)), 256, 0, st,
+                       aces_list_devptr(h + 1, P.list), gb, d_tab + ra, d_tab + ca, nr, nc, d_ints,
+                       d_ints + (size_t)n * n, n);
           count_launch();
         }
         ra += nr;

@@ -51,6 +51,7 @@ __device__ __forceinline__ void put_split(const SplitOut &so, long long idx, dou
 template <bool Wide, bool S>
 __global__ void k_permute_naive(double *__restrict__ out, PermArgs a, long long total,
                                 SplitOut so) {
+  after_previous();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     int i0, i1, i2, i3;
@@ -84,6 +85,7 @@ __global__ void k_permute_naive(double *__restrict__ out, PermArgs a, long long 
 template <bool S>
 __global__ void k_permute_rows4(double *__restrict__ out, PermArgs a, long long quads,
                                 SplitOut so) {
+  after_previous();
   for (long long qd = blockIdx.x * (long long)blockDim.x + threadIdx.x; qd < quads;
        qd += (long long)gridDim.x * blockDim.x) {
     const long long idx = qd * 4;
@@ -140,6 +142,7 @@ __global__ void k_permute_rows4(double *__restrict__ out, PermArgs a, long long 
 template <int D, bool S, int R>
 __global__ void __launch_bounds__(256) k_permute_tiled(double *__restrict__ out, PermArgs a,
                                                        SplitOut so) {
+  after_previous();
   __shared__ double tile[32][R + 1];
   constexpr int kL = R / 8;  // loads per thread and term (rows i3 = ty + 8 k)
   const int nd = a.n[D];
@@ -240,13 +243,13 @@ static void permute_launch(double *out, PermArgs &a, const PermSpec &spec, long 
       if (k != D) nb *= a.n[k];
     dim3 blk(32, 8);
     if (R == 64) {
-      if (D == 0) k_permute_tiled<0, S, 64><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
-      if (D == 1) k_permute_tiled<1, S, 64><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
-      if (D == 2) k_permute_tiled<2, S, 64><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
+      if (D == 0) launch_after(k_permute_tiled<0, S, 64>, (unsigned)nb, blk, 0, st, out, a, so);
+      if (D == 1) launch_after(k_permute_tiled<1, S, 64>, (unsigned)nb, blk, 0, st, out, a, so);
+      if (D == 2) launch_after(k_permute_tiled<2, S, 64>, (unsigned)nb, blk, 0, st, out, a, so);
     } else {
-      if (D == 0) k_permute_tiled<0, S, 32><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
-      if (D == 1) k_permute_tiled<1, S, 32><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
-      if (D == 2) k_permute_tiled<2, S, 32><<<(unsigned)nb, blk, 0, st>>>(out, a, so);
+      if (D == 0) launch_after(k_permute_tiled<0, S, 32>, (unsigned)nb, blk, 0, st, out, a, so);
+      if (D == 1) launch_after(k_permute_tiled<1, S, 32>, (unsigned)nb, blk, 0, st, out, a, so);
+      if (D == 2) launch_after(k_permute_tiled<2, S, 32>, (unsigned)nb, blk, 0, st, out, a, so);
     }
     count_launch();
   } else {
@@ -257,11 +260,11 @@ static void permute_launch(double *out, PermArgs &a, const PermSpec &spec, long 
     if (rows4) {
       long long nq = (total / 4 + 255) / 256;
       if (nq > 148 * 64) nq = 148 * 64;
-      k_permute_rows4<S><<<(unsigned)nq, 256, 0, st>>>(out, a, total / 4, so);
+      launch_after(k_permute_rows4<S>, (unsigned)nq, 256, 0, st, out, a, total / 4, so);
     } else if (S || total < (1LL << 31)) {
-      k_permute_naive<false, S><<<(unsigned)nb, 256, 0, st>>>(out, a, total, so);
+      launch_after(k_permute_naive<false, S>, (unsigned)nb, 256, 0, st, out, a, total, so);
     } else {
-      k_permute_naive<true, false><<<(unsigned)nb, 256, 0, st>>>(out, a, total, so);
+      launch_after(k_permute_naive<true, false>, (unsigned)nb, 256, 0, st, out, a, total, so);
     }
     count_launch();
   }
@@ -390,6 +393,7 @@ inline unsigned pb_grid(long long nunits, int per_sm) {
 __global__ void __launch_bounds__(kPbThreads)
     k_tau(double *__restrict__ tau, const double *__restrict__ t2,
           const double *__restrict__ t1, double c, PairBlocks P) {
+  after_previous();
   for (long long u = blockIdx.x; u < P.nunits; u += gridDim.x) {
     const long long p = u / P.nchunk;
     const int ab0 = (int)(u - p * P.nchunk) * kPbChunk + threadIdx.x;
@@ -416,7 +420,7 @@ void launch_tau(double *tau, const double *t2, const double *t1, double c, int o
                 cudaStream_t st) {
   const PairBlocks P = pair_blocks(o, v, false);
   if (P.nunits == 0) return;
-  k_tau<<<pb_grid(P.nunits, 8), kPbThreads, 0, st>>>(tau, t2, t1, c, P);
+  launch_after(k_tau, pb_grid(P.nunits, 8), kPbThreads, 0, st, tau, t2, t1, c, P);
   count_launch();
 }
 
@@ -431,6 +435,7 @@ __global__ void __launch_bounds__(256)
     k_newt(double *__restrict__ t2n, const double *__restrict__ z2, double *__restrict__ t1n,
            const double *__restrict__ z1, const double *__restrict__ eo,
            const double *__restrict__ ev, int o, int v, int tiles, long long nunits) {
+  after_previous();
   __shared__ double tz[2][32][33];   // [ij tile: a rows][ji tile: b rows]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   // T1: z1 / (e_i - e_a)
@@ -500,7 +505,7 @@ void launch_newt(double *t2n, const double *z2, double *t1n, const double *z1, c
     }
   }
   const unsigned grid = (unsigned)std::max(1LL, std::min(nunits, 148LL * per_sm));
-  k_newt<<<grid, 256, 0, st>>>(t2n, z2, t1n, z1, eo, ev, o, v, tiles, nunits);
+  launch_after(k_newt, grid, 256, 0, st, t2n, z2, t1n, z1, eo, ev, o, v, tiles, nunits);
   count_launch();
 }
 
@@ -542,6 +547,7 @@ __global__ void __launch_bounds__(kPbThreads)
     k_energy(double *__restrict__ part, const double *__restrict__ t2,
              const double *__restrict__ t1, const double *__restrict__ V,
              const double *__restrict__ fov, PairBlocks P) {
+  after_previous();
   double s[3] = {0.0, 0.0, 0.0};
   const int n1 = P.o * P.v;
   for (int e = blockIdx.x * kPbThreads + threadIdx.x; e < n1; e += gridDim.x * kPbThreads)
@@ -593,6 +599,7 @@ __global__ void __launch_bounds__(kPbThreads)
 // load in flight before the first addition, fixed order
 constexpr int kPerLane = (kRedBlocks + 31) / 32;
 __global__ void k_final_sum(double *out, const double *part, int nv) {
+  after_previous();
   const int k = blockIdx.x;
   double v[kPerLane];
 #pragma unroll
@@ -610,14 +617,15 @@ __global__ void k_final_sum(double *out, const double *part, int nv) {
 void launch_energy(double *out3, const double *t2, const double *t1, const double *voovv,
                    const double *fov, int o, int v, double *scratch, cudaStream_t st) {
   const PairBlocks P = pair_blocks(o, v, true);
-  k_energy<<<kRedBlocks, kPbThreads, 0, st>>>(scratch, t2, t1, voovv, fov, P);
+  launch_after(k_energy, kRedBlocks, kPbThreads, 0, st, scratch, t2, t1, voovv, fov, P);
   count_launch();
-  k_final_sum<<<3, 32, 0, st>>>(out3, scratch, 3); count_launch();
+  launch_after(k_final_sum, 3, 32, 0, st, out3, scratch, 3); count_launch();
 }
 
 // xn = x + damp (xn - x), two loads and a store per element
 __global__ void k_blend(double *__restrict__ xn, const double *__restrict__ x, double damp,
                         long long n) {
+  after_previous();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     xn[i] = fma(damp, xn[i] - x[i], x[i]);
@@ -626,7 +634,7 @@ __global__ void k_blend(double *__restrict__ xn, const double *__restrict__ x, d
 void launch_blend(double *xn, const double *x, double damp, long long n, cudaStream_t st) {
   long long nb = (n + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
-  k_blend<<<(unsigned)nb, 256, 0, st>>>(xn, x, damp, n); count_launch();
+  launch_after(k_blend, (unsigned)nb, 256, 0, st, xn, x, damp, n); count_launch();
 }
 
 struct HistPtrs {
@@ -645,6 +653,7 @@ __device__ inline void amax_merge(double &bv, long long &bi, double v, long long
 // amax_merge orders candidates by (|value| descending, index ascending), a
 // total order, so the merge order does not change the result
 __global__ void k_absmax_final(double *out, const double *pv, const long long *pi) {
+  after_previous();
   double v[kPerLane];
   long long w[kPerLane];
 #pragma unroll
@@ -721,6 +730,7 @@ __global__ void __launch_bounds__(kPbThreads)
     k_diff_stats(double *__restrict__ e, const double *__restrict__ xnew,
                  const double *__restrict__ xold, HistPtrs h, int nh, int self, PairBlocks P,
                  double *__restrict__ part, double *__restrict__ pv, long long *__restrict__ pi) {
+  after_previous();
   __shared__ double sh[25][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0)
@@ -812,11 +822,12 @@ int launch_diff_stats(double *e, const double *xnew, const double *xold,
   double *pv = scratch + kRedBlocks * 25;   // [kRedBlocks]
   long long *pi = (long long *)(scratch + kRedBlocks * 26);
   const PairBlocks P = pair_blocks(o, v, true);
-  k_diff_stats<<<kRedBlocks, kPbThreads, 0, st>>>(e, xnew, xold, h, nh, self, P, part, pv, pi);
+  launch_after(k_diff_stats, kRedBlocks, kPbThreads, 0, st, e, xnew, xold, h, nh, self, P, part, pv,
+               pi);
   count_launch();
-  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi);
+  launch_after(k_absmax_final, 1, 32, 0, st, absmax_out, pv, pi);
   count_launch();
-  k_final_sum<<<nh, 32, 0, st>>>(dots_out, part, 25);
+  launch_after(k_final_sum, nh, 32, 0, st, dots_out, part, 25);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
@@ -828,6 +839,7 @@ int launch_diff_stats(double *e, const double *xnew, const double *xold,
 __global__ void __launch_bounds__(kPbThreads)
     k_lincomb_absmax(double *__restrict__ out, const double *__restrict__ c, HistPtrs hp, int n,
                      PairBlocks P, double *__restrict__ pv, long long *__restrict__ pi) {
+  after_previous();
   __shared__ double cs[25];
   if (threadIdx.x < n) cs[threadIdx.x] = c[threadIdx.x];
   __syncthreads();
@@ -889,15 +901,16 @@ void launch_lincomb_absmax(double *out, const double *c, const double *const *p,
   double *pv = scratch;
   long long *pi = (long long *)(scratch + kRedBlocks);
   const PairBlocks P = pair_blocks(o, v, true);
-  k_lincomb_absmax<<<kRedBlocks, kPbThreads, 0, st>>>(out, c, a, n, P, pv, pi);
+  launch_after(k_lincomb_absmax, kRedBlocks, kPbThreads, 0, st, out, c, a, n, P, pv, pi);
   count_launch();
-  k_absmax_final<<<1, 32, 0, st>>>(absmax_out, pv, pi);
+  launch_after(k_absmax_final, 1, 32, 0, st, absmax_out, pv, pi);
   count_launch();
 }
 
 // Bordered DIIS system [[0,-1..],[-1,B]] (lam,c) = (-1,0,..) by LU with
 // partial pivoting (the pivot order of LAPACK dgetf2, libr/dodiis.F:46).
 __global__ void k_diis_solve(double *coef, int *status, const double *B, int n) {
+  after_previous();
   if (threadIdx.x != 0) return;
   double A[26][26];
   double rhs[26];
@@ -941,11 +954,12 @@ __global__ void k_diis_solve(double *coef, int *status, const double *B, int n) 
 }
 
 void launch_diis_solve(double *coef_out, int *status_out, const double *B, int n, cudaStream_t st) {
-  k_diis_solve<<<1, 32, 0, st>>>(coef_out, status_out, B, n); count_launch();
+  launch_after(k_diis_solve, 1, 32, 0, st, coef_out, status_out, B, n); count_launch();
 }
 
 __global__ void k_lincomb(double *__restrict__ out, const double *__restrict__ base,
                           const double *__restrict__ c, HistPtrs p, int n, long long len) {
+  after_previous();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len;
        i += (long long)gridDim.x * blockDim.x) {
     double acc = base ? base[i] : 0.0;
@@ -960,13 +974,14 @@ void launch_lincomb(double *out, const double *base, const double *c, const doub
   for (int k = 0; k < 25; ++k) a.p[k] = k < n ? p[k] : nullptr;
   long long nb = (len + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
-  k_lincomb<<<(unsigned)nb, 256, 0, st>>>(out, base, c, a, n, len); count_launch();
+  launch_after(k_lincomb, (unsigned)nb, 256, 0, st, out, base, c, a, n, len); count_launch();
 }
 
 // ---------------------------------------------------------------------------
 // DPD list <-> dense
 // ---------------------------------------------------------------------------
 __global__ void k_gather(double *__restrict__ dense, DpdMap m, long long total) {
+  after_previous();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     long long r = idx;
@@ -990,6 +1005,7 @@ __global__ void k_gather(double *__restrict__ dense, DpdMap m, long long total) 
 }
 
 __global__ void k_scatter(const double *__restrict__ dense, DpdMap m, long long total) {
+  after_previous();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     long long r = idx;
@@ -1012,6 +1028,7 @@ __global__ void k_scatter(const double *__restrict__ dense, DpdMap m, long long 
 // integral producer, m = (r,p), n = (s,q)), read in its own order so the loads
 // coalesce; every pair type involved stores all of its pairs (FULL).
 __global__ void k_scatter_rpsq(const double *__restrict__ X, DpdMap m, long long total) {
+  after_previous();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     long long t = idx;
@@ -1033,7 +1050,7 @@ void launch_scatter_rpsq(const double *X, const DpdMap &m, cudaStream_t st) {
   long long nb = (total + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
   if (nb < 1) nb = 1;
-  k_scatter_rpsq<<<(unsigned)nb, 256, 0, st>>>(X, m, total); count_launch();
+  launch_after(k_scatter_rpsq, (unsigned)nb, 256, 0, st, X, m, total); count_launch();
 }
 
 void launch_gather(double *dense, const DpdMap &m, cudaStream_t st) {
@@ -1041,7 +1058,7 @@ void launch_gather(double *dense, const DpdMap &m, cudaStream_t st) {
   long long nb = (total + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
   if (nb < 1) nb = 1;
-  k_gather<<<(unsigned)nb, 256, 0, st>>>(dense, m, total); count_launch();
+  launch_after(k_gather, (unsigned)nb, 256, 0, st, dense, m, total); count_launch();
 }
 
 void launch_scatter(const double *dense, const DpdMap &m, cudaStream_t st) {
@@ -1049,7 +1066,7 @@ void launch_scatter(const double *dense, const DpdMap &m, cudaStream_t st) {
   long long nb = (total + 255) / 256;
   if (nb > 148 * 32) nb = 148 * 32;
   if (nb < 1) nb = 1;
-  k_scatter<<<(unsigned)nb, 256, 0, st>>>(dense, m, total); count_launch();
+  launch_after(k_scatter, (unsigned)nb, 256, 0, st, dense, m, total); count_launch();
 }
 
 // ---------------------------------------------------------------------------
@@ -1069,6 +1086,7 @@ __global__ void __launch_bounds__(256)
     k_ladder_pack_v(double *__restrict__ Up, double *__restrict__ Um,
                     const double *__restrict__ V, const int *__restrict__ pairs, int v,
                     int ntile, LadderPlanes pl) {
+  after_previous();
   __shared__ double t1[32][33];  // [c][d]
   __shared__ double t2[32][33];  // [c][d] = V[ab][d][c]
   const int np = v * (v + 1) / 2, nm = v * (v - 1) / 2;
@@ -1132,9 +1150,10 @@ void launch_ladder_pack_v(double *Up, double *Um, const double *V, const int *pa
   const long long blocks = (long long)(v * (v + 1) / 2) * (ntile * (ntile + 1) / 2);
   const unsigned grid = (unsigned)std::min<long long>(blocks, 148 * 64);
   if (planes)
-    k_ladder_pack_v<true><<<grid, 256, 0, st>>>(Up, Um, V, pairs, v, ntile, *planes);
+    launch_after(k_ladder_pack_v<true>, grid, 256, 0, st, Up, Um, V, pairs, v, ntile, *planes);
   else
-    k_ladder_pack_v<false><<<grid, 256, 0, st>>>(Up, Um, V, pairs, v, ntile, LadderPlanes());
+    launch_after(k_ladder_pack_v<false>, grid, 256, 0, st, Up, Um, V, pairs, v, ntile,
+                 LadderPlanes());
   count_launch();
 }
 
@@ -1152,6 +1171,7 @@ template <bool S>
 __global__ void __launch_bounds__(256)
     k_ladder_pack_tau(double *__restrict__ tp, double *__restrict__ tm,
                       const double *__restrict__ tau, int v, int noo, LadderPlanes pl) {
+  after_previous();
   __shared__ double X[32][33];  // [c local][d local] of tau[ij][c][d]
   const int np = v * (v + 1) / 2, nm = v * (v - 1) / 2;
   const size_t vv = (size_t)v * v;
@@ -1207,9 +1227,9 @@ void launch_ladder_pack_tau(double *tp, double *tm, const double *tau, int v, in
   const int tiles = (v + 31) / 32;
   dim3 grid((unsigned)(tiles * (tiles + 1) / 2), (unsigned)std::min(noo, 65535));
   if (planes)
-    k_ladder_pack_tau<true><<<grid, 256, 0, st>>>(tp, tm, tau, v, noo, *planes);
+    launch_after(k_ladder_pack_tau<true>, grid, 256, 0, st, tp, tm, tau, v, noo, *planes);
   else
-    k_ladder_pack_tau<false><<<grid, 256, 0, st>>>(tp, tm, tau, v, noo, LadderPlanes());
+    launch_after(k_ladder_pack_tau<false>, grid, 256, 0, st, tp, tm, tau, v, noo, LadderPlanes());
   count_launch();
 }
 
@@ -1221,6 +1241,7 @@ void launch_ladder_pack_tau(double *tp, double *tm, const double *tau, int v, in
 __global__ void __launch_bounds__(256)
     k_ladder_unpack(double *__restrict__ Z2, const double *__restrict__ S,
                     const double *__restrict__ A, int v, int noo) {
+  after_previous();
   __shared__ double P[32][33];  // S + A at [b local][a local]
   const int np = v * (v + 1) / 2, nm = v * (v - 1) / 2;
   const size_t vv = (size_t)v * v;
@@ -1263,7 +1284,7 @@ void launch_ladder_unpack(double *Z2, const double *S, const double *A, int v, i
                           cudaStream_t st) {
   const int tiles = (v + 31) / 32;
   dim3 grid((unsigned)(tiles * (tiles + 1) / 2), (unsigned)std::min(noo, 65535));
-  k_ladder_unpack<<<grid, 256, 0, st>>>(Z2, S, A, v, noo);
+  launch_after(k_ladder_unpack, grid, 256, 0, st, Z2, S, A, v, noo);
   count_launch();
 }
 
@@ -1277,6 +1298,7 @@ __device__ __forceinline__ int find_block(const long long *pref, int nb, long lo
 
 __global__ void k_ladder_pack_v_blk(double *__restrict__ Up, double *__restrict__ Um,
                                     const double *__restrict__ V, LadderBlocks L) {
+  after_previous();
   const size_t v = L.v, vv = v * v;
   const long long nup = L.offUp[L.nirrep], total = nup + L.offUm[L.nirrep];
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -1307,12 +1329,13 @@ void launch_ladder_pack_v_blk(double *Up, double *Um, const double *V, const Lad
   const long long total = L.offUp[L.nirrep] + L.offUm[L.nirrep];
   if (total == 0) return;
   const long long nb = std::min<long long>((total + 255) / 256, 148 * 32);
-  k_ladder_pack_v_blk<<<(unsigned)nb, 256, 0, st>>>(Up, Um, V, L);
+  launch_after(k_ladder_pack_v_blk, (unsigned)nb, 256, 0, st, Up, Um, V, L);
   count_launch();
 }
 
 __global__ void k_ladder_pack_tau_blk(double *__restrict__ tp, double *__restrict__ tm,
                                       const double *__restrict__ tau, LadderBlocks L) {
+  after_previous();
   const size_t v = L.v, vv = v * v;
   const long long ntp = L.offTp[L.nirrep], total = ntp + L.offTm[L.nirrep];
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -1339,7 +1362,7 @@ void launch_ladder_pack_tau_blk(double *tp, double *tm, const double *tau, const
   const long long total = L.offTp[L.nirrep] + L.offTm[L.nirrep];
   if (total == 0) return;
   const long long nb = std::min<long long>((total + 255) / 256, 148 * 32);
-  k_ladder_pack_tau_blk<<<(unsigned)nb, 256, 0, st>>>(tp, tm, tau, L);
+  launch_after(k_ladder_pack_tau_blk, (unsigned)nb, 256, 0, st, tp, tm, tau, L);
   count_launch();
 }
 
@@ -1348,6 +1371,7 @@ void launch_ladder_pack_tau_blk(double *tp, double *tm, const double *tau, const
 // ij's local index within the occupied pairs of irrep g ^ hs
 __global__ void k_ladder_unpack_blk(double *__restrict__ Z2, const double *__restrict__ S,
                                     const double *__restrict__ A, LadderBlocks L) {
+  after_previous();
   const long long v = L.v, vv = v * v, total = (long long)L.o * L.o * vv;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -1377,7 +1401,7 @@ void launch_ladder_unpack_blk(double *Z2, const double *S, const double *A,
                               const LadderBlocks &L, cudaStream_t st) {
   const long long total = (long long)L.o * L.o * L.v * L.v;
   const long long nb = std::min<long long>((total + 255) / 256, 148 * 32);
-  k_ladder_unpack_blk<<<(unsigned)std::max(1LL, nb), 256, 0, st>>>(Z2, S, A, L);
+  launch_after(k_ladder_unpack_blk, (unsigned)std::max(1LL, nb), 256, 0, st, Z2, S, A, L);
   count_launch();
 }
 

@@ -34,6 +34,7 @@ constexpr int kDensWarps = 8, kDensCols = 16;   // up to 512 columns per sweep
 __global__ void __launch_bounds__(32 * kDensWarps)
     k_density_sums(double *__restrict__ rs, double *__restrict__ cs,
                    const double *__restrict__ l2, const double *__restrict__ t2, int v) {
+  after_previous();
   __shared__ double sh[kDensWarps][32 * kDensCols];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long base = (long long)blockIdx.x * v * v;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(32 * kDensWarps)
 __global__ void __launch_bounds__(256)
     k_density_diag(double *__restrict__ diag, const double *__restrict__ rs,
                    const double *__restrict__ cs, int o, int v) {
+  after_previous();
   __shared__ double sh[8];
   double t = 0.0;
   if ((int)blockIdx.x < v) {
@@ -155,9 +157,9 @@ int CCEngine::density(std::vector<double> &D) {
   const size_t nsum = (size_t)o * o * v;
   ACES_TRY(alloc(sums, 2 * nsum + o + v));
   double *rs = sums.p, *cs = rs + nsum, *dg = cs + nsum;
-  k_density_sums<<<o * o, 32 * kDensWarps, 0, st>>>(rs, cs, L.p + ov, X.p + ov, v);
+  launch_after(k_density_sums, o * o, 32 * kDensWarps, 0, st, rs, cs, L.p + ov, X.p + ov, v);
   count_launch();
-  k_density_diag<<<o + v, 256, 0, st>>>(dg, rs, cs, o, v);
+  launch_after(k_density_diag, o + v, 256, 0, st, dg, rs, cs, o, v);
   count_launch();
   ACES_CUDA(cudaGetLastError());
   std::vector<double> aoo((size_t)o * o), avv((size_t)v * v), aov((size_t)ov), avo((size_t)ov),

@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(128)
                            const double *__restrict__ Ioovv, const double *__restrict__ eo,
                            const double *__restrict__ ev, int o, int v,
                            double *__restrict__ part) {
+  after_previous();
   __shared__ TW cube[6][kTile][kTile + 1][kTile + 1];
   __shared__ double It[3][6][kTile][kTile + 1];
   __shared__ double ts[3][3][kTile];   // [t_i, t_j, t_k][tile position][local]
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(128)
 // sum of n (E4, E5) partial pairs: 1024 threads stride the list, then a
 // fixed-shape tree; the order of additions does not depend on timing
 __global__ void __launch_bounds__(1024) k_sum_pairs(double *out, const double *part, long long n) {
+  after_previous();
   double a = 0.0, b = 0.0;
   for (long long t = threadIdx.x; t < n; t += blockDim.x) {
     a += part[2 * t];
@@ -418,9 +420,9 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
       cv.p = Wb.p;
       ACES_TRY(gemm_nt_bf16x3_batched(Aa, Ba, 4, v * v, v, &byclass[(size_t)2 * ntrip + t0b],
                                       d_ent + 2 * ntrip + t0b, n, 1.0, 1.0, cv, true, st));
-      k_triples_energy_tiled<float><<<dim3(nblk, n), 128, 0, st>>>(
-          reinterpret_cast<const float *>(Wb.p), V3, d_trip + 3 * t0b, t1(), I_oovv.p, eo.p,
-          ev.p, o, v, part.p + (size_t)t0b * nblk * 2);
+      launch_after(k_triples_energy_tiled<float>, dim3(nblk, n), 128, 0, st,
+                   reinterpret_cast<const float *>(Wb.p), V3, d_trip + 3 * t0b, t1(), I_oovv.p,
+                   eo.p, ev.p, o, v, part.p + (size_t)t0b * nblk * 2);
       count_launch();
       ACES_CUDA(cudaGetLastError());
     }
@@ -490,15 +492,15 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
                                 cudaMemcpyHostToDevice, st));
       for (int q = 0; q < 3; ++q)
         ACES_TRY(f64_tasks_run(d_tasks + (size_t)q * n, n, plan[q], 1.0, q ? 1.0 : 0.0, st));
-      k_triples_energy_tiled<double><<<dim3(nblk, n), 128, 0, st>>>(
-          Wb.p, V3, d_trip + 3 * (size_t)t0b, t1(), I_oovv.p, eo.p, ev.p, o, v,
-          part.p + (size_t)t0b * nblk * 2);
+      launch_after(k_triples_energy_tiled<double>, dim3(nblk, n), 128, 0, st, Wb.p, V3,
+                   d_trip + 3 * (size_t)t0b, t1(), I_oovv.p, eo.p, ev.p, o, v,
+                   part.p + (size_t)t0b * nblk * 2);
       count_launch();
       ACES_CUDA(cudaGetLastError());
     }
     nparts = (long long)ntrip * nblk;
   }
-  k_sum_pairs<<<1, 1024, 0, st>>>(outp.p, part.p, nparts);
+  launch_after(k_sum_pairs, 1, 1024, 0, st, outp.p, part.p, nparts);
   count_launch();
   double h[2];
   ACES_CUDA(cudaMemcpyAsync(h, outp.p, 16, cudaMemcpyDeviceToHost, st));
