@@ -17,14 +17,16 @@ namespace {
 // a launch is a single task passed by value, or a device table of tasks.  The
 // k tiles (16 doubles, one 128-byte row per operand row) of all segments form
 // one sequence through a 4-stage cp.async pipeline.  Rows lie unpadded in
-// shared memory with the 16-byte chunk index XORed by 4 on odd rows: the
-// 8 lanes of a 128-bit load phase (two neighbouring rows x four chunks) then
-// cover all 32 banks, and so do the copies (one row per 8 lanes).
+// shared memory with the 16-byte chunk index XORed by twice the row's index
+// modulo 4: the 16 lanes of a 64-bit load phase (four neighbouring rows x four
+// k) then cover all 32 banks, and so do the copies (one row per 8 lanes).
 //
-// A thread's fragment of a k step of 8 is one double2 per row: its two k
-// values are 2t and 2t+1 (t the lane's position in its group of four) in A
-// and in B alike.  The product sums over k, so this order is as good as the
-// instruction's own (t, t+4) and takes half the shared-memory loads.
+// Every output sums its k in ascending order.  One 128-bit load per row and k
+// step, with the k taken as 0, 2, 4, 6, 1, 3, 5, 7, is 1-2 % faster (2401 x
+// 1519 x 2050: 601 us against 612), but its other last bits move values across
+// the rounding boundaries of the BF16 split: a CCSD with o = 24, v = 220 in
+// split precision then differed by up to 1e-9 with the order of its lists'
+// sums, and by 1e-17 with them in order.
 // ---------------------------------------------------------------------------
 constexpr int BK = 16, kStages = 4;
 
@@ -47,7 +49,7 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// c (16 x 8) += a (16 x 8) b (8 x 8)^T: a = rows g and g+8 x k (2t, 2t+1)
+// c (16 x 8) += a (16 x 8) b (8 x 8)^T: a = rows g and g+8 x k (t, t+4)
 __device__ __forceinline__ void dmma(double (&c)[4], const double2 &a0, const double2 &a1,
                                      const double2 &b) {
   asm volatile(
@@ -76,7 +78,7 @@ struct CopyPlan {
   static constexpr int CPR = BK / VEC;
   static constexpr int RS = kThreads / CPR;
   static constexpr int kPer = (ROWS + RS - 1) / RS;
-  static_assert(RS % 2 == 0, "a thread's rows share their parity (one swizzle)");
+  static_assert(RS % 4 == 0, "a thread's rows share their swizzle");
   const double *base;   // &X[row0 + r0][kc] of the current segment
   const double *safe;   // any valid address (the source of zero-size copies)
   long long step;       // RS rows
@@ -85,7 +87,7 @@ struct CopyPlan {
   __device__ __forceinline__ void init(int rows, int row0) {
     const int t = threadIdx.x, r0 = t / CPR;
     kc = (t % CPR) * VEC;
-    const int ch = (kc >> 1) ^ ((r0 & 1) << 2);
+    const int ch = (kc >> 1) ^ ((r0 & 3) << 1);
     soff = (r0 * BK + ch * 2 + (kc & 1)) * 8;
     live = 0;
 #pragma unroll
@@ -220,7 +222,8 @@ __global__ void __launch_bounds__(T::kThreads, T::OCC)
 
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) issue_next();
-  const int sw = (g & 1) << 2;
+  // offsets of a row's k = q and k = q + 4 within a k step of 8
+  const int sw = (g & 3) << 1;
   int slot = 0;
   for (int kt = 0; kt < nk; ++kt) {
     cp_wait<kStages - 2>();   // k tile kt has landed
@@ -232,16 +235,19 @@ __global__ void __launch_bounds__(T::kThreads, T::OCC)
     const double *b_s = reinterpret_cast<const double *>(st) + (BM + wn * T::TN + g) * BK;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const int ch = ((s * 4 + q) ^ sw) * 2;
+      const int k0 = ((s * 4 + (q >> 1)) ^ sw) * 2 + (q & 1);
+      const int k4 = ((s * 4 + 2 + (q >> 1)) ^ sw) * 2 + (q & 1);
       double2 af[MI][2], bf[NI];
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          af[i][h] = *reinterpret_cast<const double2 *>(a_s + (i * 16 + h * 8) * BK + ch);
+        for (int h = 0; h < 2; ++h) {
+          const double *r = a_s + (i * 16 + h * 8) * BK;
+          af[i][h] = make_double2(r[k0], r[k4]);
+        }
 #pragma unroll
       for (int j = 0; j < NI; ++j)
-        bf[j] = *reinterpret_cast<const double2 *>(b_s + j * 8 * BK + ch);
+        bf[j] = make_double2(b_s[j * 8 * BK + k0], b_s[j * 8 * BK + k4]);
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -441,10 +447,12 @@ __global__ void k_gemv_final(int M, int W, double alpha, const double *__restric
 }
 
 // Tiny products (at most kTinyOut outputs): one warp per output, its lanes
-// striding K (coalesced row reads), eight independent partial sums per lane
-// with all sixteen loads of a 256-wide step in flight, the ragged last step
-// included (latency bound: 50 x 50 x 1800 took 7.6 us with four and a serial
-// remainder), reduced by shuffles in a fixed order.
+// striding K (coalesced row reads) with the sixteen loads of a 256-wide step in
+// flight, the ragged last step included (latency bound: with eight and a serial
+// remainder 50 x 50 x 1800 took 7.6 us; the 280 launches of an EOM with o = 6,
+// v = 50 now take 3.8 us each).  Four partial sums per lane take the k of each
+// full 128 in turn, the first one what is left over; shuffles add them in a
+// fixed order.
 constexpr long long kTinyOut = 8192;
 __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double *__restrict__ A,
                                 long long lda, const double *__restrict__ B, long long ldb,
@@ -455,9 +463,7 @@ __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double 
   if (w >= M * N) return;  // warp-uniform
   const int m = w % M, n = w / M;
   const double *a = A + (long long)m * lda, *b = B + (long long)n * ldb;
-  double s[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) s[u] = 0.0;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   for (int k0 = lane; k0 < K; k0 += 256) {
     double x[8], y[8];
 #pragma unroll
@@ -467,9 +473,20 @@ __global__ void k_gemm_tiny_f64(int M, int N, int K, double alpha, const double 
       y[u] = k < K ? __ldg(b + k) : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) s[u] = fma(x[u], y[u], s[u]);
+    for (int u = 0; u < 8; u += 4) {
+      const bool full = k0 + 32 * u + 96 < K;
+      s0 = fma(x[u], y[u], s0);
+      if (full) {
+        s1 = fma(x[u + 1], y[u + 1], s1);
+        s2 = fma(x[u + 2], y[u + 2], s2);
+        s3 = fma(x[u + 3], y[u + 3], s3);
+      } else {
+        s0 = fma(x[u + 1], y[u + 1], s0);
+        s0 = fma(x[u + 2], y[u + 2], s0);
+      }
+    }
   }
-  double t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+  double t = (s0 + s1) + (s2 + s3);
   for (int off = 16; off; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
   if (lane == 0) {
     double *cp = C.p + cview_off(C, m, n);
