@@ -157,6 +157,8 @@ class CCEngine {
   // same tape), dropped with their cached splits when a pass is recorded
   std::map<std::tuple<const double *, int, int, long long>, DBuf> tape_tcache;
   const double *tape_transposed(const double *src, int rows, int cols, long long ld);
+  int adjoint_product(int M, int N, int K, double alpha, const double *src, long long ld,
+                      const double *B, long long ldb, const CView &C, DBuf &scratch);
   void tape_cache_clear();
   std::vector<const double *> symmetric;     // constant matrices equal to their transpose
   DBuf bwdA, bwdB, bwdC, bwdD;
@@ -168,6 +170,7 @@ class CCEngine {
   int tmp(DBuf &b, size_t n);
   const double *transposed(const double *src, int rows, int cols, long long ld, bool cst,
                            DBuf &scratch);
+  std::vector<char> first_writers();
   int backward();
   // backward() through a CUDA graph captured on its second pass over a tape
   int backward_run();
