@@ -684,6 +684,7 @@ int CCEngine::load_from_lists() {
   {
     DevMap dm;
     ACES_TRY(make_map(dm, 233, 13, 13, irr_o, irr_v, false));
+    if (s.nirrep > 1) return ladder_blocks_setup(dm.m);  // no dense copy
     ACES_TRY(alloc(I_vvvv, V * V * V * V, false));
     launch_gather(I_vvvv.p, dm.m, st);
     ACES_CUDA(cudaStreamSynchronize(st));
@@ -1035,6 +1036,78 @@ int CCEngine::residual() {
   return ACES_OK;
 }
 
+// U+ and U- of the irrep blocks, straight from list 233's blocks
+int CCEngine::ladder_blocks_setup(const DpdMap &vvvv) {
+  const int nir = state().sym.nirrep;
+  LadderBlocks &Lb = ladb;
+  // pair lists by pair irrep: symmetric c <= d and antisymmetric c < d (d
+  // slowest), occupied pairs ij by irrep; local indices of every pair
+  std::vector<int> pp, mm, pidx((size_t)v * v, -1), midx((size_t)v * v, -1), ijs, ijl(o * o);
+  Lb.nirrep = nir;
+  Lb.o = o;
+  Lb.v = v;
+  Lb.offP[0] = Lb.offM[0] = Lb.offIJ[0] = 0;
+  for (int g = 0; g < nir; ++g) {
+    int np_g = 0, nm_g = 0, nij = 0;
+    for (int d = 0; d < v; ++d)
+      for (int c = 0; c <= d; ++c) {
+        if ((irr_v[c] ^ irr_v[d]) != g) continue;
+        pp.push_back(c);
+        pp.push_back(d);
+        pidx[(size_t)c * v + d] = np_g++;
+        if (c < d) {
+          mm.push_back(c);
+          mm.push_back(d);
+          midx[(size_t)c * v + d] = nm_g++;
+        }
+      }
+    for (int ij = 0; ij < o * o; ++ij)
+      if ((irr_o[ij / o] ^ irr_o[ij % o]) == g) {
+        ijs.push_back(ij);
+        ijl[ij] = nij++;
+      }
+    Lb.nP[g] = np_g;
+    Lb.nM[g] = nm_g;
+    Lb.nIJ[g] = nij;
+    Lb.offP[g + 1] = Lb.offP[g] + np_g;
+    Lb.offM[g + 1] = Lb.offM[g] + nm_g;
+    Lb.offIJ[g + 1] = Lb.offIJ[g] + nij;
+  }
+  for (int g = nir; g < 8; ++g) Lb.nP[g] = Lb.nM[g] = Lb.nIJ[g] = 0;
+  Lb.offUp[0] = Lb.offUm[0] = 0;
+  for (int g = 0; g < nir; ++g) {
+    Lb.offUp[g + 1] = Lb.offUp[g] + (long long)Lb.nP[g] * Lb.nP[g];
+    Lb.offUm[g + 1] = Lb.offUm[g] + (long long)Lb.nM[g] * Lb.nM[g];
+  }
+  std::vector<int> tab;
+  auto put = [&](const std::vector<int> &x) {
+    const size_t at = tab.size();
+    tab.insert(tab.end(), x.begin(), x.end());
+    return at;
+  };
+  std::vector<int> io(irr_o.begin(), irr_o.end()), iv(irr_v.begin(), irr_v.end());
+  const size_t a_pp = put(pp), a_mm = put(mm), a_pi = put(pidx), a_mi = put(midx),
+               a_ijs = put(ijs), a_ijl = put(ijl), a_io = put(io), a_iv = put(iv);
+  ACES_TRY(alloc(ladpairs, (tab.size() + 1) / 2 + 1));
+  ACES_CUDA(cudaMemcpyAsync(ladpairs.p, tab.data(), tab.size() * sizeof(int),
+                            cudaMemcpyHostToDevice, st));
+  const int *base = reinterpret_cast<const int *>(ladpairs.p);
+  Lb.pp = base + a_pp;
+  Lb.mm = base + a_mm;
+  Lb.pidx = base + a_pi;
+  Lb.midx = base + a_mi;
+  Lb.ijs = base + a_ijs;
+  Lb.ijl = base + a_ijl;
+  Lb.irr_o = base + a_io;
+  Lb.irr_v = base + a_iv;
+  ACES_TRY(alloc(Up, (size_t)std::max(1LL, Lb.offUp[nir]), false));
+  ACES_TRY(alloc(Um, (size_t)std::max(1LL, Lb.offUm[nir]), false));
+  launch_ladder_pack_list(Up.p, Um.p, vvvv, Lb, st);
+  ACES_CUDA(cudaGetLastError());
+  ACES_CUDA(cudaStreamSynchronize(st));
+  return ACES_OK;
+}
+
 // Particle-particle ladder Z2[ij,ab] += sum_cd <ab|cd> tau[ij,cd] on symmetric
 // and antisymmetric pair combinations (the reference's RHF a<=b packing,
 // vcc/ladab1.F:55-64 with SYMEXP4).  With <ba|dc> = <ab|cd>:
@@ -1043,78 +1116,13 @@ int CCEngine::residual() {
 //   tau+ = tau[cd] + tau[dc] (c<d), tau[cc];  tau- = tau[cd] - tau[dc]
 //   Z2[ab] += S + A,  Z2[ba] += S - A,  Z2[aa] += S
 // Two contractions of (v(v+1)/2)^2 and (v(v-1)/2)^2 x o^2 instead of v^4 x o^2:
-// half the flops.  U+/U- are built once from the dense <ab|cd> (or the list).
+// half the flops.  U+/U- are built once from the dense <ab|cd>, or with
+// symmetry by pair irrep from the list's blocks.
 // The map is linear in tau and needs no symmetry of it, so the Lambda
 // backward pass calls it with (Z2 adjoint, tau adjoint) for in and out.
 int CCEngine::ladder_packed_blocks(const double *in, double *out) {
   const int nir = state().sym.nirrep;
   LadderBlocks &Lb = ladb;
-  if (!Up.p) {
-    // pair lists by pair irrep: symmetric c <= d and antisymmetric c < d (d
-    // slowest), occupied pairs ij by irrep; local indices of every pair
-    std::vector<int> pp, mm, pidx((size_t)v * v, -1), midx((size_t)v * v, -1), ijs, ijl(o * o);
-    Lb.nirrep = nir;
-    Lb.o = o;
-    Lb.v = v;
-    Lb.offP[0] = Lb.offM[0] = Lb.offIJ[0] = 0;
-    for (int g = 0; g < nir; ++g) {
-      int np_g = 0, nm_g = 0, nij = 0;
-      for (int d = 0; d < v; ++d)
-        for (int c = 0; c <= d; ++c) {
-          if ((irr_v[c] ^ irr_v[d]) != g) continue;
-          pp.push_back(c);
-          pp.push_back(d);
-          pidx[(size_t)c * v + d] = np_g++;
-          if (c < d) {
-            mm.push_back(c);
-            mm.push_back(d);
-            midx[(size_t)c * v + d] = nm_g++;
-          }
-        }
-      for (int ij = 0; ij < o * o; ++ij)
-        if ((irr_o[ij / o] ^ irr_o[ij % o]) == g) {
-          ijs.push_back(ij);
-          ijl[ij] = nij++;
-        }
-      Lb.nP[g] = np_g;
-      Lb.nM[g] = nm_g;
-      Lb.nIJ[g] = nij;
-      Lb.offP[g + 1] = Lb.offP[g] + np_g;
-      Lb.offM[g + 1] = Lb.offM[g] + nm_g;
-      Lb.offIJ[g + 1] = Lb.offIJ[g] + nij;
-    }
-    for (int g = nir; g < 8; ++g) Lb.nP[g] = Lb.nM[g] = Lb.nIJ[g] = 0;
-    Lb.offUp[0] = Lb.offUm[0] = 0;
-    for (int g = 0; g < nir; ++g) {
-      Lb.offUp[g + 1] = Lb.offUp[g] + (long long)Lb.nP[g] * Lb.nP[g];
-      Lb.offUm[g + 1] = Lb.offUm[g] + (long long)Lb.nM[g] * Lb.nM[g];
-    }
-    std::vector<int> tab;
-    auto put = [&](const std::vector<int> &x) {
-      const size_t at = tab.size();
-      tab.insert(tab.end(), x.begin(), x.end());
-      return at;
-    };
-    std::vector<int> io(irr_o.begin(), irr_o.end()), iv(irr_v.begin(), irr_v.end());
-    const size_t a_pp = put(pp), a_mm = put(mm), a_pi = put(pidx), a_mi = put(midx),
-                 a_ijs = put(ijs), a_ijl = put(ijl), a_io = put(io), a_iv = put(iv);
-    ACES_TRY(alloc(ladpairs, (tab.size() + 1) / 2 + 1));
-    ACES_CUDA(cudaMemcpyAsync(ladpairs.p, tab.data(), tab.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, st));
-    const int *base = reinterpret_cast<const int *>(ladpairs.p);
-    Lb.pp = base + a_pp;
-    Lb.mm = base + a_mm;
-    Lb.pidx = base + a_pi;
-    Lb.midx = base + a_mi;
-    Lb.ijs = base + a_ijs;
-    Lb.ijl = base + a_ijl;
-    Lb.irr_o = base + a_io;
-    Lb.irr_v = base + a_iv;
-    ACES_TRY(alloc(Up, (size_t)std::max(1LL, Lb.offUp[nir])));
-    ACES_TRY(alloc(Um, (size_t)std::max(1LL, Lb.offUm[nir])));
-    launch_ladder_pack_v_blk(Up.p, Um.p, I_vvvv.p, Lb, st);
-    ACES_CUDA(cudaStreamSynchronize(st));
-  }
   // per-call blocks of the vector's symmetry
   Lb.hs = ladder_sym;
   Lb.offTp[0] = Lb.offTm[0] = 0;

@@ -70,6 +70,7 @@ class CCEngine {
   // the same on irrep blocks (more than one irrep): pair irrep g of (a,b) and
   // (c,d) with occupied pairs of irrep g ^ ladder_sym (0 for the amplitudes
   // and Lambda, the state's irrep for EOM products)
+  int ladder_blocks_setup(const DpdMap &vvvv);
   int ladder_packed_blocks(const double *in, double *out);
   int ladder_sym = 0;
   LadderBlocks ladb{};  // block tables (device pointers into ladpairs)

@@ -122,8 +122,8 @@ struct LadderBlocks {
   long long offUp[9], offUm[9], offTp[9], offTm[9];
   const int *pp, *mm, *pidx, *midx, *ijs, *ijl, *irr_o, *irr_v;
 };
-void launch_ladder_pack_v_blk(double *Up, double *Um, const double *V, const LadderBlocks &L,
-                              cudaStream_t st);
+void launch_ladder_pack_list(double *Up, double *Um, const DpdMap &vvvv, const LadderBlocks &L,
+                             cudaStream_t st);
 void launch_ladder_pack_tau_blk(double *tp, double *tm, const double *tau, const LadderBlocks &L,
                                 cudaStream_t st);
 void launch_ladder_unpack_blk(double *Z2, const double *S, const double *A,
