@@ -202,7 +202,7 @@ const double *CCEngine::transposed(const double *src, int rows, int cols, long l
   DBuf *dst = &scratch;
   DBuf fresh;
   if (cst) dst = &fresh;
-  if (alloc(*dst, (size_t)rows * cols) != ACES_OK) return nullptr;
+  if (alloc(*dst, (size_t)rows * cols, false) != ACES_OK) return nullptr;
   PermSpec s;
   s.n[0] = 1; s.n[1] = 1; s.n[2] = cols; s.n[3] = rows;
   s.nterms = 1;
@@ -223,7 +223,7 @@ const double *CCEngine::tape_transposed(const double *src, int rows, int cols, l
   auto it = tape_tcache.find(key);
   if (it != tape_tcache.end()) return it->second.p;
   DBuf fresh;
-  if (alloc(fresh, (size_t)rows * cols) != ACES_OK) return nullptr;
+  if (alloc(fresh, (size_t)rows * cols, false) != ACES_OK) return nullptr;
   PermSpec s;
   s.n[0] = 1; s.n[1] = 1; s.n[2] = cols; s.n[3] = rows;
   s.nterms = 1;

@@ -110,7 +110,7 @@ int CCEngine::copy(double *dst, const double *src, size_t n) {
     tape.push_back(op);
   }
   memo_written(dst, (long long)n);
-  if (n) ACES_CUDA(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToDevice, st));
+  launch_copy(dst, src, (long long)n, st);
   return ACES_OK;
 }
 

@@ -187,7 +187,7 @@ int CCEngine::eom_sigma(const double *x, double *out, int h, const int *d_irr_o,
   const double *g = adj(X.p);
   // pair symmetriser on the doubles: out2 = (g2 + g2^T) / 2, g2^T[i,j,a,b] = g2[j,i,b,a]
   const long long s2[4] = {O * V * V, V * V, V, 1};
-  ACES_CUDA(cudaMemcpyAsync(out, g, ov * 8, cudaMemcpyDeviceToDevice, st));
+  launch_copy(out, g, ov, st);
   PermSpec ps;
   ps.n[0] = o; ps.n[1] = o; ps.n[2] = v; ps.n[3] = v;
   ps.nterms = 2;
@@ -378,7 +378,7 @@ extern "C" int xvee_run(aces_eom_config *cfg) {
         ACES_CUDA(cudaMemcpyAsync(cdev.p, Y[r].data(), m * 8, cudaMemcpyHostToDevice, E.st));
         combine(xr.p, nullptr, Vm, m, cdev.p);
         combine(sr.p, nullptr, Sm, m, cdev.p);
-        ACES_CUDA(cudaMemcpyAsync(rv.p, sr.p, len * 8, cudaMemcpyDeviceToDevice, E.st));
+        launch_copy(rv.p, sr.p, len, E.st);
         launch_axpy(rv.p, xr.p, -wsel[r], len, E.st);
         ACES_TRY(dots(rv.p, 1, rv.p, 1.0, cdev.p));
         rn[r] = std::sqrt(std::max(0.0, host_scalar(cdev.p)));
@@ -397,8 +397,7 @@ extern "C" int xvee_run(aces_eom_config *cfg) {
             ACES_TRY(dots(dv.p, 1, dv.p, 1.0, cdev.p));
             const double nd = std::sqrt(std::max(0.0, host_scalar(cdev.p)));
             if (nd > 1e-10) {
-              ACES_CUDA(cudaMemcpyAsync(row(Vm, m), dv.p, len * 8, cudaMemcpyDeviceToDevice,
-                                        E.st));
+              launch_copy(row(Vm, m), dv.p, len, E.st);
               launch_scale(row(Vm, m), 1.0 / nd, len, E.st);
               ACES_TRY(E.eom_sigma(row(Vm, m), row(Sm, m), h, d_irr_o, d_irr_v));
               ++total_sigma;

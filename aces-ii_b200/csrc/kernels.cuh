@@ -44,6 +44,8 @@ void launch_newt(double *t2n, const double *z2, double *t1n, const double *z1, c
 void launch_energy(double *out2, const double *t2, const double *t1, const double *voovv,
                    const double *fov, int o, int v, double *scratch, cudaStream_t st);
 
+// dst[0..n) = src[0..n) (not overlapping)
+void launch_copy(double *dst, const double *src, long long n, cudaStream_t st);
 // DAMP_CC_RESIDUAL (vcc/damp_cc_residual.F): xn = x + damp (xn - x)
 void launch_blend(double *xn, const double *x, double damp, long long n, cudaStream_t st);
 // e = xnew - xold (T1 + T2 of a pair-symmetric vector) with, in the same pass,

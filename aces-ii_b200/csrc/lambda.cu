@@ -133,7 +133,7 @@ int CCEngine::lambda_rhs() {
   ACES_TRY(backward_run());
   double *xb = adj(X.p);
   ACES_TRY(alloc(lrhs, len));
-  ACES_CUDA(cudaMemcpyAsync(lrhs.p, gE.p, len * 8, cudaMemcpyDeviceToDevice, st));
+  launch_copy(lrhs.p, gE.p, len, st);
   launch_axpy(lrhs.p, xb, 1.0, len, st);
   ACES_CUDA(cudaGetLastError());
   return ACES_OK;
