@@ -319,6 +319,10 @@ std::vector<char> CCEngine::first_writers() {
   return first;
 }
 
+// The launches go out one by one: overlapped with one another they keep up with
+// the device, and a graph of a pass costs more than it saves (capture and
+// instantiation once per tape, 100-200 us before each replay starts: EOM o = 6,
+// v = 50 12.1 ms with one and 11.9 without, Lambda o = 10, v = 90 19.8 and 19.2).
 int CCEngine::backward() {
   // walk the tape in reverse; adjoint buffers already hold the seeds
   const bool rec = recording;
@@ -448,54 +452,6 @@ void CCEngine::zero_adjoints() {
     if (++n == kZeroBufs) flush();
   }
   flush();
-}
-
-void CCEngine::drop_backward_graph() {
-  if (backward_exec) cudaGraphExecDestroy(backward_exec);
-  backward_exec = nullptr;
-  backward_passes = 0;
-}
-
-// The reverse replay, directly or through its captured graph: every Lambda
-// iteration and EOM product replays the same tape on the same buffers (some
-// 200 launches; from the host they leave gaps as long as the kernels of a
-// small system).  The first pass allocates and fills the caches, the second
-// is captured; a new tape or another symmetry of the replayed vector starts
-// over.
-int CCEngine::backward_run() {
-  if (backward_sym != ladder_sym) {
-    drop_backward_graph();
-    backward_sym = ladder_sym;
-  }
-  if (backward_exec) {
-    ACES_CUDA(cudaGraphLaunch(backward_exec, st));
-    g_launches.fetch_add(backward_launches, std::memory_order_relaxed);
-    return ACES_OK;
-  }
-  if (backward_passes++ == 0) return backward();
-  const long long l0 = g_launches.load();
-  cudaGraph_t graph = nullptr;
-  ACES_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  const int s = backward();
-  const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-  if (s != ACES_OK) {
-    if (graph) cudaGraphDestroy(graph);
-    return s;
-  }
-  if (ce != cudaSuccess) {
-    set_error("backward graph capture failed: %s", cudaGetErrorString(ce));
-    return ACES_ERR_CUDA;
-  }
-  backward_launches = g_launches.load() - l0;
-  const cudaError_t ie = cudaGraphInstantiate(&backward_exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (ie != cudaSuccess) {
-    backward_exec = nullptr;
-    set_error("backward graph instantiation failed: %s", cudaGetErrorString(ie));
-    return ACES_ERR_CUDA;
-  }
-  ACES_CUDA(cudaGraphLaunch(backward_exec, st));
-  return ACES_OK;
 }
 
 }  // namespace acesb200

@@ -31,7 +31,6 @@ std::vector<DBuf *> CCEngine::registry() {
 }
 
 void CCEngine::release() {
-  drop_backward_graph();
   for (auto &kv : adjoint) if (kv.second.p) dev_free(kv.second.p);
   adjoint.clear();
   for (auto &kv : tcache) if (kv.second.p) dev_free(kv.second.p);

@@ -173,12 +173,6 @@ class CCEngine {
                            DBuf &scratch);
   std::vector<char> first_writers();
   int backward();
-  // backward() through a CUDA graph captured on its second pass over a tape
-  int backward_run();
-  void drop_backward_graph();
-  cudaGraphExec_t backward_exec = nullptr;
-  int backward_passes = 0, backward_sym = 0;
-  long long backward_launches = 0;
   void zero_adjoints();
   int record_residual(bool fock_active);
   int tau_op(double *out, const double *t2, const double *t1, double c);

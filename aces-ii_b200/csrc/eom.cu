@@ -181,7 +181,7 @@ int CCEngine::eom_sigma(const double *x, double *out, int h, const int *d_irr_o,
   // the ladder couples occupied pairs of irrep g ^ h with virtual pairs of
   // irrep g for a vector of irrep h
   ladder_sym = h;
-  const int bs = backward_run();
+  const int bs = backward();
   ladder_sym = 0;
   ACES_TRY(bs);
   const double *g = adj(X.p);

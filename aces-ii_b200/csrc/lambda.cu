@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(256)
 
 int CCEngine::record_residual(bool fock_active) {
   // the forward values the previous tape's backward pass cached may change
-  drop_backward_graph();
   tape_cache_clear();
   tape.clear();
   active.clear();
@@ -130,7 +129,7 @@ int CCEngine::lambda_rhs() {
   if (!z1b || !z2b) return ACES_ERR_NOMEM;
   launch_axpy(z1b, L.p, 1.0, ov, st);
   launch_axpy(z2b, L.p + ov, 1.0, len - ov, st);
-  ACES_TRY(backward_run());
+  ACES_TRY(backward());
   double *xb = adj(X.p);
   ACES_TRY(alloc(lrhs, len));
   launch_copy(lrhs.p, gE.p, len, st);
