@@ -77,6 +77,65 @@ __global__ void k_permute_naive(double *__restrict__ out, PermArgs a, long long 
   }
 }
 
+// The gather of k_permute_naive where every source has unit stride along an
+// innermost extent of at least kRowMin that is no multiple of 4: a warp owns one
+// output row, so the index is split once per row and the loads of 128
+// elements are in flight (16-byte accesses would need aligned rows).  Bound by
+// memory: o = 17, v = 151, 53 MB with planes, 35 us one element per thread, 26 a
+// warp per row; o = 12, v = 65 4.9 and 3.9 us; 50-wide rows are a tie and
+// 34-wide ones slower (4.5 and 5.7 us), and few rows leave SMs idle.
+constexpr int kRowMin = 64, kRowsMin = 148 * 16;
+template <bool S>
+__global__ void __launch_bounds__(256)
+    k_permute_rows(double *__restrict__ out, PermArgs a, unsigned rows, SplitOut so) {
+  after_previous();
+  const int lane = threadIdx.x & 31, n3 = a.n[3];
+  const unsigned step = gridDim.x * (blockDim.x >> 5);
+  for (unsigned row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += step) {
+    unsigned r = row, q;
+    q = a.fd2.div(r); const int i2 = (int)(r - q * a.fd2.d); r = q;
+    q = a.fd1.div(r); const int i1 = (int)(r - q * a.fd1.d);
+    const int i0 = (int)q;
+    const long long idx = (long long)row * n3;
+    // the row's place in the planes; a row may run over the end of an operand row
+    long long p = 0;
+    bool whole = false;
+    if (S) {
+      const unsigned rr = so.fk.div((unsigned)idx), c = (unsigned)idx - rr * so.fk.d;
+      p = (long long)rr * so.k_pad + c;
+      whole = c + (unsigned)n3 <= so.fk.d;
+    }
+    for (int b = lane; b < n3; b += 128) {
+      double acc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        acc[u] = a.beta != 0.0 && b + 32 * u < n3 ? a.beta * out[idx + b + 32 * u] : 0.0;
+      for (int t = 0; t < a.nterms; ++t) {
+        const double *src = a.src[t] + i0 * a.s[t][0] + i1 * a.s[t][1] + i2 * a.s[t][2] + b;
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = b + 32 * u < n3 ? __ldg(src + 32 * u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] += a.alpha[t] * x[u];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i3 = b + 32 * u;
+        if (i3 >= n3) break;
+        if (!S || out) out[idx + i3] = acc[u];
+        if (S && whole) {
+          __nv_bfloat16 h, l;
+          split_bf16(acc[u], h, l);
+          so.hi[p + i3] = h;
+          so.lo[p + i3] = l;
+        } else if (S) {
+          put_split(so, idx + i3, acc[u]);
+        }
+      }
+    }
+  }
+}
+
 // The gather of k_permute_naive for outputs whose innermost extent is a
 // multiple of 4 (every source has unit stride along it): a thread owns 4
 // consecutive outputs of one row, splits its index once and issues 4
@@ -261,6 +320,11 @@ static void permute_launch(double *out, PermArgs &a, const PermSpec &spec, long 
       long long nq = (total / 4 + 255) / 256;
       if (nq > 148 * 64) nq = 148 * 64;
       launch_after(k_permute_rows4<S>, (unsigned)nq, 256, 0, st, out, a, total / 4, so);
+    } else if (all_unit3 && a.n[3] >= kRowMin && total / a.n[3] >= kRowsMin &&
+               total / a.n[3] < (1LL << 31)) {
+      const long long rows = total / a.n[3];
+      const long long nr = std::min<long long>((rows + 7) / 8, 148 * 64);
+      launch_after(k_permute_rows<S>, (unsigned)nr, 256, 0, st, out, a, (unsigned)rows, so);
     } else if (S || total < (1LL << 31)) {
       launch_after(k_permute_naive<false, S>, (unsigned)nb, 256, 0, st, out, a, total, so);
     } else {
