@@ -22,6 +22,8 @@ void engine_reset();
 // returns every cached block to the driver
 cudaError_t dev_alloc(void **ptr, size_t bytes);
 void dev_free(void *ptr);
+// whether dev_alloc would serve this size from a cached block
+bool dev_cached(size_t bytes);
 void pool_trim();
 
 // number of kernels the library has launched (reported by the benchmarks)

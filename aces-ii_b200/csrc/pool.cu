@@ -100,6 +100,20 @@ cudaError_t dev_alloc(void **ptr, size_t bytes) {
   return cudaSuccess;
 }
 
+bool dev_cached(size_t bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t cls = size_class(bytes);
+  Pool &P = pool();
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto it = P.free_blocks.lower_bound({dev, cls});
+  return it != P.free_blocks.end() && it->first.first == dev &&
+         it->first.second <= cls + cls / 4;
+}
+
 void dev_free(void *ptr) {
   if (!ptr) return;
   Pool &P = pool();

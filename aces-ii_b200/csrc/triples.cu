@@ -246,6 +246,20 @@ __global__ void __launch_bounds__(1024) k_sum_pairs(double *out, const double *p
     if (lane == 0) { out[0] = a; out[1] = b; }
   }
 }
+// Batch size of `slot`-byte W slots: up to 4 GB, and within a quarter of the
+// free memory unless the buffer is already in the allocator's cache (asking the
+// driver takes 0.1 to 70 ms on a machine that other processes allocate on: (T)
+// of o = 8, v = 70 3.0 ms, but 3 to 77 from run to run with the question).
+int batch_slots(double slot, int most) {
+  int nb = (int)std::max(1.0, std::min((double)most, 4.0e9 / slot));
+  if (dev_cached((size_t)(slot * nb))) return nb;
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    fr = 0;
+  }
+  return (int)std::max(1.0, std::min((double)nb, 0.25 * (double)fr / slot));
+}
 }  // namespace
 
 // The 12 contractions of a triplet (6 permutations x 2 terms) fall into three
@@ -303,17 +317,17 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
   const long long s3[4] = {O * O * V, O * V, V, 1};      // I_ooov[m,n,i,e]
   const long long st2[4] = {O * V * V, V * V, V, 1};     // t2[i,j,a,b]
   // Gv[k,b,c,d] = (bd|ck) = <bc|dk> = I_ovvv[k,d,c,b]; GvT[k,c,b,d] = Gv[k,b,c,d]
-  ACES_TRY(alloc(Gv, O * V3));
+  ACES_TRY(alloc(Gv, O * V3, false));
   ACES_TRY(perm(Gv.p, o, v, v, v, 0.0, {PermTerm{I_ovvv.p, 1.0, {sv[0], sv[3], sv[2], sv[1]}}}));
-  ACES_TRY(alloc(GvT, O * V3));
+  ACES_TRY(alloc(GvT, O * V3, false));
   ACES_TRY(perm(GvT.p, o, v, v, v, 0.0, {PermTerm{I_ovvv.p, 1.0, {sv[0], sv[2], sv[3], sv[1]}}}));
   // t2P[i,a,b,l] = t2[i,l,a,b]; t2Q[i,b,a,l] = t2[i,l,a,b]
-  ACES_TRY(alloc(t2P, O * O * V2));
+  ACES_TRY(alloc(t2P, O * O * V2, false));
   ACES_TRY(perm(t2P.p, o, v, v, o, 0.0, {PermTerm{t2(), 1.0, {st2[0], st2[2], st2[3], st2[1]}}}));
-  ACES_TRY(alloc(t2Q, O * O * V2));
+  ACES_TRY(alloc(t2Q, O * O * V2, false));
   ACES_TRY(perm(t2Q.p, o, v, v, o, 0.0, {PermTerm{t2(), 1.0, {st2[0], st2[3], st2[2], st2[1]}}}));
   // Hn[j,k,c,l] = -(ck|jl) = -I_ooov[l,k,j,c] (the second terms enter with a minus sign)
-  ACES_TRY(alloc(Hn, O * O * O * V));
+  ACES_TRY(alloc(Hn, O * O * O * V, false));
   ACES_TRY(perm(Hn.p, o, o, v, o, 0.0, {PermTerm{I_ooov.p, -1.0, {s3[2], s3[1], s3[3], s3[0]}}}));
   // triplets i >= j >= k of this shard: index t (i, then j <= i, then k <= j)
   // with t % nranks == rank
@@ -354,16 +368,8 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
       dev_free(b->p);
       b->p = nullptr;
     }
-    // batch size: FP32 W slots within a quarter of the free memory, <= 4 GB
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-      cudaGetLastError();
-      fr = 0;
-    }
-    const double slot = (double)V3 * sizeof(float);
-    const double budget = std::min(0.25 * (double)fr, 4.0e9);
-    const int nb = (int)std::max(1.0, std::min((double)std::max(ntrip, 1), budget / slot));
-    ACES_TRY(alloc(Wb, (size_t)((V3 * nb + 1) / 2)));  // FP32 slots in a double buffer
+    const int nb = batch_slots((double)V3 * sizeof(float), std::max(ntrip, 1));
+    ACES_TRY(alloc(Wb, (size_t)((V3 * nb + 1) / 2), false));  // FP32 slots in a double buffer
     // class c runs transposed on the 256 x 192 tiles (M = (a,b), N = c: the
     // ragged side is the one whose MMA N is cut to the live columns, where on
     // 128-row tiles M = c = v would leave 256 - v rows idle), and stores W
@@ -401,7 +407,7 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
     const SplitOperand Aa[4] = {sGv, sGvT, sT2P, sT2Q}, Ba[4] = {sT2, sT2, sHn, sHn};
     const int nt = (v + kTile - 1) / kTile;
     const int nblk = nt * (nt + 1) * (nt + 2) / 6;   // tile triples A >= B >= C
-    ACES_TRY(alloc(part, (size_t)std::max(ntrip, 1) * nblk * 2));
+    ACES_TRY(alloc(part, (size_t)std::max(ntrip, 1) * nblk * 2, false));
     for (int t0b = 0; t0b < ntrip; t0b += nb) {
       const int n = std::min(nb, ntrip - t0b);
       CView cv = c_wide ? vcT : vc;
@@ -432,19 +438,12 @@ int CCEngine::triples(double *e4, double *e5, double *seconds, int rank, int nra
     // batch is one launch over a table of tasks (four K segments each).  One
     // triplet at a time took 13 launches of about 10 us each at o = 8, v = 70:
     // 13.5 ms of kernels and 7 ms of gaps between them.
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-      cudaGetLastError();
-      fr = 0;
-    }
-    const double slot = (double)V3 * sizeof(double);
-    const double budget = std::min(0.25 * (double)fr, 4.0e9);
-    const int nb = (int)std::max(
-        1.0, std::min({(double)std::max(ntrip, 1), budget / slot, (double)kMaxTasks}));
-    ACES_TRY(alloc(Wb, V3 * nb));
+    const int nb =
+        batch_slots((double)V3 * sizeof(double), std::min(std::max(ntrip, 1), kMaxTasks));
+    ACES_TRY(alloc(Wb, V3 * nb, false));
     const int nt = (v + kTile - 1) / kTile;
     const int nblk = nt * (nt + 1) * (nt + 2) / 6;
-    ACES_TRY(alloc(part, (size_t)std::max(ntrip, 1) * nblk * 2));
+    ACES_TRY(alloc(part, (size_t)std::max(ntrip, 1) * nblk * 2, false));
     auto T2p = [&](int x, int y) { return t2() + ((long long)x * o + y) * V * V; };
     auto Hp = [&](int y, int z) { return Hn.p + ((long long)y * o + z) * V * O; };
     auto Gp = [&](int z) { return Gv.p + (long long)z * V2 * V; };
