@@ -738,7 +738,8 @@ namespace {
 // per SM, 33.9 with 128 x 64 and two, 29.7 with 128 x 128 and one (the
 // m8n8k4 and the m16n8k8 form of the instruction measure the same); and the
 // last wave and the ragged edges of a 64-wide grid cost less: 2401 x 1519 x
-// 2050 takes 525 us against 734.  32 x 32 tiles serve outputs too small for
+// 2050 takes 525 us against 734 (shapes measured with 128-bit fragment loads; k
+// in ascending order, as now, costs 1-2 %).  32 x 32 tiles serve outputs too small for
 // that: 120 x 96 x 150 in 8.7 us against 41.9 on one 128 x 128 tile.  The
 // 16- and 32-wide tiles are for products with a short side, which stream
 // their long operand: 404600 x 14 x 170 in 113 us (550 MB, 4.9 TB/s) against

@@ -15,9 +15,9 @@
 // G_h = F_h F_h'^T per pair irrep h over the packed rows F[(pr)][L], and only
 // the lower triangle of tiles where both sides are the same pairs (lists 13,
 // 16 and 233).  Bandwidth-bound kernels then write the list blocks from G.
-// o = 20, v = 180, naux = 600: 52.4 ms of dense products became 7.4 ms of
-// packed ones (32.7 TFLOP/s) and 3.2 ms of expansion; with 8 irreps the products shrink by
-// another factor of 64 at most.
+// o = 20, v = 180, naux = 600: 52.4 ms of dense products became 7.5 ms of
+// packed ones (32 TFLOP/s) and 3.2 ms of expansion; with 8 irreps the products
+// shrink by another factor of 64 at most.
 //
 // The factors are symmetric by contract; factors that are not (beyond
 // rounding: 64 units in the last place of the largest element) take dense
