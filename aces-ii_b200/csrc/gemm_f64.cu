@@ -852,7 +852,11 @@ int gemm_dispatch(int M, int N, int K, double alpha, const double *A, long long 
   L.beta = beta;
   const int nkt = f64_ktiles(t);
   const size_t kOwn = size_t(1) << 25;  // of the library's own workspace: 256 MB
-  const F64Plan p = plan_f64(t.M, t.N, nkt, ws ? cap : kOwn);
+  F64Plan p = plan_f64(t.M, t.N, nkt, ws ? cap : kOwn);
+  if (p.Z > 1) {
+    L.part = ws ? ws : splitk_workspace((size_t)p.Z * t.M * t.N);
+    if (!L.part) p = plan_f64(t.M, t.N, nkt, 0);  // no room for the partials: unsplit
+  }
   const long long tiles = (long long)((t.M + kTile[p.tile].BM - 1) / kTile[p.tile].BM) *
                           ((t.N + kTile[p.tile].BN - 1) / kTile[p.tile].BN);
   if (tiles > 0x7fffffffLL) {
@@ -863,11 +867,6 @@ int gemm_dispatch(int M, int N, int K, double alpha, const double *A, long long 
   if (Z > 1) {
     L.kchunk = (nkt + Z - 1) / Z;
     Z = (nkt + L.kchunk - 1) / L.kchunk;
-    L.part = ws ? ws : splitk_workspace((size_t)Z * t.M * t.N);
-    if (!L.part) {
-      set_error("gemm_nt_f64: split-K workspace allocation failed");
-      return ACES_ERR_NOMEM;
-    }
   }
   if (vec2_ok(t))
     ACES_TRY(launch_id<2>(p.tile, L, (unsigned)tiles, (unsigned)Z, st));

@@ -1682,18 +1682,15 @@ int multi_run(const TuneChoice &ch, const SplitOperand *A, const SplitOperand *B
     P.ktc = (P.kTilesTotal + Z - 1) / Z;
     Z = (P.kTilesTotal + P.ktc - 1) / P.ktc;
     part = splitk_workspace((size_t)Z * M * N);
-    if (!part) {
-      set_error("gemm_nt_bf16x3: split-K workspace allocation failed");
-      return ACES_ERR_NOMEM;
+    if (!part) {  // no room for the partials: one slice needs none
+      Z = 1;
+      P.ktc = P.kTilesTotal;
     }
   }
   if (Z == 1 && L.cg == 1) plan_tail(P, 0, nsm);
   if (P.tailZ) {
     part = splitk_workspace(tail_doubles(P));
-    if (!part) {
-      set_error("gemm_nt_bf16x3: split-K workspace allocation failed");
-      return ACES_ERR_NOMEM;
-    }
+    if (!part) P.tailZ = 0;  // whole tiles
   }
   const long long nTiles = P.tailZ ? tail_tiles(P) : tiles * Z;
   if (nTiles > (1LL << 31) - 1) {
@@ -1730,12 +1727,11 @@ int grouped_run(int cg, const GroupedProblem *probs, int nprob, double alpha, do
   double *part = nullptr;
   if (L.cg == 1) plan_tail(P, P.tile0, num_sms());
   if (P.tailZ) {
-    tiles = P.tile0 + tail_tiles(P);
     part = splitk_workspace(tail_doubles(P));
-    if (!part) {
-      set_error("gemm_nt_bf16x3_grouped: split-K workspace allocation failed");
-      return ACES_ERR_NOMEM;
-    }
+    if (part)
+      tiles = P.tile0 + tail_tiles(P);
+    else
+      P.tailZ = 0;  // no room for the parts: whole tiles
   }
   if (tiles > (1LL << 31) - 1) {
     set_error("gemm_nt_bf16x3_grouped: %lld output tiles exceed the scheduler range", tiles);
