@@ -26,6 +26,31 @@ void dev_free(void *ptr);
 bool dev_cached(size_t bytes);
 void pool_trim();
 
+// One call of an entry point on its host thread.  A block that dev_free takes
+// back during the call may still be read or written by kernels the call has
+// launched, so it stays with the thread: the thread's own dev_alloc hands it out
+// again (the later use is ordered by the stream), other threads get it only
+// after the call has waited for its streams.
+class CallScope {
+ public:
+  CallScope();
+  ~CallScope();  // waits, unless wait() has been called
+  CallScope(const CallScope &) = delete;
+  CallScope &operator=(const CallScope &) = delete;
+  // a stream of the call besides stream 0 (read when the scope waits)
+  void also(const cudaStream_t *st) { extra = st; }
+  // waits for the call's streams; no launch may follow
+  cudaError_t wait();
+
+ private:
+  const cudaStream_t *extra = nullptr;
+  bool waited = false;
+};
+// scratch of the running call, at least `bytes` long: one buffer that the
+// call's products use in turn, given back when the call ends; nullptr outside a
+// call or when there is no memory
+void *call_workspace(size_t bytes);
+
 // number of kernels the library has launched (reported by the benchmarks)
 extern std::atomic<long long> g_launches;
 // Launches that follow one another on a stream.  A kernel launched with

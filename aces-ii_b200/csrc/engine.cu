@@ -1488,8 +1488,10 @@ extern "C" int xvcc_run(aces_cc_config *cfg) {
     return ACES_ERR_ARG;
   }
   if (cfg->precision != ACES_PREC_FP64 && cfg->precision != ACES_PREC_BF16X3) return ACES_ERR_ARG;
+  CallScope call;
   engine_reset();
   CCEngine &E = *engine_instance(true);
+  call.also(&E.st);
   E.prec = cfg->precision;
   E.use_graph = cfg->use_graph != 0;
   if (!(cfg->damp >= 0.0 && cfg->damp <= 1.0)) {

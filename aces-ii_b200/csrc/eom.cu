@@ -228,6 +228,8 @@ extern "C" int xvee_run(aces_eom_config *cfg) {
       return ACES_ERR_ARG;
     }
   if (cfg->precision != ACES_PREC_FP64 && cfg->precision != ACES_PREC_BF16X3) return ACES_ERR_ARG;
+  CallScope call;
+  call.also(&E.st);
   E.prec = cfg->precision;
   const int o = E.o, v = E.v;
   const long long ov = (long long)o * v, len = ov + (long long)o * o * v * v;

@@ -638,37 +638,10 @@ static int launch_lowrank(int M, int N, int K, double alpha, const double *A, lo
   return ACES_OK;
 }
 
-// split-K partials: one buffer per host thread and device, grown on demand and
-// given back when the thread ends.  A call's products run on one stream in
-// order, and every entry point waits for its stream before it returns, so
-// calls of one thread share the buffer and those of different threads (a
-// product beside a CC solve) do not.
+// split-K partials: the running call's workspace, which its products use in
+// turn on one stream
 double *splitk_workspace(size_t doubles) {
-  struct Ws {
-    double *p[64] = {nullptr};
-    size_t cap[64] = {0};
-    ~Ws() {
-      for (double *q : p)
-        if (q) dev_free(q);
-    }
-  };
-  static thread_local Ws ws;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (doubles > ws.cap[dev]) {
-    if (ws.p[dev]) dev_free(ws.p[dev]);
-    ws.p[dev] = nullptr;
-    ws.cap[dev] = 0;
-    if (dev_alloc((void **)&ws.p[dev], doubles * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    ws.cap[dev] = doubles;
-  }
-  return ws.p[dev];
+  return static_cast<double *>(call_workspace(doubles * sizeof(double)));
 }
 
 int splitk_reduce(const CView &C, const double *part, int M, int N, int Z, double alpha,

@@ -202,11 +202,10 @@ int tri_tiles(int n) {
   return t * (t + 1) / 2;
 }
 
-// Device memory of one call, given back (after the stream is done) at its end.
+// Device memory of one call, given back at its end.
 struct Scratch {
   std::vector<void *> p;
   ~Scratch() {
-    cudaStreamSynchronize(0);
     for (void *q : p) dev_free(q);
   }
   void *get(size_t bytes) {
@@ -427,12 +426,12 @@ extern "C" int aces_intprc_df(const double *B, int naux, int on_device) {
     set_error("aces_intprc_df: empty occupied or virtual space");
     return ACES_ERR_ARG;
   }
+  CallScope call;
   cudaStream_t st = 0;
   std::vector<void *> owned;
   struct Free {
     std::vector<void *> &p;
     ~Free() {
-      cudaStreamSynchronize(0);
       for (void *q : p) dev_free(q);
     }
   } release{owned};

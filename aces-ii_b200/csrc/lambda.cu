@@ -213,6 +213,8 @@ extern "C" int xlambda_run(aces_cc_config *cfg) {
     return ACES_ERR_ARG;
   }
   CCEngine &E = *Ep;
+  CallScope call;
+  call.also(&E.st);
   E.prec = cfg->precision;
   const long long O = E.o, V = E.v, ov = O * V, len = ov + O * O * V * V;
   ACES_TRY(E.alloc(E.L, len));
@@ -308,6 +310,8 @@ extern "C" int xdens_1pdm(aces_cc_config *cfg) {
     set_error("xdens_1pdm: no converged Lambda (run xvcc_run and xlambda_run first)");
     return ACES_ERR_ARG;
   }
+  CallScope call;
+  call.also(&Ep->st);
   std::vector<double> D;
   ACES_TRY(Ep->density(D));
   for (double x : D)

@@ -17,9 +17,11 @@
 namespace acesb200 {
 
 namespace {
+using Blocks = std::multimap<std::pair<int, size_t>, void *>;
+
 struct Pool {
   std::mutex mu;
-  std::multimap<std::pair<int, size_t>, void *> free_blocks;   // (device, bytes) -> block
+  Blocks free_blocks;                                          // (device, bytes) -> block
   std::unordered_map<void *, std::pair<int, size_t>> live;     // block -> (device, bytes)
   std::map<int, size_t> cached;                                // device -> cached bytes
   std::map<int, size_t> cap;                                   // device -> cache limit
@@ -51,16 +53,73 @@ size_t size_class(size_t bytes) {
   while (c < bytes) c <<= 1;
   return c;
 }
-void trim_device(Pool &P, int dev) {
-  for (auto it = P.free_blocks.begin(); it != P.free_blocks.end();) {
+// the running call of this thread (CallScope): its depth, the blocks it has
+// given back, and its workspace
+struct Call {
+  int depth = 0;
+  Blocks held;
+  std::map<int, size_t> bytes;  // device -> held bytes
+  void *ws = nullptr;
+  size_t ws_bytes = 0;
+  int ws_dev = -1;
+};
+Call &call() {
+  static thread_local Call c;
+  return c;
+}
+
+void trim_device(Blocks &blocks, std::map<int, size_t> &bytes, int dev) {
+  for (auto it = blocks.begin(); it != blocks.end();) {
     if (it->first.first == dev) {
       cudaFree(it->second);
-      it = P.free_blocks.erase(it);
+      it = blocks.erase(it);
     } else {
       ++it;
     }
   }
-  P.cached[dev] = 0;
+  bytes[dev] = 0;
+}
+// smallest block of the device that fits without wasting more than a quarter of
+// the size asked for
+Blocks::iterator best_fit(Blocks &blocks, int dev, size_t cls) {
+  auto it = blocks.lower_bound({dev, cls});
+  return it != blocks.end() && it->first.first == dev && it->first.second <= cls + cls / 4
+             ? it
+             : blocks.end();
+}
+// largest block of the device
+Blocks::iterator largest(Blocks &blocks, int dev) {
+  auto it = blocks.lower_bound({dev + 1, 0});
+  if (it == blocks.begin()) return blocks.end();
+  --it;
+  return it->first.first == dev ? it : blocks.end();
+}
+
+// keeps a block: with the running call (its kernels may still use it), else in
+// the pool; over the limit, cached blocks go to the driver, largest first
+// (cudaFree waits for the device), then the block itself if it still does not
+// fit
+void keep(Pool &P, Call &C, int dev, size_t bytes, void *ptr) {
+  int cur = -1;
+  cudaGetDevice(&cur);
+  const size_t cap = cur == dev ? cache_cap(P, dev) : 0;
+  while (P.cached[dev] + C.bytes[dev] + bytes > cap) {
+    auto p = largest(P.free_blocks, dev), h = largest(C.held, dev);
+    if (p == P.free_blocks.end() && h == C.held.end()) break;
+    const bool mine = p == P.free_blocks.end() ||
+                      (h != C.held.end() && h->first.second > p->first.second);
+    Blocks &from = mine ? C.held : P.free_blocks;
+    auto it = mine ? h : p;
+    cudaFree(it->second);
+    (mine ? C.bytes : P.cached)[dev] -= it->first.second;
+    from.erase(it);
+  }
+  if (P.cached[dev] + C.bytes[dev] + bytes > cap) {
+    cudaFree(ptr);
+    return;
+  }
+  (C.depth ? C.held : P.free_blocks).emplace(std::make_pair(dev, bytes), ptr);
+  (C.depth ? C.bytes : P.cached)[dev] += bytes;
 }
 }  // namespace
 
@@ -72,23 +131,26 @@ cudaError_t dev_alloc(void **ptr, size_t bytes) {
   const size_t cls = size_class(bytes);
   g_alloc_calls.fetch_add(1, std::memory_order_relaxed);
   Pool &P = pool();
+  Call &C = call();
   std::lock_guard<std::mutex> lk(P.mu);
-  // smallest cached block of this device that fits without wasting more than
-  // a quarter of it
-  auto it = P.free_blocks.lower_bound({dev, cls});
-  if (it != P.free_blocks.end() && it->first.first == dev &&
-      it->first.second <= cls + cls / 4) {
+  auto p = best_fit(P.free_blocks, dev, cls), h = best_fit(C.held, dev, cls);
+  if (p != P.free_blocks.end() || h != C.held.end()) {
+    const bool mine = p == P.free_blocks.end() ||
+                      (h != C.held.end() && h->first.second <= p->first.second);
+    Blocks &from = mine ? C.held : P.free_blocks;
+    auto it = mine ? h : p;
     *ptr = it->second;
     P.live[*ptr] = it->first;
-    P.cached[dev] -= it->first.second;
-    P.free_blocks.erase(it);
+    (mine ? C.bytes : P.cached)[dev] -= it->first.second;
+    from.erase(it);
     return cudaSuccess;
   }
   g_driver_allocs.fetch_add(1, std::memory_order_relaxed);
   e = cudaMalloc(ptr, cls);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    trim_device(P, dev);
+    trim_device(P.free_blocks, P.cached, dev);
+    trim_device(C.held, C.bytes, dev);
     e = cudaMalloc(ptr, cls);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -109,9 +171,9 @@ bool dev_cached(size_t bytes) {
   const size_t cls = size_class(bytes);
   Pool &P = pool();
   std::lock_guard<std::mutex> lk(P.mu);
-  auto it = P.free_blocks.lower_bound({dev, cls});
-  return it != P.free_blocks.end() && it->first.first == dev &&
-         it->first.second <= cls + cls / 4;
+  Call &C = call();
+  return best_fit(P.free_blocks, dev, cls) != P.free_blocks.end() ||
+         best_fit(C.held, dev, cls) != C.held.end();
 }
 
 void dev_free(void *ptr) {
@@ -123,28 +185,53 @@ void dev_free(void *ptr) {
   const int dev = it->second.first;
   const size_t bytes = it->second.second;
   P.live.erase(it);
-  int cur = -1;
-  cudaGetDevice(&cur);
-  const size_t cap = cur == dev ? cache_cap(P, dev) : 0;
-  if (P.cached[dev] + bytes > cap) {
-    // over the limit: release cached blocks of this device, largest first,
-    // then the block itself if it still does not fit
-    while (P.cached[dev] + bytes > cap) {
-      auto last = P.free_blocks.lower_bound({dev + 1, 0});
-      if (last == P.free_blocks.begin()) break;
-      --last;
-      if (last->first.first != dev) break;
-      cudaFree(last->second);
-      P.cached[dev] -= last->first.second;
-      P.free_blocks.erase(last);
-    }
-    if (P.cached[dev] + bytes > cap) {
-      cudaFree(ptr);
-      return;
-    }
+  keep(P, call(), dev, bytes, ptr);
+}
+
+CallScope::CallScope() { ++call().depth; }
+
+cudaError_t CallScope::wait() {
+  waited = true;
+  cudaError_t e = cudaStreamSynchronize(0);
+  if (extra && *extra) {
+    const cudaError_t x = cudaStreamSynchronize(*extra);
+    if (e == cudaSuccess) e = x;
   }
-  P.free_blocks.emplace(std::make_pair(dev, bytes), ptr);
-  P.cached[dev] += bytes;
+  return e;
+}
+
+CallScope::~CallScope() {
+  if (!waited) wait();
+  Call &C = call();
+  if (--C.depth) return;
+  if (C.ws) dev_free(C.ws);
+  C.ws = nullptr;
+  Pool &P = pool();
+  std::lock_guard<std::mutex> lk(P.mu);
+  Blocks held;
+  held.swap(C.held);
+  C.bytes.clear();
+  for (auto &b : held) keep(P, C, b.first.first, b.first.second, b.second);
+}
+
+void *call_workspace(size_t bytes) {
+  Call &C = call();
+  int dev = 0;
+  if (!C.depth || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (C.ws && C.ws_dev == dev && C.ws_bytes >= bytes) return C.ws;
+  if (C.ws) dev_free(C.ws);
+  C.ws = nullptr;
+  if (dev_alloc(&C.ws, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    C.ws = nullptr;
+    return nullptr;
+  }
+  C.ws_dev = dev;
+  C.ws_bytes = bytes;
+  return C.ws;
 }
 
 void pool_trim() {

@@ -43,6 +43,7 @@ extern "C" int aces_xgemm(char transa, char transb, int m, int n, int k, double 
     set_error("aces_xgemm: lda %d or ldb %d below the operand's row count", lda, ldb);
     return ACES_ERR_ARG;
   }
+  CallScope call;
   cudaStream_t st = 0;
   // NT form: Ak[i*K + l] = op(A)(i,l), Bk[j*K + l] = op(B)(l,j)
   const double *Ak = A, *Bk = B;
@@ -57,7 +58,6 @@ extern "C" int aces_xgemm(char transa, char transb, int m, int n, int k, double 
     if (status == ACES_OK)
       status = tb == 'T' ? split_pack_t(sb, B, ldb, n, k, st) : split_pack(sb, B, ldb, n, k, st);
     if (status == ACES_OK) status = gemm_nt_bf16x3(sa, sb, m, n, alpha, beta, C, st);
-    cudaStreamSynchronize(st);
     if (sa.hi) dev_free(sa.hi);
     if (sb.hi) dev_free(sb.hi);
   } else {
@@ -74,7 +74,7 @@ extern "C" int aces_xgemm(char transa, char transb, int m, int n, int k, double 
     if (status == ACES_OK)
       status = gemm_nt_f64(m, n, k, alpha, Ak, ldak, Bk, ldbk, beta, C, st);
   }
-  cudaError_t e = cudaStreamSynchronize(st);
+  cudaError_t e = call.wait();
   if (tA) dev_free(tA);
   if (tB) dev_free(tB);
   if (status == ACES_OK && e != cudaSuccess) {

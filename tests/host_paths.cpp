@@ -13,10 +13,7 @@ static int product(int precision, int m, int n, int k, size_t budget) {
   host::launches.clear();
   pool_trim();
   host::budget = host::live + budget;
-  int rc = 0;
-  std::thread([&] {  // a thread that holds no workspace yet
-    rc = aces_xgemm('T', 'N', m, n, k, 1.0, addr(0), k, addr(1), k, 0.0, addr(2), m, precision);
-  }).join();
+  const int rc = aces_xgemm('T', 'N', m, n, k, 1.0, addr(0), k, addr(1), k, 0.0, addr(2), m, precision);
   host::budget = ~size_t(0);
   return rc == ACES_OK ? (int)host::launches.size() : -1;
 }
@@ -46,11 +43,107 @@ static int no_room_for_partials() {
     pool_trim();
     host::budget = host::live + (room ? 256 * MB : 0);
     int rc = 0;
-    std::thread([&] { rc = gemm_nt_bf16x3_grouped(pr, 2, 1.0, 0.0, 0); }).join();
+    {
+      CallScope call;
+      rc = gemm_nt_bf16x3_grouped(pr, 2, 1.0, 0.0, 0);
+    }
     CHECK(rc == ACES_OK);
     CHECK((int)host::launches.size() == 1 + room);
     host::budget = ~size_t(0);
   }
+  return 0;
+}
+
+// Blocks given back during a call stay with its thread until the call has
+// waited for its streams.
+static int blocks_stay_with_their_call() {
+  const size_t MB = size_t(1) << 20;
+  cudaStream_t st;
+  cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  void *q = nullptr, *own = nullptr, *a = nullptr, *b = nullptr;
+  double *p = nullptr;
+  {
+    CallScope call;
+    call.also(&st);
+    p = splitk_workspace(1000);
+    CHECK(p && dev_alloc(&q, MB) == cudaSuccess);
+    host::launch(nullptr, st, dim3(1), true);   // reads both
+    CHECK(splitk_workspace(1000) == p && splitk_workspace(8 * MB) != p);
+    dev_free(q);
+    std::thread([&] {
+      dev_alloc(&a, 8000);
+      dev_alloc(&b, MB);
+    }).join();
+    CHECK(a && b && a != p && b != q);
+    CHECK(dev_alloc(&own, MB) == cudaSuccess && own == q);
+    dev_free(own);
+    CHECK(host::pending[st] == 1);
+  }
+  CHECK(host::pending[st] == 0);
+  std::thread([&] { dev_alloc(&b, MB); }).join();
+  CHECK(b == q);
+  return 0;
+}
+
+// a system of o occupied and v virtual orbitals, its lists filled with zeros
+static int small_system(int o, int v) {
+  const int list[6][3] = {{13, 14, 14}, {10, 14, 18}, {16, 13, 14},
+                          {25, 11, 11}, {30, 13, 11}, {233, 13, 13}};
+  int rc = aces_init(0);
+  if (rc == ACES_OK) rc = aces_sym_init(1, &o, &v);
+  for (auto &l : list)
+    if (rc == ACES_OK) rc = aces_inipck(1, l[1], l[2], l[0], 1);
+  std::vector<double> eps(o + v);
+  for (int i = 0; i < o + v; ++i) eps[i] = i < o ? -1.0 : 1.0 + i;
+  return rc == ACES_OK ? aces_putrec("SCFEVALA", (long long)eps.size() * 8, eps.data()) : rc;
+}
+
+// Every entry point that launches does so inside a call, and no stream is left
+// running when it returns, an error included.
+static int entry_points_wait() {
+  int outside = 0;
+  host::on_launch = [&] { outside += call_workspace(1) == nullptr; };
+  auto idle = [] {
+    for (auto &s : host::pending)
+      if (s.second) return false;
+    return true;
+  };
+  std::vector<double> B(30 * 14 * 14, 0.1);
+  aces_cc_config cc{};
+  cc.cc_conv = 7;
+  cc.cc_maxcyc = 5;
+  cc.cc_exporder = 5;
+  CHECK(small_system(4, 10) == ACES_OK);
+  CHECK(aces_intprc_df(B.data(), 30, 0) == ACES_OK && idle());
+  for (int prec : {ACES_PREC_FP64, ACES_PREC_BF16X3}) {
+    cc.precision = prec;
+    cc.triples = 1;
+    CHECK(xvcc_run(&cc) == ACES_OK && idle());
+    CHECK(xlambda_run(&cc) == ACES_OK && idle());
+    CHECK(xdens_1pdm(&cc) == ACES_OK && idle());
+    CHECK(aces_xgemm('N', 'T', 200, 150, 6000, 1.0, addr(0), 200, addr(1), 150, 0.0, addr(2), 200,
+                     prec) == ACES_OK && idle());
+  }
+  aces_eom_config eom{};
+  eom.nroots[0] = 1;
+  eom.eom_conv = 5;
+  eom.eom_maxcyc = 2;
+  const int ee = xvee_run(&eom);
+  CHECK((ee == ACES_OK || ee == ACES_ERR_NOCONV) && idle());
+  CHECK(outside == 0);
+  // out of memory somewhere in the solve
+  const size_t n0 = host::launches.size();
+  int failed = 0;
+  for (size_t room = 1; room < 64; room += 4) {
+    CHECK(small_system(8, 40) == ACES_OK);
+    pool_trim();
+    host::budget = host::live + (room << 20);
+    failed += xvcc_run(&cc) == ACES_ERR_NOMEM;
+    host::budget = ~size_t(0);
+    CHECK(idle());
+  }
+  CHECK(failed > 2 && host::launches.size() > n0);
+  host::on_launch = [] {};
   return 0;
 }
 
@@ -60,6 +153,8 @@ struct Case {
 };
 static const Case cases[] = {
     {"no_room_for_partials", no_room_for_partials},
+    {"blocks_stay_with_their_call", blocks_stay_with_their_call},
+    {"entry_points_wait", entry_points_wait},
 };
 
 int main(int argc, char **argv) {
