@@ -50,6 +50,8 @@ class CallScope {
 // call's products use in turn, given back when the call ends; nullptr outside a
 // call or when there is no memory
 void *call_workspace(size_t bytes);
+// whether the running call has launched nothing yet; true once per call
+bool call_first_launch();
 
 // number of kernels the library has launched (reported by the benchmarks)
 extern std::atomic<long long> g_launches;
@@ -63,6 +65,8 @@ extern std::atomic<long long> g_launches;
 // the new one has started.  Back-to-back dependent launches, direct or from a
 // captured graph, lose 1-1.5 us each without it: EOM o = 6, v = 50 (2900
 // launches) 15.2 -> 13.4 ms, CCSD o = 5, v = 21 3.10 -> 2.72 ms.
+// The first kernel of a call follows a kernel of the caller, which may release
+// its successors early: it is launched in plain stream order.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -78,7 +82,7 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = call_first_launch() ? 0 : 1;
   // an error stays for the caller's cudaGetLastError, as after <<< >>>
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }

@@ -57,6 +57,7 @@ size_t size_class(size_t bytes) {
 // given back, and its workspace
 struct Call {
   int depth = 0;
+  bool launched = false;
   Blocks held;
   std::map<int, size_t> bytes;  // device -> held bytes
   void *ws = nullptr;
@@ -188,7 +189,17 @@ void dev_free(void *ptr) {
   keep(P, call(), dev, bytes, ptr);
 }
 
-CallScope::CallScope() { ++call().depth; }
+CallScope::CallScope() {
+  Call &C = call();
+  if (C.depth++ == 0) C.launched = false;
+}
+
+bool call_first_launch() {
+  Call &C = call();
+  const bool first = !C.launched;
+  C.launched = true;
+  return first;
+}
 
 cudaError_t CallScope::wait() {
   waited = true;

@@ -106,6 +106,7 @@ extern "C" int aces_xgemm_static(char transa, char transb, int m, int n, int k, 
   }
   double *scratch = nullptr;
   ACES_TRY(scratch_address(&scratch));
+  CallScope call;
   cudaStream_t st = 0;
   const double *Ak = A, *Bk = B;
   long long ldak = lda, ldbk = ldb;
@@ -128,7 +129,7 @@ extern "C" int aces_xgemm_static(char transa, char transb, int m, int n, int k, 
   size_t cap = used < kStaticScratchDoubles ? kStaticScratchDoubles - used : 0;
   int status = gemm_nt_f64_scratch(m, n, k, alpha, Ak, ldak, Bk, ldbk, beta,
                                    cview_colmajor(Cm, ldc), ws, cap, st);
-  cudaError_t e = cudaStreamSynchronize(st);
+  cudaError_t e = call.wait();
   if (status == ACES_OK && e != cudaSuccess) {
     set_error("aces_xgemm_static: %s", cudaGetErrorString(e));
     status = ACES_ERR_CUDA;

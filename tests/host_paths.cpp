@@ -147,6 +147,34 @@ static int entry_points_wait() {
   return 0;
 }
 
+// The first kernel of a call waits in plain stream order for whatever the
+// caller launched before it; the later ones may be set up early.
+static int first_launch_in_order() {
+  auto ordered = [](size_t n) {
+    if (host::launches.size() < n || host::launches[0].overlapped) return false;
+    for (size_t i = 1; i < host::launches.size(); ++i)
+      if (!host::launches[i].overlapped) return false;
+    return true;
+  };
+  for (int prec : {ACES_PREC_FP64, ACES_PREC_BF16X3})
+    for (int rep = 0; rep < 2; ++rep) {
+      host::launches.clear();
+      CHECK(aces_xgemm('N', 'T', 200, 150, 6000, 1.0, addr(0), 200, addr(1), 150, 0.0, addr(2), 200,
+                       prec) == ACES_OK);
+      CHECK(ordered(3));
+      host::launches.clear();
+      CHECK(aces_xgemm_static('N', 'T', 200, 150, 600, 1.0, addr(0), 200, addr(1), 150, 0.0,
+                              addr(2), 200) == ACES_OK);
+      CHECK(ordered(2));
+    }
+  std::vector<double> B(30 * 14 * 14, 0.0);
+  CHECK(small_system(4, 10) == ACES_OK);
+  host::launches.clear();
+  CHECK(aces_intprc_df(B.data(), 30, 0) == ACES_OK);
+  CHECK(ordered(3));
+  return 0;
+}
+
 struct Case {
   const char *name;
   int (*run)();
@@ -155,6 +183,7 @@ static const Case cases[] = {
     {"no_room_for_partials", no_room_for_partials},
     {"blocks_stay_with_their_call", blocks_stay_with_their_call},
     {"entry_points_wait", entry_points_wait},
+    {"first_launch_in_order", first_launch_in_order},
 };
 
 int main(int argc, char **argv) {
