@@ -173,9 +173,20 @@ struct PairType {
 };
 PairType pair_type(int type);   // type 1..25
 
-// aces_inipck with the choice of leaving a new list's memory unfilled (for a
-// producer that writes every element)
-int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, bool zero);
+// New list blocks whose memory a producer writes whole: created without the
+// zero fill, and zeroed after all when the producer ends without calling
+// written() (an error must not leave old device memory in a list).
+class UnfilledLists {
+ public:
+  ~UnfilledLists();
+  void add(double *p, size_t bytes) { blocks.push_back({p, bytes}); }
+  void written() { blocks.clear(); }
+
+ private:
+  std::vector<std::pair<double *, size_t>> blocks;
+};
+// aces_inipck; with `unfilled`, the memory of new blocks is left to the producer
+int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, UnfilledLists *unfilled);
 
 // Orbital count of irrep h (0-based) for 'O'/'V' (RHF: alpha == beta).
 inline int norb(const SymInfo &s, char c, int h) { return c == 'O' ? s.pop[h] : s.vrt[h]; }

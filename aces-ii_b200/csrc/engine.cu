@@ -1418,12 +1418,14 @@ int CCEngine::write_amplitudes(const double *a1, const double *a2, int list1, in
   const long long st2[4] = {O * V * V, V * V, V, 1};
   double *lp = nullptr;
   ACES_CUDA(cudaStreamSynchronize(0));  // pending device reads of the old contents
+  UnfilledLists unfilled;
   if (s.nirrep == 1) {
-    ACES_TRY(list_inipck(1, 13, 14, list2ab, 1, false));
+    ACES_TRY(list_inipck(1, 13, 14, list2ab, 1, &unfilled));
     ACES_TRY(c1_list(list2ab, 13, 14, &lp));
   }
   if (lp) {  // a + b v + i v^2 + j v^2 o
     ACES_TRY(perm(lp, o, o, v, v, 0.0, {PT(a2, 1.0, st2[1], st2[0], st2[3], st2[2])}));
+    unfilled.written();
   } else {
     ACES_TRY(perm(tmpb.p, v, v, o, o, 0.0, {PT(a2, 1.0, st2[2], st2[3], st2[0], st2[1])}));
     DevMap dm;

@@ -453,12 +453,16 @@ extern "C" int aces_intprc_df(const double *B, int naux, int on_device) {
   }
   // every irrep of the lists, without the zero fill: all their pair types are
   // FULL, so each element is written below
-  for (const ListSpec &L : kLists)
-    ACES_TRY(list_inipck(1, L.typeL, L.typeR, L.list, 1, false));
+  UnfilledLists unfilled[6];   // by list
+  for (int k = 0; k < 6; ++k)
+    ACES_TRY(list_inipck(1, kLists[k].typeL, kLists[k].typeR, kLists[k].list, 1, &unfilled[k]));
   {
     bool done = false;
     ACES_TRY(produce_packed(dB, naux, irr_o, irr_v, st, &done));
-    if (done) return ACES_OK;
+    if (done) {
+      for (auto &u : unfilled) u.written();
+      return ACES_OK;
+    }
   }
   // ---- any factors: dense products over all ordered pairs,
   //   <pq|rs> = sum_L B_RP[r][p][L] B_SQ[s][q][L]
@@ -507,6 +511,7 @@ extern "C" int aces_intprc_df(const double *B, int naux, int on_device) {
       ACES_CUDA(cudaGetLastError());
     }
     ACES_CUDA(cudaStreamSynchronize(st));
+    unfilled[&L - kLists].written();
   }
   return ACES_OK;
 }

@@ -123,7 +123,14 @@ static int copy_cols(double *ext, int first, int ncols, int irrep, int list, boo
   return ACES_OK;
 }
 
-static int list_touch(int ncols, int nrows, int irrep, int list, bool zero) {
+UnfilledLists::~UnfilledLists() {
+  if (blocks.empty()) return;
+  cudaDeviceSynchronize();  // what the producer had launched
+  for (auto &b : blocks) cudaMemset(b.first, 0, b.second);
+  cudaGetLastError();
+}
+
+static int list_touch(int ncols, int nrows, int irrep, int list, UnfilledLists *unfilled) {
   State &st = state();
   std::lock_guard<std::recursive_mutex> lk(st.mu);
   if (irrep < 1 || irrep > 8 || list < 0 || list > 1000 || ncols < 0 || nrows < 0) {
@@ -145,14 +152,17 @@ static int list_touch(int ncols, int nrows, int irrep, int list, bool zero) {
     set_error("aces_list_touch: out of device memory for %zu bytes", bytes);
     return ACES_ERR_NOMEM;
   }
-  if (bytes && zero) ACES_CUDA(cudaMemset(p, 0, bytes));
+  if (unfilled)
+    unfilled->add((double *)p, bytes);
+  else if (bytes)
+    ACES_CUDA(cudaMemset(p, 0, bytes));
   b.nrows = nrows;
   b.ncols = ncols;
   b.dev = (double *)p;
   return ACES_OK;
 }
 
-int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, bool zero) {
+int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, UnfilledLists *unfilled) {
   State &st = state();
   std::lock_guard<std::recursive_mutex> lk(st.mu);
   const SymInfo &s = st.sym;
@@ -164,7 +174,8 @@ int list_inipck(int irrepx, int sytypl, int sytypr, int list, int iset, bool zer
   }
   for (int r = 1; r <= s.nirrep; ++r) {
     int l = aces_dirprd(r, irrepx);
-    ACES_TRY(list_touch(s.irpdpd[r - 1][sytypr - 1], s.irpdpd[l - 1][sytypl - 1], r, list, zero));
+    ACES_TRY(
+        list_touch(s.irpdpd[r - 1][sytypr - 1], s.irpdpd[l - 1][sytypl - 1], r, list, unfilled));
   }
   if (iset) st.isytyp[list == 0 ? 100 : list] = {sytypl, sytypr};
   return ACES_OK;
@@ -270,7 +281,7 @@ int aces_dirprd(int i, int j) {
 
 int aces_list_touch(int ncols, int nrows, int irrep, int list, int nofrag) {
   (void)nofrag;
-  return list_touch(ncols, nrows, irrep, list, true);
+  return list_touch(ncols, nrows, irrep, list, nullptr);
 }
 
 int aces_updmoi(int ncols, int nrows, int irrep, int list, int iarg1, int iarg2) {
@@ -280,7 +291,7 @@ int aces_updmoi(int ncols, int nrows, int irrep, int list, int iarg1, int iarg2)
 }
 
 int aces_inipck(int irrepx, int sytypl, int sytypr, int list, int iset) {
-  return list_inipck(irrepx, sytypl, sytypr, list, iset, true);
+  return list_inipck(irrepx, sytypl, sytypr, list, iset, nullptr);
 }
 
 int aces_isytyp(int which, int list) {

@@ -175,6 +175,34 @@ static int first_launch_in_order() {
   return 0;
 }
 
+// A producer that fails leaves zeros in the lists it has created, not old
+// device memory, and lists that were there as they were.
+static int failed_producer_leaves_zeros() {
+  const int o = 4, v = 30, n = o + v, naux = 30, list[6] = {13, 10, 16, 25, 30, 233};
+  const size_t MB = size_t(1) << 20;
+  std::vector<double> B((size_t)naux * n * n, 0.0);
+  for (int there = 0; there < 2; ++there) {
+    CHECK(aces_init(0) == ACES_OK && aces_sym_init(1, &o, &v) == ACES_OK);
+    pool_trim();
+    if (there) CHECK(small_system(o, v) == ACES_OK);
+    std::vector<double> two((size_t)o * o, 2.0);
+    if (there) CHECK(aces_putlst(two.data(), 1, 1, 1, 13) == ACES_OK);
+    // room for the lists' memory and for nothing else of size
+    host::budget = host::live + (there ? 0 : 256 * MB) + MB / 8;
+    CHECK(aces_intprc_df(B.data(), naux, 1) == ACES_ERR_NOMEM);
+    host::budget = ~size_t(0);
+    for (int l : list) {
+      int nc = 0, nr = 0;
+      CHECK(aces_list_dims(1, l, &nc, &nr) == ACES_OK && nc > 0 && nr > 0);
+      std::vector<double> x((size_t)nc * nr, 1.0);
+      CHECK(aces_getlst(x.data(), 1, nc, 1, l) == ACES_OK);
+      for (size_t i = 0; i < x.size(); ++i)
+        CHECK(x[i] == (there && l == 13 && i < two.size() ? 2.0 : 0.0));
+    }
+  }
+  return 0;
+}
+
 struct Case {
   const char *name;
   int (*run)();
@@ -184,6 +212,7 @@ static const Case cases[] = {
     {"blocks_stay_with_their_call", blocks_stay_with_their_call},
     {"entry_points_wait", entry_points_wait},
     {"first_launch_in_order", first_launch_in_order},
+    {"failed_producer_leaves_zeros", failed_producer_leaves_zeros},
 };
 
 int main(int argc, char **argv) {
