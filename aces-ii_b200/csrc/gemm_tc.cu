@@ -689,7 +689,7 @@ __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep
     const int live = min(BN, P.N - T.n0), per = (live + 63) / 64 * 32;
     const int c0 = half * per, ncol = min(per, live - c0);  // ncol may be <= 0
     const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c0);
-    const bool frag = C.sm0 != 1;  // unit n stride (checked by the host)
+    const bool frag = C.sm0 != 1;  // contiguous columns (checked by the host)
     uint32_t r[kC / 32][32];
     if (frag) {
 #pragma unroll
@@ -1756,7 +1756,10 @@ int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOpera
   // this path from v = 128 on)
   int kt = 0;
   for (int s = 0; s < nseg; ++s) kt += Apar[s].k_pad / TBK;
-  const bool fits = f32out && N <= TBN_WIDE && kt <= chunk_for(kt);
+  // the wide epilogue takes neighbouring columns as contiguous where the unit
+  // stride runs along n: a view that splits n goes to the other tiles
+  const bool fits = f32out && N <= TBN_WIDE && kt <= chunk_for(kt) &&
+                    (C.sm0 == 1 || C.ndiv > 0x7fffffff);
   if (L.cg == 2)
     L.bn = TBN;
   else if (ch.bn)

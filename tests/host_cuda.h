@@ -22,6 +22,7 @@ struct Launch {
   cudaStream_t stream;
   dim3 grid;
   bool overlapped;   // may be set up while the kernel before it runs
+  bool cluster;      // CTA pairs
 };
 inline std::vector<Launch> launches;
 inline std::map<void *, size_t> blocks;          // live device blocks
@@ -30,8 +31,9 @@ inline std::map<cudaStream_t, int> pending;      // launches since the stream wa
 inline std::function<void()> on_launch = [] {};
 inline cudaError_t last = cudaSuccess;
 
-inline void launch(const void *f, cudaStream_t s, dim3 grid, bool overlapped) {
-  launches.push_back({f, s, grid, overlapped});
+inline void launch(const void *f, cudaStream_t s, dim3 grid, bool overlapped,
+                   bool cluster = false) {
+  launches.push_back({f, s, grid, overlapped, cluster});
   ++pending[s];
   on_launch();
 }
@@ -143,11 +145,13 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **, size_t, cu
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
-  bool over = false;
-  for (unsigned i = 0; i < c->numAttrs; ++i)
+  bool over = false, cluster = false;
+  for (unsigned i = 0; i < c->numAttrs; ++i) {
     over = over || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
                     c->attrs[i].val.programmaticStreamSerializationAllowed);
-  host::launch(f, c->stream, c->gridDim, over);
+    cluster = cluster || c->attrs[i].id == cudaLaunchAttributeClusterDimension;
+  }
+  host::launch(f, c->stream, c->gridDim, over, cluster);
   return cudaSuccess;
 }
 static CUresult host_encode(CUtensorMap *, ...) { return CUDA_SUCCESS; }

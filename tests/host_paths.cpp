@@ -203,6 +203,38 @@ static int failed_producer_leaves_zeros() {
   return 0;
 }
 
+// a batched FP32-output launch of 40 entries with K = 64; the launch, or
+// nullptr when it failed
+static const host::Launch *batched(int N, const CView &C, double beta = 0.0) {
+  SplitOperand a, b;
+  for (SplitOperand *x : {&a, &b}) {
+    x->hi = addr(3);
+    x->lo = addr(4);
+    x->rows = x->rows_pad = 40000;
+    x->k = x->k_pad = 64;
+  }
+  std::vector<BatchEntry> e(40);
+  for (int i = 0; i < 40; ++i) e[i] = BatchEntry{{i}, {i}, 0};
+  host::launches.clear();
+  CallScope call;
+  const int rc = gemm_nt_bf16x3_batched(&a, &b, 1, 600, N, e.data(), e.data(), 40, 1.0, beta, C,
+                                        true, 0);
+  return rc == ACES_OK && !host::launches.empty() ? &host::launches.back() : nullptr;
+}
+
+// The wide tiles take outputs with unit m stride or whole contiguous rows; a
+// view that splits n runs on the other tiles.
+static int wide_tiles_need_plain_rows() {
+  const long long plain = 1LL << 62;
+  const CView rows{addr(5), plain, 0, 170, plain, 0, 1}, cols{addr(5), 600, 0, 1, plain, 0, 600},
+      split{addr(5), plain, 0, 170, 10, 100, 1};
+  const host::Launch *l;
+  CHECK((l = batched(170, rows)) && l->cluster);
+  CHECK((l = batched(170, cols)) && l->cluster);
+  CHECK((l = batched(170, split)) && !l->cluster);
+  return 0;
+}
+
 struct Case {
   const char *name;
   int (*run)();
@@ -213,6 +245,7 @@ static const Case cases[] = {
     {"entry_points_wait", entry_points_wait},
     {"first_launch_in_order", first_launch_in_order},
     {"failed_producer_leaves_zeros", failed_producer_leaves_zeros},
+    {"wide_tiles_need_plain_rows", wide_tiles_need_plain_rows},
 };
 
 int main(int argc, char **argv) {
