@@ -1455,8 +1455,8 @@ namespace {
 // >= 256 rows), split K at the wave-efficiency slice count or none (single
 // products), and for batched FP32-output launches 128 x TBN_1 or 256 x 192
 // tiles.  A class is the launch
-// kind, the K segment (or problem) count, FP32 output, eligibility for pairs,
-// and the output tile counts and k tile count rounded to two significant
+// kind, the K segment (or problem) count, FP32 output, eligibility for pairs
+// and for the wide tiles, and the output tile counts and k tile count rounded to two significant
 // bits.  Each candidate runs once untimed and three times timed (CUDA events)
 // on the product's stream, into the product's own output when beta = 0 and
 // into a zeroed scratch array with unit m stride otherwise (the layout whose
@@ -1472,6 +1472,9 @@ struct TuneChoice {
   int nosplit = 0;  // single products: 1 = no split K
   int changed = 0;  // cached entries: the choice differs from the built-in rule
 };
+constexpr int kTuneWide = 16;   // flag of the classes that the 256 x 192 tiles can serve
+                                // (8 was N > 256 in files of older builds, whose wide
+                                // tile was another: their choices match no such class)
 struct TuneKey {
   int dev, kind, nseg, flags, tm, tn, kt;
   bool operator==(const TuneKey &o) const {
@@ -1742,6 +1745,18 @@ int grouped_run(int cg, const GroupedProblem *probs, int nprob, double alpha, do
   return P.tailZ ? tail_reduce(P, part, alpha, beta, st) : ACES_OK;
 }
 
+// FP32 output whose every tile is one accumulation chunk, 128 <= N <= 192: one
+// wide tile across N.  (T), o = 10 at v = 128 / 136 / 144 / 145: 5.9 / 8.0 / 8.8
+// / 10.7 ms on wide tiles, 6.4 / 9.4 / 10.4 / 15.4 on 144-wide ones; o = 8,
+// v = 192: 11.3 against 15.3 (smaller N was not measured: (T) takes this path
+// from v = 128 on).  The wide epilogue takes neighbouring columns as contiguous
+// where the unit stride runs along n: a view that splits n goes to the other
+// tiles.
+bool wide_fits(int kt, int N, bool f32out, const CView &C) {
+  return f32out && N >= kWideMinN && N <= TBN_WIDE && kt <= chunk_for(kt) &&
+         (C.sm0 == 1 || C.ndiv > 0x7fffffff);
+}
+
 int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOperand *Bpar,
                 int nseg, int M, int N, const BatchEntry *d_entries, int nbatch, double alpha,
                 double beta, const CView &C, bool f32out, cudaStream_t st) {
@@ -1749,23 +1764,15 @@ int batched_run(const TuneChoice &ch, const SplitOperand *Apar, const SplitOpera
   memset(&L, 0, sizeof(L));
   L.nprob = 1;
   L.cg = ch.cg == 2 ? 2 : 1;
-  // FP32 output whose every tile is one accumulation chunk, 128 <= N <= 192:
-  // one wide tile across N.  (T), o = 10 at v = 128 / 136 / 144 / 145: 5.9 / 8.0
-  // / 8.8 / 10.7 ms on wide tiles, 6.4 / 9.4 / 10.4 / 15.4 on 144-wide ones;
-  // o = 8, v = 192: 11.3 against 15.3 (smaller N was not measured: (T) takes
-  // this path from v = 128 on)
   int kt = 0;
   for (int s = 0; s < nseg; ++s) kt += Apar[s].k_pad / TBK;
-  // the wide epilogue takes neighbouring columns as contiguous where the unit
-  // stride runs along n: a view that splits n goes to the other tiles
-  const bool fits = f32out && N <= TBN_WIDE && kt <= chunk_for(kt) &&
-                    (C.sm0 == 1 || C.ndiv > 0x7fffffff);
+  const bool fits = wide_fits(kt, N, f32out, C);
   if (L.cg == 2)
     L.bn = TBN;
   else if (ch.bn)
     L.bn = ch.bn == kWideTag && fits ? kWideTag : TBN_1;
   else
-    L.bn = fits && N >= kWideMinN && g_tc_wide.load() ? kWideTag : TBN_1;
+    L.bn = fits && g_tc_wide.load() ? kWideTag : TBN_1;
   if (L.bn == kWideTag) L.cg = 2;
   ACES_TRY(set_problem(L, 0, Apar, Bpar, nseg, M, N, C));
   Problem &P = L.prob[0];
@@ -1942,7 +1949,7 @@ int gemm_nt_bf16x3_batched(const SplitOperand *Apar, const SplitOperand *Bpar, i
   const long long tm = (M + TBM - 1) / TBM, tn = (N + TBN_1 - 1) / TBN_1;
   const TuneKey key{current_device(), 2, nseg,
                     (M >= 2 * TBM ? 1 : 0) | (f32out ? 2 : 0) | (N > TBN_1 ? 4 : 0) |
-                        (N > kWideTag ? 8 : 0),
+                        (wide_fits(kt, N, f32out, C) ? kTuneWide : 0),
                     bucket2(tm * nbatch), bucket2(tn), bucket2(kt)};
   TuneChoice ch;
   if (tune_lookup(key, &ch))
@@ -1952,10 +1959,10 @@ int gemm_nt_bf16x3_batched(const SplitOperand *Apar, const SplitOperand *Bpar, i
   if (beta != 0.0 || !can_time(st))
     return batched_run(def, Apar, Bpar, nseg, M, N, d_entries, nbatch, alpha, beta, C, f32out,
                        st);
-  // both widths of the one-CTA tile (cands[0] keeps the default rule); the
-  // CTA pairs stay with the aces_set_tc_pairs switch here
+  // the 144-wide tiles and the wide ones of a CTA pair (cands[0] keeps the
+  // default rule); the 128-wide pairs stay with the aces_set_tc_pairs switch
   std::vector<TuneChoice> cands{def};
-  if (def.cg == 1 && f32out && N >= kWideMinN && N <= TBN_WIDE && kt <= chunk_for(kt)) {
+  if (def.cg == 1 && wide_fits(kt, N, f32out, C)) {
     TuneChoice c;
     c.bn = g_tc_wide.load() ? TBN_1 : kWideTag;
     cands.push_back(c);
@@ -2067,7 +2074,7 @@ int tc_autotune_load(const char *path) {
     // each choice must be one the tuner could have made for its class
     const bool ok =
         n == 10 && kind >= 0 && kind <= 2 && nseg >= 1 &&
-        nseg <= (kind == 1 ? kMaxProb : kMaxSeg) && flags >= 0 && flags <= 15 && v[3] >= 0 &&
+        nseg <= (kind == 1 ? kMaxProb : kMaxSeg) && flags >= 0 && flags <= 31 && v[3] >= 0 &&
         v[4] >= 0 && v[5] >= 0 && (cg == 1 || (cg == 2 && (flags & 1))) &&
         (bn == 0 || (kind == 2 && (flags & 2) && cg == 1 && (bn == TBN_1 || bn == kWideTag))) &&
         (nosplit == 0 || (nosplit == 1 && kind == 0 && cg == 1)) && (changed == 0 || changed == 1);

@@ -1,6 +1,9 @@
 // Cases of test_host_paths.py: one function each, run by name; 0 = passed.
 #include "host_cuda.h"
 
+#include <unistd.h>
+
+#include <string>
 #include <thread>
 
 using namespace acesb200;
@@ -235,6 +238,50 @@ static int wide_tiles_need_plain_rows() {
   return 0;
 }
 
+// Tile choices of batched launches: widths that the wide tiles serve and widths
+// that they do not are different classes, and a saved choice of the wide tiles
+// is not applied to the latter.
+static int tile_choices_by_width() {
+  const long long plain = 1LL << 62;
+  const CView cols{addr(5), plain, 0, 1, plain, 0, 600};
+  const int others[2][2] = {{100, 140}, {220, 170}};   // not served, served: as many 144-wide tiles
+  for (auto &w : others) {
+    aces_set_autotune(2);
+    aces_set_autotune(1);
+    long long n[3] = {0, 0, 0}, changed;
+    double ms;
+    CHECK(batched(w[0], cols));
+    aces_autotune_stats(&n[0], &changed, &ms);
+    CHECK(batched(w[1], cols));
+    aces_autotune_stats(&n[1], &changed, &ms);
+    CHECK(n[0] == 1 && n[1] == 2);
+    // the file takes the choices through save and load, and one of the wide tiles
+    // for every class of batched launches keeps to the widths they serve
+    char path[] = "/tmp/tile_choicesXXXXXX";
+    CHECK(mkstemp(path) >= 0 && aces_autotune_save(path) == ACES_OK);
+    FILE *f = std::fopen(path, "r");
+    std::string text;
+    for (int c; (c = std::fgetc(f)) != EOF;) text += (char)c;
+    std::fclose(f);
+    for (size_t at; (at = text.find(" 1 0 0 0\n")) != std::string::npos;)
+      text.replace(at, 9, " 1 256 0 1\n");
+    f = std::fopen(path, "w");
+    std::fputs(text.c_str(), f);
+    std::fclose(f);
+    aces_set_autotune(2);
+    CHECK(aces_autotune_load(path) == ACES_OK);
+    aces_autotune_stats(&n[2], &changed, &ms);
+    CHECK(n[2] == 2 && changed == 2);
+    const host::Launch *l;
+    CHECK((l = batched(w[0], cols)) && !l->cluster);
+    CHECK((l = batched(w[1], cols)) && l->cluster);
+    std::remove(path);
+    aces_set_autotune(0);
+    aces_set_autotune(2);
+  }
+  return 0;
+}
+
 struct Case {
   const char *name;
   int (*run)();
@@ -246,6 +293,7 @@ static const Case cases[] = {
     {"first_launch_in_order", first_launch_in_order},
     {"failed_producer_leaves_zeros", failed_producer_leaves_zeros},
     {"wide_tiles_need_plain_rows", wide_tiles_need_plain_rows},
+    {"tile_choices_by_width", tile_choices_by_width},
 };
 
 int main(int argc, char **argv) {
