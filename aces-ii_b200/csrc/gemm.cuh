@@ -91,7 +91,7 @@ int gemm_nt_f64_scratch(int M, int N, int K, double alpha, const double *A, long
                         double *ws, size_t cap, cudaStream_t st);
 
 // Several FP64 products in one launch: a device table of tasks, each
-//   C = alpha * sum_s A_s B_s^T + beta * C   over up to 4 K segments.
+//   C = alpha * sum_s A_s B_s^T + beta * C   over up to 4 K segments, none empty.
 // tri: C is symmetric (the two sides of every segment are the same rows, M = N,
 // beta = 0): only the lower triangle of tiles is computed, each stored twice.
 struct F64Seg {

@@ -878,6 +878,11 @@ int f64_tasks_plan(F64Task *tasks, int n, F64TaskPlan *plan) {
       set_error("f64 tasks: task %d is %d x %d with %d segments", i, t.M, t.N, t.nseg);
       return ACES_ERR_ARG;
     }
+    for (int s = 0; s < t.nseg; ++s)  // the kernel steps from one segment to the next
+      if (t.seg[s].K < 1) {
+        set_error("f64 tasks: segment %d of task %d has K = %d", s, i, t.seg[s].K);
+        return ACES_ERR_ARG;
+      }
     const int nkt = f64_ktiles(t);
     for (int b = 0; b < 2; ++b) {
       const int nt = f64_tiles(t.M, t.N, t.tri, kTile[b].BM, kTile[b].BN);

@@ -282,6 +282,21 @@ static int tile_choices_by_width() {
   return 0;
 }
 
+// A task table with an empty K segment is refused (the kernel would take a tile
+// of the next segment for it).
+static int empty_segments_are_refused() {
+  for (int empty = -1; empty < 3; ++empty) {
+    F64Task t{};
+    t.nseg = 3;
+    t.M = t.N = 40;
+    t.C = cview_colmajor(addr(5), 40);
+    for (int s = 0; s < 3; ++s) t.seg[s] = F64Seg{addr(0), addr(1), 50, 50, s == empty ? 0 : 50};
+    F64TaskPlan plan;
+    CHECK((f64_tasks_plan(&t, 1, &plan) == ACES_OK) == (empty < 0));
+  }
+  return 0;
+}
+
 struct Case {
   const char *name;
   int (*run)();
@@ -294,6 +309,7 @@ static const Case cases[] = {
     {"failed_producer_leaves_zeros", failed_producer_leaves_zeros},
     {"wide_tiles_need_plain_rows", wide_tiles_need_plain_rows},
     {"tile_choices_by_width", tile_choices_by_width},
+    {"empty_segments_are_refused", empty_segments_are_refused},
 };
 
 int main(int argc, char **argv) {

@@ -36,7 +36,7 @@ def exe(tmp_path_factory):
 @pytest.mark.parametrize("case", ["no_room_for_partials", "blocks_stay_with_their_call",
                                   "entry_points_wait", "first_launch_in_order",
                                   "failed_producer_leaves_zeros", "wide_tiles_need_plain_rows",
-                                  "tile_choices_by_width"])
+                                  "tile_choices_by_width", "empty_segments_are_refused"])
 def test_host_path(exe, case):
     r = subprocess.run([exe, case], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
