@@ -19,10 +19,9 @@
 // packed ones (32 TFLOP/s) and 3.2 ms of expansion; with 8 irreps the products
 // shrink by another factor of 64 at most.
 //
-// The factors are symmetric by contract; factors that are not (beyond
-// rounding: 64 units in the last place of the largest element) take dense
-// products over all ordered pairs, as they are.  So do systems whose packed
-// G does not fit beside the lists.
+// That takes factors equal to their transposes bit for bit.  Others, symmetric
+// to rounding only or not at all, take dense products over all ordered pairs,
+// as they are; so do systems whose packed G does not fit beside the lists.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -282,7 +281,7 @@ int produce_packed(const double *dB, int naux, const std::vector<int> &irr_o,
   double stats[2];
   ACES_CUDA(cudaMemcpyAsync(stats, d_stats, 16, cudaMemcpyDeviceToHost, st));
   ACES_CUDA(cudaStreamSynchronize(st));
-  if (!std::isfinite(stats[0]) || !(stats[1] <= stats[0] * 0x1p-46)) return ACES_OK;
+  if (!std::isfinite(stats[0]) || stats[1] != 0.0) return ACES_OK;   // (a NaN too)
   double *F = (double *)mem.get((size_t)nrows * kp * 8);
   double *G = (double *)mem.get(std::max(need_small, need_vv) * 8);
   // one upload: rows, the pair-type tables of the irrep blocks, indices

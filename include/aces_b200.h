@@ -120,9 +120,10 @@ double *aces_list_devptr(int irrep, int list);
  * orbitals in DPD order -- occupied by irrep, then virtual by irrep -- with
  * (pq|rs) = sum_L B[L][p][q] B[L][r][s]) it creates lists 13 <Ij|Kl>,
  * 10 <Ij|Ka>, 16 <Ab|Ij>, 25 <Ai|Bj>, 30 <Ab|Ci> and 233 <Ab|Cd> in every irrep
- * (INIPCK) and fills them in FP64.  Symmetric factors (to 64 units in the last
- * place of the largest element) are multiplied once per distinct integral,
- * others over all ordered pairs as they are.  `B` is a device pointer when on_device is
+ * (INIPCK) and fills them in FP64.  Factors equal to their transposes bit for
+ * bit are multiplied once per distinct integral, others over all ordered pairs
+ * as they are (several times slower: symmetrise factors that a transformation
+ * left symmetric to rounding).  `B` is a device pointer when on_device is
  * nonzero, else host memory copied in.  Requires aces_sym_init; the orbital
  * energies (record SCFEVALA) are the caller's, as with PUTLST. */
 int aces_intprc_df(const double *B, int naux, int on_device);
