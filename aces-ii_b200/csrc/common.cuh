@@ -63,7 +63,7 @@ extern std::atomic<long long> g_launches;
 // measured slower (its blocks take slots from a last wave: EOM o = 6, v = 50
 // 14.2 ms), and this way no load of the old kernel can refill an L1 line after
 // the new one has started.  Back-to-back dependent launches, direct or from a
-// captured graph, lose 1-1.5 us each without it: EOM o = 6, v = 50 (2900
+// captured graph, lose 1-1.5 us each without it: EOM o = 6, v = 50 (2600
 // launches) 15.2 -> 13.4 ms, CCSD o = 5, v = 21 3.10 -> 2.72 ms.
 // The first kernel of a call follows a kernel of the caller, which may release
 // its successors early: it is launched in plain stream order.

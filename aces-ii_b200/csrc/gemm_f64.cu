@@ -21,12 +21,14 @@ namespace {
 // modulo 4: the 16 lanes of a 64-bit load phase (four neighbouring rows x four
 // k) then cover all 32 banks, and so do the copies (one row per 8 lanes).
 //
-// Every output sums its k in ascending order.  One 128-bit load per row and k
-// step, with the k taken as 0, 2, 4, 6, 1, 3, 5, 7, is 1-2 % faster (2401 x
-// 1519 x 2050: 601 us against 612), but its other last bits move values across
-// the rounding boundaries of the BF16 split: a CCSD with o = 24, v = 220 in
-// split precision then differed by up to 1e-9 with the order of its lists'
-// sums, and by 1e-17 with them in order.
+// Every output of an unsplit product, and every slice of a split one, sums its k
+// in ascending order.  (Split K regroups the sums by slice, k_gemm_tiny_f64 by
+// lane.)  One 128-bit load per row and k step, with the k taken as 0, 2, 4, 6, 1,
+// 3, 5, 7, is 1-2 % faster (the call of 2401 x 1519 x 2049, N/N: 601 us against
+// 612), but its other last bits move values across the rounding boundaries of
+// the BF16 split: a CCSD with o = 24, v = 220 in split precision, whose lists
+// are unsplit products, then differed by up to 1e-9, and by 1e-17 with their
+// sums in order.
 // ---------------------------------------------------------------------------
 constexpr int BK = 16, kStages = 4;
 
@@ -707,15 +709,15 @@ int gemv_f64(int M, int K, double alpha, const double *A, long long lda, const d
 namespace {
 // Tile shapes.  The DMMA pipe of an SM is filled by several small blocks rather
 // than one large one: while one block waits at its k tile's barrier the others
-// issue.  8192 x 4096 x 4096: 34.8 TFLOP/s with 64 x 64 tiles and three blocks
+// issue.  8192 x 4096 x 4096: 34.6 TFLOP/s with 64 x 64 tiles and three blocks
 // per SM, 33.9 with 128 x 64 and two, 29.7 with 128 x 128 and one (the
 // m8n8k4 and the m16n8k8 form of the instruction measure the same); and the
 // last wave and the ragged edges of a 64-wide grid cost less: 2401 x 1519 x
-// 2050 takes 525 us against 734 (shapes measured with 128-bit fragment loads; k
-// in ascending order, as now, costs 1-2 %).  32 x 32 tiles serve outputs too small for
-// that: 120 x 96 x 150 in 8.7 us against 41.9 on one 128 x 128 tile.  The
+// 2050 takes 513 us against 734 (2049, with the 8-byte copies of odd rows: 578).
+// 32 x 32 tiles serve outputs too small for that: 120 x 96 x 150 in 6.5 us
+// against 41.9 on one 128 x 128 tile.  The
 // 16- and 32-wide tiles are for products with a short side, which stream
-// their long operand: 404600 x 14 x 170 in 113 us (550 MB, 4.9 TB/s) against
+// their long operand: 404600 x 14 x 170 in 111 us (550 MB, 4.9 TB/s) against
 // 690 us for an FMA kernel with synchronous 64 x 32 tiles.
 using T64 = TileF64<64, 64, 2, 2, 3>;
 using T32 = TileF64<32, 32, 2, 2, 6>;

@@ -12,7 +12,7 @@
 //   warp 0  TMA producer (all lanes wait, one elected lane issues)
 //   warp 1  TMEM allocator + MMA issuer (all lanes wait, one elected lane issues)
 //   warps 2.. epilogue: two or three warps per TMEM lane quadrant, each
-//             thread one output row x 48, 64 or 128 columns, accumulated in
+//             thread one output row x 48, 64 or 96 columns, accumulated in
 //             FP64 across K chunks
 // Three variants: one CTA per 128 x 144 output tile (14 warps, 3-stage
 // mbarrier pipeline; the default), a cluster pair of CTAs (tcgen05
@@ -194,10 +194,10 @@ constexpr int kRowBytes = TBK * 2;                    // one swizzled smem row
 constexpr int kUnit = 64 / TBK;                       // k tiles per 64 K elements
 constexpr int TILE_A = TBM * TBK * 2;                 // bytes of one BF16 plane tile of A
 constexpr int kSmemLimit = 227 * 1024;
-// Per-CTA pipeline geometry of the two variants: CG = 1, one CTA per 128 x 128
-// output tile (A and B tiles of 128 rows); CG = 2, a CTA pair per 256 x 128
-// tile (tcgen05 cta_group::2), each CTA holding its 128 rows of A and half of
-// the B rows, so a k tile brings 48 KB per CTA into shared memory instead of
+// Per-CTA pipeline geometry of the variants: CG = 1, one CTA per 128 x BN
+// output tile (128 rows of A, BN of B); CG = 2, a CTA pair per 256 x BN tile
+// (tcgen05 cta_group::2), each CTA holding its 128 rows of A and half of the B
+// rows, so with BN = 128 a k tile brings 48 KB per CTA into shared memory instead of
 // 64 KB for the same products.
 template <int CG, int BN = TBN>
 struct Geom {
@@ -219,8 +219,8 @@ inline int chunk_for(int kTilesTotal) {
   if (kTilesTotal <= 1152 * kUnit) return 4 * kUnit;
   return 2 * kUnit;
 }
-// Epilogue warps of a tile width: 2 per TMEM lane quadrant (64 or 128 columns
-// each), or 3 per quadrant for the 144-wide tiles (48 columns each, whose
+// Epilogue warps of a tile width: 2 per TMEM lane quadrant (64 columns each, 96
+// of the wide tiles), or 3 per quadrant for the 144-wide tiles (48 columns each, whose
 // FP64 sums fit the registers of a 14-warp block)
 template <int BN>
 constexpr int epi_warps() { return BN % 64 == 0 ? 8 : 12; }
@@ -232,9 +232,9 @@ constexpr int block_threads() { return 32 * (2 + epi_warps<BN>()); }
 // accumulation chunk with FP32 output (the batched (T) classes: one tile across
 // N = v <= 192).  No FP64 chunk sums to hold, so the epilogue streams the TMEM
 // columns straight to the output.  Their K is short (8 k tiles), so the copies'
-// latency bounds them: with one CTA per 128 x 256 tile only two stages of
-// 96 KB fit, and a k tile took 2600 cycles against the 1056 of its products; a
-// pair shares B, which leaves 56 KB per CTA and stage and four stages.
+// latency bounds them: with one CTA per 128 x 256 tile only two stages of 96 KB
+// fit; a pair shares B, which leaves 56 KB per CTA and stage and four stages
+// ((T) classes of o = 14, v = 170: 27.5 ms on the former, 21.9 on pairs).
 constexpr int TBN_WIDE = 192;
 constexpr int kWideMinN = 128;
 constexpr int kWideTag = 256;   // the wide variant in a launch's bn and in saved tile choices
@@ -422,11 +422,9 @@ __device__ __forceinline__ uint32_t idesc_for(int n_live) {
 }
 
 // The producer and MMA warps run their loops with all 32 lanes and issue from
-// one elected lane.  A loop under `lane == 0` is divergent code, where every
-// tcgen05.mma first moves its descriptors into uniform registers: measured
-// 62-87 cycles of issue per instruction, above the 64-72 cycles that a
-// 128 x 128 or 128 x 144 product takes, and 600 cycles of bookkeeping per k
-// tile; warp-uniform code issues one in 46.
+// one elected lane.  In a loop under `lane == 0`, divergent code, the issue of a
+// tcgen05.mma took longer than its product (16290 x 400 x 16290: 594 us, 548 with
+// warp-uniform code; 24310 x 576 x 24310: 1815 and 1690).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -660,11 +658,10 @@ __device__ __forceinline__ StageAt stage_at(const Problem &P, const TileRef &T,
 // Unit n stride (stores only): the columns are loaded as product fragments,
 // so an access covers 8 rows x 8 columns and writes whole 32-byte sectors (a
 // row per lane would touch 32 sectors with 4 or 16 bytes each).
-// This code was the bound of the (T) class launches: about 24 instructions
-// per column (the view walk, two conversions and an FP64 product, dead
-// columns) on 2 warps per SM sub-partition took 24k cycles per tile, the
-// tensor pipe busy for 8.7k of them (v = 170, o = 4: 440 us per accumulating
-// launch and 650 us for the storing one).
+// A view walk, two conversions and an FP64 product per column, dead columns
+// included, on two warps per SM sub-partition bounded the (T) class launches
+// (o = 14, v = 170: 41.1 ms, 27.5 with this code on the same tiles; o = 4,
+// v = 170: 440 us per accumulating launch and 650 us for the storing one before).
 template <int CG, int BN>
 __device__ __forceinline__ void epilogue_wide(const Launch &L, int t0, int tstep, uint32_t tmem,
                                               uint64_t *acc_full, uint64_t *acc_empty,
@@ -1267,8 +1264,8 @@ MapCache &map_cache() {
 // The map's K extent is the operand's true K (rows stay k_pad elements apart):
 // the tail of the last k tile of a segment is the TMA's zero fill, read from
 // neither L2 nor DRAM (for a K = nocc segment, 20 of the 64 columns of a k
-// tile are data).  The padding in memory is zero as well, so the products
-// are the same either way.
+// tile are data).  The extent must be the true K: the padding in memory need not have
+// been written (the ladder's U+- planes).
 int make_map(CUtensorMap *m, void *base, int rows_pad, int k_pad, int k, int box_rows) {
   const MapKey key{base, rows_pad, k_pad, k, box_rows};
   MapCache &mc = map_cache();

@@ -686,7 +686,6 @@ void launch_energy(double *out3, const double *t2, const double *t1, const doubl
   launch_after(k_final_sum, 3, 32, 0, st, out3, scratch, 3); count_launch();
 }
 
-// xn = x + damp (xn - x), two loads and a store per element
 // dst[i] = src[i].  A kernel rather than cudaMemcpyAsync: its launch overlaps
 // the kernel before it, and the next one's overlaps its own (EOM o = 6, v = 50,
 // 136 copies: 12.9 -> 12.5 ms; 223 MB take 78 us either way).
@@ -726,6 +725,7 @@ void launch_copy(double *dst, const double *src, long long n, cudaStream_t st) {
   count_launch();
 }
 
+// xn = x + damp (xn - x), two loads and a store per element
 __global__ void k_blend(double *__restrict__ xn, const double *__restrict__ x, double damp,
                         long long n) {
   after_previous();

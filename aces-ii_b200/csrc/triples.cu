@@ -65,10 +65,10 @@ __device__ __forceinline__ void decode_set(int n, int &a, int &b, int &c) {
 // ordered pair of the three tiles, and the t1 rows and orbital energies of the
 // three tiles.  Each of its 128 threads then evaluates four sets that share
 // (b, c): what depends on these alone is read once.
-// Instruction bound (W is read once, at 10 % of the DRAM rate): index splits
-// per staged element, 36 shared-memory reads and a general 6 x 6 form per set,
-// and a per-ordering sum for repeated virtuals took 1830 instructions per warp
-// (o = 14, v = 170: 14.0 ms; with the form above and these loop orders 8.3).
+// Instruction bound (W is read once, at 16 % of the DRAM rate, the issue slots
+// two thirds full): with index splits per staged element, 36 shared-memory reads
+// and a general 6 x 6 form per set, and a per-ordering sum for repeated virtuals
+// o = 14, v = 170 took 14.0 ms; with the form above and these loop orders 8.3.
 constexpr int kTile = 8;
 // triplets of one FP64 batch (the energy launch's grid.y holds 65535)
 constexpr int kMaxTasks = 32768;

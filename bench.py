@@ -593,13 +593,14 @@ def run_ours(a, rank, world, local_rank):
 
 
 # DRAM bytes of the grouped packed-ladder launch of the c2 cycle: an ncu
-# capture of its symmetric product alone (--kernel-case ladder-packed, M = K =
-# 16290, N = 400: 1161.2 MB read + 45.4 MB written) scaled by the units the
-# grouped launch processes, (16290^2 + 16110^2) / 16290^2
-LADDER_TRAFFIC = {"c2": (1161.2e6 + 45.4e6) * (16290 ** 2 + 16110 ** 2) / 16290 ** 2}
+# capture of its symmetric product alone with the reduction of its last wave
+# (--kernel-case ladder-packed, M = K = 16290, N = 400: 1315.3 + 35.2 MB read,
+# 63.9 MB written) scaled by the units the grouped launch processes,
+# (16290^2 + 16110^2) / 16290^2
+LADDER_TRAFFIC = {"c2": (1315.3e6 + 35.2e6 + 63.9e6) * (16290 ** 2 + 16110 ** 2) / 16290 ** 2}
 LADDER_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the symmetric ladder "
-                         "product (--kernel-case ladder-packed) scaled to the grouped launch by "
-                         "(n+^2 + n-^2) / n+^2")
+                         "product and its reduction (--kernel-case ladder-packed) scaled to the "
+                         "grouped launch by (n+^2 + n-^2) / n+^2")
 
 
 def cublas_fp64_reference(o, v, dev, reps=5):
@@ -921,7 +922,7 @@ PROGRAM_CASES = {
     "triples-o10-v180": dict(nocc=10, nvir=180, naux=540, seed=5, bscale=0.25),
     # the same kernels on a few GB of device memory (56 triplets, one batch)
     "triples-o6-v128": dict(nocc=6, nvir=128, naux=300, seed=5, bscale=0.25),
-    # v = 136 > 128: the (T) classes on 128 x 256 tiles, a few GB on the device
+    # the (T) classes on 256 x 192 pair tiles, a few GB on the device
     "triples-o4-v136": dict(nocc=4, nvir=136, naux=200, seed=5, bscale=0.25),
     # Lambda + density on the convergent C4 system (split precision)
     "lambda-c4": dict(nocc=20, nvir=180, naux=600, seed=3, bscale=0.25, lam=True),
