@@ -285,7 +285,9 @@ int xvcc_run(aces_cc_config *cfg);
  * by xvcc_run; writes L1 to list 190 (irrep 1), L2(AB) to list 146 and
  * L2(AA) = L2 - L2~ to list 144, in the reference's convention (the
  * multipliers its own xlambda leaves there: L1 = l1/2, L2 = (2 l2 + l2~)/3 of
- * the Lagrange multipliers l of the spin-adapted residual). */
+ * the Lagrange multipliers l of the spin-adapted residual).  Without symmetry
+ * list 233 is read in place by a later program that runs in another precision
+ * than xvcc_run did (here and in xvee_run): it has to keep its integrals. */
 int xlambda_run(aces_cc_config *cfg);
 
 /* DENSOO/DENSVV/DENSVO (dens/densoo.F, densvv.F, densvo.F): the CCSD
